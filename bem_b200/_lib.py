@@ -24,6 +24,8 @@ N_COUNTERS = len(COUNTERS)
 SEG_FIELDS = 11
 BLOCK_SEGS = 32
 RUN_NODES = 8
+MAP_TAG, MAP_UNIT, MAP_HEADER, MAP_N = 0x4D50, 64, 8, 12
+MAP_REC = 8 + 2 * MAP_N * MAP_N
 
 _d = ctypes.c_double
 _i32 = ctypes.c_int32
@@ -105,6 +107,8 @@ SIGNATURES = {
     "spt_accel": (ctypes.c_int, [ctypes.POINTER(SptAccelArgs), ctypes.POINTER(SptGeometry),
                                  ctypes.POINTER(SptBem), _p]),
     "spt_bem_field": (ctypes.c_int, [_p, _p, _p, _i64, ctypes.POINTER(SptBem), _i32, _p, _p, _p, _p]),
+    "spt_map_classify": (ctypes.c_int, [_p, _i32, ctypes.POINTER(SptBem), _d, _p, _p, _p]),
+    "spt_map_cells": (ctypes.c_int, [_p, _i32, ctypes.POINTER(SptBem), _p, _p, _p, _p, _p, _p]),
     "spt_surrogate_field": (ctypes.c_int, [_p, _p, _p, _i64, ctypes.POINTER(SptBem), ctypes.POINTER(SptTraceParams),
                                            _p, _p, _p, _p]),
     "spt_compact_groups": (ctypes.c_int, [_p, _i32, _p, _p, _p, _p]),

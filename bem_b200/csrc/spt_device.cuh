@@ -286,6 +286,7 @@ struct Ctx {
     double* base;    // dynamic smem
     Layout L;
     double *y0, *nw_, *sp, *kp, *kv, *tb, *td, *q, *m, *cps, *fld, *img, *bpt, *tiles, *red, *imgs;
+    double* ntmp;    // near sums' E_z per record (stride 3): fld, or img while fld holds mapped fields
     int* live;
     int* list;
     unsigned char* nflag;
@@ -342,6 +343,7 @@ __device__ inline void bind(Ctx& c, double* smem, int E, int far_rule, double* s
     c.m = smem + L.m;
     c.cps = smem + L.cps;
     c.fld = smem + L.fld;
+    c.ntmp = c.fld;
     c.img = smem + L.img;
     c.bpt = smem + L.bpt;
     c.imgs = smem + L.imgs;
@@ -446,7 +448,7 @@ __device__ __forceinline__ void round_reduce(Ctx& c, int r0, int np_, double* ar
             sabs += c.red[w * 3 * kRound + 2 * kRound + tid];
         }
         const int k = r0 + tid;
-        const double er = sr + P[8 * k + 7], ez = sz + c.fld[3 * k + 2];
+        const double er = sr + P[8 * k + 7], ez = sz + c.ntmp[3 * k + 2];
         P[8 * k + 5] = er;
         P[8 * k + 6] = ez;
         if (MIX) {
@@ -665,6 +667,98 @@ __device__ __forceinline__ void cluster_field(const double* rec, int nt, double 
     const double e_r = A * sc, e_t = s * B * sc;
     er = e_r * s + e_t * u;
     ez = e_r * u - e_t * s;
+}
+
+// ---------------------------------------------------------------------------
+// Field map (SptBem.reserved, spt_map.cu): square cells of a quadtree over the
+// (rho, z) half plane, each holding (E_rho, E_z) as polynomials of degree
+// SPT_MAP_N - 1 in either coordinate.  The field is analytic away from the
+// surface, so cells a few half-widths from it converge to rounding; cells
+// within SPT_MAP_BAND panel lengths of a panel hold none, and points there
+// take the direct sum.
+__device__ __forceinline__ const double* field_map(const SptBem& b) {
+    return ((unsigned)b.reserved >> 16) == SPT_MAP_TAG ? b.clusters + (size_t)(b.reserved & 0xffff) * SPT_MAP_UNIT
+                                                       : nullptr;
+}
+
+// Cell that holds (rho, z), or -1: three quadtree levels per table of 64
+// entries, so a point's cell is at most ten dependent loads away; one lane
+// per point.
+__device__ __forceinline__ int map_find(const double* map, double rho, double z) {
+    const double u = rho * __ldg(map), v = (z - __ldg(map + 1)) * __ldg(map);
+    if (!(u < 1.0 && v >= 0.0 && v < 1.0)) return -1;
+    const unsigned iu = (unsigned)(u * 1073741824.0), iv = (unsigned)(v * 1073741824.0);
+    const int* tab = reinterpret_cast<const int*>(map + SPT_MAP_HEADER);
+    int node = 0;
+    for (int sh = 27; sh >= 0; sh -= 3) {
+        const int e = __ldg(tab + node * 64 + ((iv >> sh) & 7) * 8 + ((iu >> sh) & 7));
+        if (e >= -1) return e;
+        node = -2 - e;
+    }
+    return -1;
+}
+
+// (E_rho, E_z) at (rho, z) of cell `leaf`, by one warp; every lane returns
+// both.  Lane i of each half takes row i (power i of the rho coordinate, lower
+// half E_rho, upper half E_z) as a polynomial in z: the row's coefficients
+// are one coalesced line per power, the Horner chains of all rows run side by
+// side, and four shuffles add the rows.  Bound by the record's 2.3 KB through
+// L1/L2: a million points off the benchmark tip take 0.33 ms, their direct
+// sums (the closest-segment, near and far phases, ~6300 warp instructions a
+// point) 20 ms.  Twelve orders: eight need cells a third as wide for 1e-14,
+// sixteen twice the bytes a point.
+__device__ __forceinline__ void map_field(const double* map, int leaf, double rho, double z, double& er, double& ez) {
+    const double* rec = map + (size_t)__ldg(map + 2) + (size_t)leaf * SPT_MAP_REC;
+    const int lane = threadIdx.x & 31, i = lane & 15;
+    const bool on = i < SPT_MAP_N;
+    const double* a = rec + 8 + (lane >> 4) * SPT_MAP_N + (on ? i : 0);
+    double c[SPT_MAP_N];
+#pragma unroll
+    for (int j = 0; j < SPT_MAP_N; ++j) c[j] = __ldg(a + j * 2 * SPT_MAP_N);
+    const double iw = __ldg(rec + 2);
+    const double x = (rho - __ldg(rec)) * iw, y = (z - __ldg(rec + 1)) * iw;
+    const double x2 = x * x, x4 = x2 * x2, y2 = y * y;
+    double p = (i & 1) ? x : 1.0;
+    if (i & 2) p *= x2;
+    if (i & 4) p *= x4;
+    if (i & 8) p *= x4 * x4;
+    double e = c[SPT_MAP_N - 2], o = c[SPT_MAP_N - 1];
+#pragma unroll
+    for (int j = SPT_MAP_N - 4; j >= 0; j -= 2) {
+        e = fma(e, y2, c[j]);
+        o = fma(o, y2, c[j + 1]);
+    }
+    double r = on ? fma(o, y, e) * p : 0.0;
+#pragma unroll
+    for (int s = 8; s > 0; s >>= 1) r += __shfl_xor_sync(0xffffffffu, r, s);
+    er = __shfl_sync(0xffffffffu, r, 0);
+    ez = __shfl_sync(0xffffffffu, r, 16);
+}
+
+// Perturbation field of this lane's point (rho, z) where leaf >= 0, the warp
+// taking its lanes' points one after another.
+__device__ __forceinline__ void map_field_lanes(const double* map, int leaf, double rho, double z, double& er,
+                                                double& ez) {
+    const int lane = threadIdx.x & 31;
+    for (unsigned m = __ballot_sync(0xffffffffu, leaf >= 0); m; m &= m - 1) {
+        const int j = __ffs(m) - 1;
+        double fr, fz;
+        map_field(map, __shfl_sync(0xffffffffu, leaf, j), __shfl_sync(0xffffffffu, rho, j),
+                  __shfl_sync(0xffffffffu, z, j), fr, fz);
+        if (lane == j) {
+            er = fr;
+            ez = fz;
+        }
+    }
+}
+
+// E_rho at (x, y) turned into (E_x, E_y)
+__device__ __forceinline__ void rotate_rho(double x, double y, double rho, double e_rho, double& ex, double& ey) {
+    ex = ey = 0.0;
+    if (rho != 0.0) {
+        ex = e_rho * (x / rho);
+        ey = e_rho * (y / rho);
+    }
 }
 
 constexpr int kWarpRuns = kWarpChunk / SPT_BLOCK_SEGS;
@@ -904,7 +998,7 @@ __device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& f
         const double va = MIX ? warp_sum((double)sa[p]) : 0.0;
         if (lane == 0 && p < np_) {
             const int k = r0 + p;
-            const double er = vr + P[8 * k + 7], ez = vz + c.fld[3 * k + 2];
+            const double er = vr + P[8 * k + 7], ez = vz + c.ntmp[3 * k + 2];
             P[8 * k + 5] = er;
             P[8 * k + 6] = ez;
             if (MIX) {
@@ -928,7 +1022,7 @@ __device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& f
 __device__ __forceinline__ void closest_point(Ctx& c, int k, bool frame) {
     const SptBem& b = c.bem;
     const int lane = threadIdx.x & 31;
-    double* P = c.bpt;  // record k: [0]x [1]y [2]z [3]rho_e [4]z_e [5]ax [6]ay [7]near_r ; near_z in fld tmp
+    double* P = c.bpt;  // record k: [0]x [1]y [2]z [3]rho_e [4]z_e [5]ax [6]ay [7]near_r ; near_z in ntmp
     const int nseg = b.n_seg;
     {
         const double x = P[8 * k + 0], y = P[8 * k + 1], z = P[8 * k + 2];
@@ -1026,7 +1120,7 @@ static __device__ void bem_closest(Ctx& c, int n, bool frame) {
 
 // B for one record k, by one warp: the near-segment sinh quadrature
 // (bem/axisymmetric.py:566-600); lane 0 ends with near_r in record slot 7 and
-// near_z in fld[3k + 2].
+// near_z in ntmp[3k + 2].
 __device__ __forceinline__ void near_point(Ctx& c, int k, unsigned long long& n_near, unsigned long long& n_ring_near) {
     const SptBem& b = c.bem;
     const int lane = threadIdx.x & 31;
@@ -1081,7 +1175,7 @@ __device__ __forceinline__ void near_point(Ctx& c, int k, unsigned long long& n_
         acc_z = warp_sum(acc_z);
         if (lane == 0) {
             P[8 * k + 7] = acc_r;
-            c.fld[3 * k + 2] = acc_z;  // temporary near_z (fld is rewritten after the far sum)
+            c.ntmp[3 * k + 2] = acc_z;
         }
     }
 }
@@ -1132,9 +1226,25 @@ __device__ __forceinline__ void bem_sums(Ctx& c, int n, int* status_flag) {
     const int nseg = b.n_seg;
     const int nps = b.nodes_per_seg;
     if (n <= 0) return;
+    // Adaptive rule with a field map: the map gives the points its cells hold
+    // (phases B and C then leave them out).
+    const double* const map = FAR == SPT_FAR_ADAPTIVE ? field_map(b) : nullptr;
+    auto mapped = [&](int k) { return map && map_find(map, P[8 * k + 3], P[8 * k + 4]) >= 0; };
     // B: near-segment sinh quadrature (one warp per point)
     unsigned long long n_near = 0, n_ring_near = 0;
-    for (int k = warp; k < n; k += c.nw) near_point(c, k, n_near, n_ring_near);
+    for (int k = warp; k < n; k += c.nw) {
+        if (mapped(k)) {
+            double er, ez;
+            map_field(map, map_find(map, P[8 * k + 3], P[8 * k + 4]), P[8 * k + 3], P[8 * k + 4], er, ez);
+            if (lane == 0) {
+                P[8 * k + 5] = er;
+                P[8 * k + 6] = ez;
+                atomicAdd(c.cnt + SPT_CNT_CLUSTER_EVALS, 1ull);
+            }
+        } else {
+            near_point(c, k, n_near, n_ring_near);
+        }
+    }
     count_add(c, SPT_CNT_NEAR_PAIRS, n_near);
     count_add(c, SPT_CNT_RING_NEAR, n_ring_near);
     __syncthreads();
@@ -1152,7 +1262,8 @@ __device__ __forceinline__ void bem_sums(Ctx& c, int n, int* status_flag) {
         if (tid == 0) s_far_task = c.nw;
         __syncthreads();
         unsigned long long cl_evals = 0;
-        for (int k = warp; k < n; k = next_task(&s_far_task)) far_point<FORM>(c, k, far_evals, cl_evals);
+        for (int k = warp; k < n; k = next_task(&s_far_task))
+            if (!mapped(k)) far_point<FORM>(c, k, far_evals, cl_evals);
         count_add(c, SPT_CNT_CLUSTER_EVALS, cl_evals);
         __syncthreads();
     } else {
@@ -1592,23 +1703,50 @@ __device__ void stage_accel(Ctx& c, double* out, int* status_flag) {
 
     // 1. external field
     if (KIND == SPT_GEOM_TIP_BEM || KIND == SPT_GEOM_WELL_BEM || KIND == SPT_GEOM_POST_BEM) {
-        // compact the particles that need the BEM sum into c.list (stable order)
+        // Field map (float64 adaptive form): warp w takes particles w, w + nw,
+        // ... (one per lane, spread over all warps of a small group), the
+        // mapped ones are evaluated here and the rest compacted into c.list;
+        // without a map every particle that needs the field is listed.
+        const double* map = nullptr;
+        if constexpr (FORM == SPT_FORM_FP64 && FAR == SPT_FAR_ADAPTIVE) map = field_map(c.bem);
+        for (int i = tid; i < 3 * E; i += c.nt) c.fld[i] = 0.0;
         __shared__ int s_wcount[kMaxWarps + 1];
         int n_list = 0;
         for (int base = 0; base < E; base += c.nt) {
-            const int i = base + tid;
+            const int i = map ? base + (tid >> 5) + c.nw * (tid & 31) : base + tid;
             bool need = false;
+            double rho = 0.0, zi = 0.0;
             if (i < E && c.live[i]) {
                 const double x = sx[i], y = sy[i], z = sz[i];
                 need = bem_valid<KIND>(x, y, z, g) && blend_weight(z, g.z_handoff) > 0.0;
+                if (map && need) {
+                    rho = hypot(x, y);
+                    zi = z;
+                }
+            }
+            bool mapped = false;
+            double mx = 0.0, my = 0.0, mz = 0.0;
+            if (map) {
+                const int leaf = need ? map_find(map, rho, zi) : -1;
+                mapped = leaf >= 0;
+                double er = 0.0;
+                map_field_lanes(map, leaf, rho, zi, er, mz);
+                if (mapped) rotate_rho(sx[i], sy[i], rho, er, mx, my);
+                need = need && !mapped;
+                count_add(c, SPT_CNT_CLUSTER_EVALS, mapped ? 1ull : 0ull);
             }
             const unsigned bal = __ballot_sync(0xffffffffu, need);
             if ((tid & 31) == 0) s_wcount[tid >> 5] = __popc(bal);
-            __syncthreads();
+            __syncthreads();  // also: every zero of c.fld is written before a field
             if (tid == 0) {
                 int acc = 0;
                 for (int w = 0; w < c.nw; ++w) { const int t = s_wcount[w]; s_wcount[w] = acc; acc += t; }
                 s_wcount[c.nw] = acc;
+            }
+            if (mapped) {
+                c.fld[3 * i + 0] = mx;
+                c.fld[3 * i + 1] = my;
+                c.fld[3 * i + 2] = mz;
             }
             __syncthreads();
             if (need) {
@@ -1622,19 +1760,18 @@ __device__ void stage_accel(Ctx& c, double* out, int* status_flag) {
             __syncthreads();
         }
         if (n_list > 0) {
+            c.ntmp = map ? c.img : c.fld;
             if constexpr (FORM == SPT_FORM_SURROGATE)
                 surrogate_points<FAR>(c, n_list, status_flag);
             else
                 bem_points<FORM, FAR>(c, n_list, false, status_flag);
-        }
-        // scatter: fld[i] = blended field
-        for (int i = tid; i < E; i += c.nt) { c.fld[3 * i + 0] = 0.0; c.fld[3 * i + 1] = 0.0; c.fld[3 * i + 2] = 0.0; }
-        __syncthreads();
-        for (int k = tid; k < n_list; k += c.nt) {
-            const int i = c.list[k];
-            c.fld[3 * i + 0] = c.bpt[8 * k + 5];
-            c.fld[3 * i + 1] = c.bpt[8 * k + 6];
-            c.fld[3 * i + 2] = c.bpt[8 * k + 7];
+            // scatter: fld[i] = blended field
+            for (int k = tid; k < n_list; k += c.nt) {
+                const int i = c.list[k];
+                c.fld[3 * i + 0] = c.bpt[8 * k + 5];
+                c.fld[3 * i + 1] = c.bpt[8 * k + 6];
+                c.fld[3 * i + 2] = c.bpt[8 * k + 7];
+            }
         }
         __syncthreads();
     }
@@ -2345,14 +2482,48 @@ struct WarpTeam {
     }
 };
 
+// Direct field of the point (x, y, z) by this warp (closest segment, near
+// quadrature, adaptive far sum, rotation); lane 0 returns it.  Uses the
+// warp's own record c.bpt and near sum c.ntmp.
+struct PointCounts {
+    unsigned long long n_near = 0, n_ring_near = 0, far_evals = 0, cl_evals = 0;
+};
+
+template <int FORM>
+__device__ __forceinline__ void direct_point(Ctx& c, double x, double y, double z, PointCounts& n, double& ex,
+                                             double& ey, double& ez) {
+    double* const P = c.bpt;
+    if ((threadIdx.x & 31) == 0) {
+        P[0] = x;
+        P[1] = y;
+        P[2] = z;
+    }
+    __syncwarp();
+    closest_point(c, 0, false);
+    __syncwarp();
+    near_point(c, 0, n.n_near, n.n_ring_near);
+    __syncwarp();
+    far_point<FORM>(c, 0, n.far_evals, n.cl_evals);
+    __syncwarp();
+    rotate_rho(x, y, hypot(x, y), P[5], ex, ey);
+    ez = P[6];
+    __syncwarp();
+}
+
+__device__ __forceinline__ void count_points(Ctx& c, const PointCounts& n) {
+    count_add(c, SPT_CNT_NEAR_PAIRS, n.n_near);
+    count_add(c, SPT_CNT_RING_NEAR, n.n_ring_near);
+    count_add(c, SPT_CNT_RING_FAR, n.far_evals);
+    count_add(c, SPT_CNT_CLUSTER_EVALS, n.cl_evals);
+}
+
 // The CTA's BEM task pool of one stage: entries (warp << 5 | particle),
 // drawn one per warp task; every warp calls, between the barriers that close
 // the appends and open the next stage.
 template <int FORM>
-__device__ __forceinline__ void pool_bem_points(Ctx& c, double* smem, const int* entries, int count, int* next) {
+__device__ __forceinline__ void pool_bem_points(Ctx& c, double* smem, const int* entries, int count, int* next,
+                                                PointCounts& n) {
     const int lane = threadIdx.x & 31;
-    double* const P = c.bpt;
-    unsigned long long n_near = 0, n_ring_near = 0, far_evals = 0, cl_evals = 0;
     for (;;) {
         int t = 0;
         if (lane == 0) t = atomicAdd(next, 1);
@@ -2361,37 +2532,15 @@ __device__ __forceinline__ void pool_bem_points(Ctx& c, double* smem, const int*
         const int e = entries[t];
         const WarpTeam own(smem, c.nw, e >> 5);
         const int k = e & 31;
+        double ex, ey, ez;
+        direct_point<FORM>(c, own.sx[k], own.sy[k], own.sz[k], n, ex, ey, ez);
         if (lane == 0) {
-            P[0] = own.sx[k];
-            P[1] = own.sy[k];
-            P[2] = own.sz[k];
-        }
-        __syncwarp();
-        closest_point(c, 0, false);
-        __syncwarp();
-        near_point(c, 0, n_near, n_ring_near);
-        __syncwarp();
-        far_point<FORM>(c, 0, far_evals, cl_evals);
-        __syncwarp();
-        if (lane == 0) {  // rotation to (x, y), as bem_points_fused
-            const double x = P[0], y = P[1];
-            const double rho = hypot(x, y);
-            const double e_rho = P[5];
-            double ex = 0.0, ey = 0.0;
-            if (rho != 0.0) {
-                ex = e_rho * (x / rho);
-                ey = e_rho * (y / rho);
-            }
             own.fld[3 * k + 0] = ex;
             own.fld[3 * k + 1] = ey;
-            own.fld[3 * k + 2] = P[6];
+            own.fld[3 * k + 2] = ez;
         }
         __syncwarp();
     }
-    count_add(c, SPT_CNT_NEAR_PAIRS, n_near);
-    count_add(c, SPT_CNT_RING_NEAR, n_ring_near);
-    count_add(c, SPT_CNT_RING_FAR, far_evals);
-    count_add(c, SPT_CNT_CLUSTER_EVALS, cl_evals);
 }
 
 // The rest of a stage for this warp's group, after the pool: images, pair
@@ -2487,11 +2636,11 @@ trace_warp_kernel(const __grid_constant__ SptState st, const __grid_constant__ S
     static_assert(FORM == SPT_FORM_FP64, "the warp team runs the float64 form");
     extern __shared__ __align__(16) double smem[];
     __shared__ unsigned long long s_cnt[SPT_N_COUNTERS];
-    __shared__ int s_pool[2][kMaxThreads];  // two stages' task pools, used alternately
-    __shared__ int s_pool_n[2], s_pool_next[2];
+    __shared__ int s_pool[3][kMaxThreads];  // three stages' task pools, used in turn
+    __shared__ int s_pool_n[3], s_pool_next[3];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int k = threadIdx.x; k < SPT_N_COUNTERS; k += blockDim.x) s_cnt[k] = 0;
-    if (threadIdx.x < 2) s_pool_n[threadIdx.x] = s_pool_next[threadIdx.x] = 0;
+    if (threadIdx.x < 3) s_pool_n[threadIdx.x] = s_pool_next[threadIdx.x] = 0;
     Ctx c(geo, bem);
     c.cm = prm.charge_to_mass;
     c.kc = prm.coulomb_constant;
@@ -2504,7 +2653,9 @@ trace_warp_kernel(const __grid_constant__ SptState st, const __grid_constant__ S
     c.tiles = smem;  // far-rule scratch of every warp (far_adaptive_warp takes its own by warp index)
     const WarpTeam w(smem, nw, warp);
     c.bpt = w.rec;
-    c.fld = w.nfld;
+    c.fld = c.ntmp = w.nfld;
+    const double* const map = field_map(bem);
+    PointCounts pts;
     c.live = w.live;
     double* const slot = slots + ((size_t)blockIdx.x * nw + warp) * kWarpSlotDoubles + lane;
     auto ld = [&](int k) { return __ldcg(slot + 32 * k); };
@@ -2534,7 +2685,7 @@ trace_warp_kernel(const __grid_constant__ SptState st, const __grid_constant__ S
         }
         have = false;
     };
-    int tick = 0;  // stages taken by the CTA (the pool parity)
+    int pp = 0;  // the current stage's pool
     for (;;) {
         // ready this warp's group for an attempt: take groups from the work
         // queue until one is running and within this call's attempt budget
@@ -2618,8 +2769,7 @@ trace_warp_kernel(const __grid_constant__ SptState st, const __grid_constant__ S
         c.E = E;
         const bool live = run && in && (t >= tb) && (t < td);
         // seven stage evaluations (batched_rk45.py:326-370), in step across the CTA
-        for (int s = 0; s < 7; ++s, ++tick) {
-            const int pp = tick & 1;
+        for (int s = 0; s < 7; ++s, pp = pp == 2 ? 0 : pp + 1) {
             double px = 0.0, py = 0.0, pz = 0.0;
             bool need = false;
             if (run) {
@@ -2665,22 +2815,45 @@ trace_warp_kernel(const __grid_constant__ SptState st, const __grid_constant__ S
                 w.sz[lane] = pz;
                 w.live[lane] = live;
                 // the BEM field of the live particles inside the valid region
-                // with blend weight > 0 goes to the CTA's pool
+                // with blend weight > 0: mapped points here, by their own
+                // warp, the others to the CTA's pool
                 need = live && bem_valid<KIND>(px, py, pz, geo) && blend_weight(pz, geo.z_handoff) > 0.0;
-                const unsigned m = __ballot_sync(0xffffffffu, need);
+                bool direct = need;
+                if (map) {
+                    const double rho = need ? hypot(px, py) : 0.0;
+                    const int leaf = need ? map_find(map, rho, pz) : -1;
+                    double er = 0.0, ez = 0.0;
+                    map_field_lanes(map, leaf, rho, pz, er, ez);
+                    if (leaf >= 0) {
+                        direct = false;
+                        double ex, ey;
+                        rotate_rho(px, py, rho, er, ex, ey);
+                        w.fld[3 * lane + 0] = ex;
+                        w.fld[3 * lane + 1] = ey;
+                        w.fld[3 * lane + 2] = ez;
+                        ++pts.cl_evals;
+                    }
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, direct);
                 int at = 0;
                 if (lane == 0 && m) at = atomicAdd(&s_pool_n[pp], __popc(m));
                 at = __shfl_sync(0xffffffffu, at, 0);
-                if (need) s_pool[pp][at + __popc(m & ((1u << lane) - 1u))] = (warp << 5) | lane;
+                if (direct) s_pool[pp][at + __popc(m & ((1u << lane) - 1u))] = (warp << 5) | lane;
             }
             __syncthreads();
-            // the other pool is free until the next stage's appends, which follow the barrier below
+            // The pool after next was last read before this barrier and is
+            // next appended to after the next stage's: cleared in between, so
+            // a stage without direct points needs no second barrier.
             if (threadIdx.x == 0) {
-                s_pool_n[pp ^ 1] = 0;
-                s_pool_next[pp ^ 1] = 0;
+                const int p2 = pp == 0 ? 2 : pp - 1;
+                s_pool_n[p2] = 0;
+                s_pool_next[p2] = 0;
             }
-            pool_bem_points<FORM>(c, smem, s_pool[pp], s_pool_n[pp], &s_pool_next[pp]);
-            __syncthreads();
+            const int n_direct = s_pool_n[pp];
+            if (n_direct > 0) {  // alike in every thread
+                pool_bem_points<FORM>(c, smem, s_pool[pp], n_direct, &s_pool_next[pp], pts);
+                __syncthreads();
+            }
             if (run) {
                 double ax, ay, az;
                 stage_finish_warp<KIND>(c, w, live, need, px, py, pz, mi, ax, ay, az);
@@ -2766,6 +2939,7 @@ trace_warp_kernel(const __grid_constant__ SptState st, const __grid_constant__ S
         if (isnan(err)) status = SPT_GROUP_NONFINITE;
         ++att;
     }
+    count_points(c, pts);
     __syncthreads();
     flush_counters(c, prm.counters);
 }

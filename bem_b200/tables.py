@@ -22,6 +22,9 @@ Built once per geometry, like the reference's per-device field cache
   of each whole run.  A run is flagged for it only when it is straight and,
   at probe points RATIO_RUN arclengths away, its 8-point sum matches the
   segment-wise Gauss-4 sum to RUN_TOL;
+* field map (field_map.py): the field as polynomials over cells of a quadtree,
+  built on the GPU at the first adaptive view, for the adaptive rule's
+  float64 form.  Not in the reference;
 * cluster table [n_cluster, CLUSTER_TERMS + 2]: a binary tree over the runs
   (level l: clusters of 2^l consecutive runs) with, per cluster, its centre
   on the axis, its radius and the axisymmetric multipole moments of its
@@ -30,6 +33,7 @@ Built once per geometry, like the reference's per-device field cache
 """
 
 import ctypes
+import threading
 
 import numpy as np
 
@@ -281,6 +285,8 @@ class BemTables:
             ct, levels = cluster_tables(self.profile, self.sigma, self.n_subdiv)
             self.clusters = torch.as_tensor(np.ascontiguousarray(ct), device=device)
             self.cluster_levels = levels
+        self._map = None          # (doubles, SptBem.reserved) of the field map, or False: none
+        self._map_lock = threading.Lock()
         self.struct = _lib.SptBem()
         s = self.struct
         s.n_seg = n_seg
@@ -316,13 +322,35 @@ class BemTables:
         self.image = solution
         self.struct.image = solution.struct
 
+    def field_map(self):
+        """(doubles, SptBem.reserved) of the field map, built on first use, or
+        None: no clusters or CUDA device, nothing to map, no memory for it,
+        or the current stream is being captured (the direct sums then serve;
+        a later view outside the capture builds it)."""
+        import torch
+        if self.clusters is None or self.seg.device.type != "cuda":
+            return None
+        with self._map_lock:
+            if self._map is None:
+                if torch.cuda.is_current_stream_capturing():
+                    return None
+                from . import field_map
+                try:
+                    self._map = field_map.build(self) or False
+                except torch.cuda.OutOfMemoryError:
+                    self._map = False
+            return self._map or None
+
     def view(self, far_rule="reference", ratio4=RATIO4, ratio2=RATIO2, ratio_run=RATIO_RUN, bounds=True,
-             cluster_kappa=None):
+             cluster_kappa=None, field_map=True):
         """An SptBem over these tables with the given far rule (the tables
         must outlive it); ratio_run <= 0 turns the run rule off; bounds=False
         leaves out the run bounds, so every per-point scan visits every
         segment (and the run rule and the clusters are off);
-        cluster_kappa <= 0 turns the cluster expansions off."""
+        cluster_kappa <= 0 turns the cluster expansions off.  The adaptive
+        rule at its default thresholds takes the field map with it
+        (field_map=False leaves it out): other thresholds ask for the sums
+        they describe."""
         v = _lib.SptBem()
         ctypes.pointer(v)[0] = self.struct
         v.far_rule = _lib.FAR_RULES[far_rule] if isinstance(far_rule, str) else int(far_rule)
@@ -332,6 +360,11 @@ class BemTables:
         if not bounds:
             v.blk, v.blk_stride = None, 0
             v.clusters, v.cluster_kappa = None, 0.0
+        if (field_map and bounds and v.far_rule == _lib.FAR_ADAPTIVE
+                and (v.ratio4, v.ratio2, v.ratio_run, v.cluster_kappa) == (RATIO4, RATIO2, RATIO_RUN, CLUSTER_KAPPA)):
+            m = self.field_map()
+            if m is not None:
+                v.clusters, v.reserved = m[0].data_ptr(), m[1]
         return v
 
     @property

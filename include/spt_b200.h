@@ -82,7 +82,7 @@ extern "C" {
 #define SPT_CNT_FP64_TARGETS 9       /* mixed form: pair-sum targets recomputed in float64 */
 #define SPT_CNT_LIVE_STEPS 10        /* sum over accepted group-steps of the particles alive (born, not
                                         killed) at the step start */
-#define SPT_CNT_CLUSTER_EVALS 11     /* cluster-expansion evaluations of the adaptive far rule */
+#define SPT_CNT_CLUSTER_EVALS 11     /* expansions evaluated by the adaptive far rule: clusters, and points of the field map */
 #define SPT_N_COUNTERS 12
 
 /* Geometry parameters.  Fields a kind does not use are ignored. */
@@ -155,6 +155,11 @@ typedef struct {
      * 6 nodes per segment: the 4 Gauss-4 nodes, then the 2 Gauss-2 nodes.
      * ratio4 >= 1 (coarse segments are never near), ratio2 >= ratio4. */
     int32_t far_rule;
+    /* 0, or SPT_MAP_TAG << 16 | u: a field map (spt_map_cells) starts u *
+     * SPT_MAP_UNIT doubles after `clusters`.  The float64 form of the adaptive
+     * far rule reads the field of the points its cells hold from it; the
+     * other points, forms and rule sum directly.  The map stands for the
+     * field itself: it takes precedence over the thresholds below. */
     int32_t reserved;
     double ratio4;
     double ratio2;
@@ -207,6 +212,25 @@ typedef struct {
 #define SPT_TRACE_IMAGE_MODES 16
 
 #define SPT_MAX_CLUSTER_RUNS 256
+
+/* Field map of a BEM solution (no counterpart in the reference): square cells
+ * of a quadtree over the (rho, z) half plane that hold the perturbation field
+ * as polynomials of SPT_MAP_N coefficients in each coordinate.  Layout, in
+ * doubles: a header of SPT_MAP_HEADER (1 / side of the root square, its lowest
+ * z, the offset of the cell records; its lowest rho is 0), int32 tables of 64
+ * entries (three quadtree levels each, entry 8 * z index + rho index: a cell's
+ * number, -1 for none, or -2 - the number of the next table), then one record
+ * of SPT_MAP_REC per cell: centre rho, centre z, 1 / half-width, 5 unused, and
+ * coefficient (component c, rho power i, z power j) at 8 + (2 j + c) *
+ * SPT_MAP_N + i. */
+#define SPT_MAP_TAG 0x4d50u
+#define SPT_MAP_UNIT 64
+#define SPT_MAP_HEADER 8
+#define SPT_MAP_N 12
+#define SPT_MAP_REC (8 + 2 * SPT_MAP_N * SPT_MAP_N)
+/* a cell keeps this many panel lengths from each panel: the quadrature changes
+ * at one length, and at two its own error is far below rounding */
+#define SPT_MAP_BAND 2.0
 
 #define SPT_RUN_NODES 8
 
@@ -372,6 +396,25 @@ int spt_compact_groups(const int32_t* order, int32_t n, const int32_t* status, i
  * (x, y, z) -> (ex, ey, ez), all [n] device arrays. */
 int spt_bem_field(const double* x, const double* y, const double* z, int64_t n, const SptBem* bem,
                   int32_t form, double* ex, double* ey, double* ez, void* stream);
+
+/* Candidate cells of a field map: cells [n, 3] holds centre rho, centre z and
+ * half-width.  flag[k] = 1: the cell is SPT_MAP_BAND panel lengths from every
+ * panel and its centre at least `kappa` half-widths from the surface, so it can
+ * be sampled; 0: it must be divided first; 2: it lies in the band, on the
+ * conductor's side of the surface, or is small against the panels near it: no
+ * map there.  far[k]: distance of the centre to the surface / half-width. */
+int spt_map_classify(const double* cells, int32_t n, const SptBem* bem, double kappa, int32_t* flag,
+                     double* far_ratio, void* stream);
+
+/* Samples the field of each candidate cell at its SPT_MAP_N x SPT_MAP_N
+ * Chebyshev points (adaptive far rule with bem's thresholds, which must be
+ * without a map; no panel may be near) and writes the cell's record, and
+ * tail[k] = its largest Chebyshev coefficient of the two highest orders over
+ * its largest one.  cheb: the SPT_MAP_N nodes; dct [N, N]: values at the nodes
+ * to Chebyshev coefficients; mono [N, N]: mono[k * N + i] = coefficient of
+ * power i in T_k. */
+int spt_map_cells(const double* cells, int32_t n, const SptBem* bem, const double* cheb, const double* dct,
+                  const double* mono, double* rec, double* tail, void* stream);
 
 /* Learned-form perturbation field at n points: the surrogate MLP (sur_*
  * fields of `sur`; the other fields are ignored) outside sur_band metres of

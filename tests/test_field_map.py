@@ -1,0 +1,59 @@
+"""Lookup tables of the field map (bem_b200/field_map.py): every point of a
+cell finds it, points outside every cell find none (CPU; the walk below is
+the device's map_find)."""
+
+import numpy as np
+import pytest
+
+from bem_b200 import field_map as fm
+
+
+def _find(tab, u, v):
+    iu, iv, node = int(u * 2**30), int(v * 2**30), 0
+    for sh in range(27, -1, -3):
+        e = tab[node, ((iv >> sh) & 7) * 8 + ((iu >> sh) & 7)]
+        if e >= -1:
+            return e
+        node = -2 - e
+    return -1
+
+
+@pytest.mark.parametrize("depth", [1, 2, 3, 4, 7, 12])
+def test_link_tables_find_every_cell(depth):
+    rng = np.random.default_rng(depth)
+    i = j = np.zeros(1, dtype=np.int64)
+    divided, cells = {}, []
+    for level in range(depth + 1):
+        split = np.ones(len(i), bool) if level == 0 else rng.random(len(i)) < (0.55 if level < depth else 0.0)
+        for a, b in zip(i[~split], j[~split]):
+            if rng.random() < 0.8:  # the rest: squares without a cell
+                cells.append((level, a, b))
+        i, j = i[split][:40], j[split][:40]
+        if len(i) == 0:
+            break
+        divided[level] = (i, j)
+        i, j = (np.concatenate([2 * i + a for a in (0, 1) for _ in (0, 1)]),
+                np.concatenate([2 * j + b for _ in (0, 1) for b in (0, 1)]))
+    level, ci, cj = (np.array(c, dtype=np.int64) for c in zip(*cells))
+    tab = fm.link_tables((level, ci, cj, np.arange(len(cells))), divided)
+    for k, (l, a, b) in enumerate(cells):
+        for fu, fv in ((0.0, 0.0), (0.5, 0.5), (1 - 1e-4, 0.0), (0.3, 1 - 1e-4)):
+            assert _find(tab, (a + fu) / 2.0**l, (b + fv) / 2.0**l) == k
+    taken = {}
+    for l, a, b in cells:
+        taken.setdefault(l, set()).add((a, b))
+    for u, v in rng.random((200, 2)):
+        hit = any((int(u * 2**l), int(v * 2**l)) in s for l, s in taken.items())
+        assert (_find(tab, u, v) >= 0) == hit
+
+
+def test_power_coefficients_reproduce_the_samples():
+    """Nodes -> Chebyshev -> powers, evaluated back at the nodes: the products
+    of 12-term rows leave a few rounding errors of the largest value."""
+    rng = np.random.default_rng(0)
+    x = fm.NODES
+    f = np.exp(x[:, None] * 0.7) * np.cos(x[None, :] + 0.2) + rng.normal(size=(fm.N, fm.N)) * 1e-15
+    c = fm.DCT @ f @ fm.DCT.T
+    p = fm.MONO.T @ c @ fm.MONO
+    V = x[:, None] ** np.arange(fm.N)
+    assert np.abs(V @ p @ V.T - f).max() < 1e-13

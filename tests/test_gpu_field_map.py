@@ -1,0 +1,94 @@
+"""The field map against the reference quadrature and the direct sums, where it can go wrong:
+cell edges and corners, the band's edge, outside the root square, remainders
+of the kernel's chunks, and non-finite points."""
+
+import ctypes
+
+import numpy as np
+import pytest
+
+from conftest import load_golden
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("needs a CUDA device", allow_module_level=True)
+
+from bem_b200 import _lib, engine  # noqa: E402
+from bem_b200.tables import BemTables  # noqa: E402
+
+
+def _direct(tab, pts):
+    v = tab.view("adaptive", field_map=False)
+    x, y, z = (torch.as_tensor(np.ascontiguousarray(pts[:, k]), device="cuda") for k in range(3))
+    e = [torch.empty_like(x) for _ in range(3)]
+    _lib.check(_lib.lib().spt_bem_field(x.data_ptr(), y.data_ptr(), z.data_ptr(), len(pts), ctypes.byref(v), 0,
+                                        e[0].data_ptr(), e[1].data_ptr(), e[2].data_ptr(),
+                                        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "spt_bem_field")
+    return torch.stack(e, -1).cpu().numpy()
+
+
+def _cells(tab):
+    m, tag = tab.field_map()
+    m = m[(tag & 0xFFFF) * _lib.MAP_UNIT:].cpu().numpy()
+    rec = m[int(m[2]):].reshape(-1, _lib.MAP_REC)
+    return rec[:, 0], rec[:, 1], 1.0 / rec[:, 2]
+
+
+@pytest.mark.parametrize("fixture", ["bem_sphere", "bem_well", "bem_post", "sigma_c1", "sigma_c3"])
+def test_map_matches_reference_quadrature_at_cell_edges(fixture):
+    """Corners, edge midpoints and centres of cells of every size, a rounding
+    error inside and outside: 2e-12 of the larger of the cell's field and the
+    uniform one (the adaptive rule's 1e-12 bound, twice, as the samples are
+    its sums with tighter thresholds; the truncation, 2e-14, is far below).
+    Against the reference quadrature; points an edge leaves without a cell
+    are the direct sums bit for bit (at their default thresholds those are
+    themselves 3e-12 off it in places of the 3000-panel well)."""
+    g = load_golden(fixture)
+    tab = BemTables(g["profile"], g["sigma"], int(g["n_subdiv"]) if "n_subdiv" in g else 8)
+    rc, zc, h = _cells(tab)
+    rng = np.random.default_rng(1)
+    pick = rng.choice(len(rc), min(len(rc), 400), replace=False)
+    fr = np.array([-1, 1, -1, 1, 0, 0, -1, 1, 0]) * (1 + np.array([0, 0, 1, 1, 0, 0, 1, -1, 0]) * 1e-9)
+    fz = np.array([-1, -1, 1, 1, 0, -1, 0, 0, 1]) * (1 - np.array([0, 1, 0, 1, 0, 1, 0, 0, -1]) * 1e-9)
+    rho = np.abs(rc[pick, None] + h[pick, None] * fr)
+    z = zc[pick, None] + h[pick, None] * fz
+    ph = rng.uniform(0, 2 * np.pi, rho.shape)
+    pts = np.stack([rho * np.cos(ph), rho * np.sin(ph), z], -1).reshape(-1, 3)
+    got, ref = engine.bem_field(tab, pts, far_rule="adaptive").cpu().numpy(), engine.bem_field(tab, pts).cpu().numpy()
+    norm = np.linalg.norm(ref, axis=-1).reshape(rho.shape).max(axis=1, keepdims=True)
+    uniform = np.abs(float(g["E_gun"])) if "E_gun" in g else np.linalg.norm(ref, axis=-1).max()
+    err = np.abs(got - ref).max(axis=-1).reshape(rho.shape)
+    direct = np.all(got == _direct(tab, pts), axis=-1).reshape(rho.shape)
+    assert direct[:, 4].mean() < 0.05  # the cells did take part: every centre (column 4) lies in one
+    assert (err / np.maximum(norm, uniform))[~direct].max() < 2e-12
+
+
+def test_chunks_and_band_leave_each_point_its_value():
+    """A point's value does not depend on the points beside it or on their
+    number (chunks of 8 to 256, a remainder in each), near the surface or in
+    a cell; and other thresholds than the map's are the direct sums."""
+    g = load_golden("sigma_c1")
+    tab = BemTables(g["profile"], g["sigma"], 8)
+    rng = np.random.default_rng(2)
+    n = 5 * 148 * 2 * 8 + 3
+    d, th = 10 ** rng.uniform(-10, -6, n), rng.uniform(0, 1.2, n)
+    pts = np.stack([(50e-9 + d) * np.sin(th), np.zeros(n), 5e-6 + (50e-9 + d) * np.cos(th)], -1)
+    whole = engine.bem_field(tab, pts, far_rule="adaptive")
+    for a, b in ((0, 1), (1, 8), (8, 17), (100, 357), (357, 357 + 2369), (3000, n)):
+        assert torch.equal(engine.bem_field(tab, pts[a:b], far_rule="adaptive"), whole[a:b])
+    assert tab.view("adaptive").reserved >> 16 == _lib.MAP_TAG
+    for kw in (dict(ratio4=9.0), dict(ratio2=200.0), dict(ratio_run=5.0), dict(cluster_kappa=0.0), dict(bounds=False)):
+        assert tab.view("adaptive", **kw).reserved == 0
+    assert tab.view("reference").reserved == 0
+
+
+def test_points_without_a_cell():
+    """Outside the root square, and non-finite: the direct path's results."""
+    g = load_golden("bem_sphere")
+    tab = BemTables(g["profile"], g["sigma"], int(g["n_subdiv"]))
+    nan, inf = float("nan"), float("inf")
+    pts = np.array([[1.0, 0, 0], [0, 0, -5.0], [0, 0, 7.0], [nan, 0, 0], [0, nan, 1e-6], [0, 0, nan], [inf, 0, 0],
+                    [0, 0, inf], [0, 0, -inf]])
+    np.testing.assert_array_equal(engine.bem_field(tab, pts, far_rule="adaptive").cpu().numpy(), _direct(tab, pts))
