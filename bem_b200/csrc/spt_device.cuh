@@ -563,19 +563,23 @@ __device__ void far_round(Ctx& c, int r0, int np_, int n_tiles, int segs_per_til
                         }
                     }
                 } else {
+                // a point's NQ terms are added first: one step of the running sum's chain for all of them
 #pragma unroll
                 for (int p = 0; p < NP; ++p) {
+                    double tr_ = 0.0, tz_ = 0.0;
 #pragma unroll
                     for (int j = 0; j < NQ; ++j) {
                         if (p < np_ && in[j] && !c.nflag[p * 256 + sl[j]]) {
                             const double dz = pz[p] - zq[j];
                             double er, ez;
                             ring_field_far(pr[p], pinv[p], dz, rq[j], er, ez);
-                            ar[p] = fma(wq[j], er, ar[p]);
-                            az[p] = fma(wq[j], ez, az[p]);
+                            tr_ = fma(wq[j], er, tr_);
+                            tz_ = fma(wq[j], ez, tz_);
                             ++far_evals;
                         }
                     }
+                    ar[p] += tr_;
+                    az[p] += tz_;
                 }
                 }
             }
