@@ -315,12 +315,12 @@ __device__ __forceinline__ void count_add(Ctx& c, int k, unsigned long long v) {
 }
 
 __device__ inline void bind(Ctx& c, double* smem, int E, int far_rule, double* slot, unsigned long long* s_cnt,
-                            bool sur = false) {
+                            bool sur = false, bool tiles = true) {
     c.base = smem;
     c.E = E;
     c.nt = blockDim.x;
     c.nw = blockDim.x >> 5;
-    c.L = make_layout(E, far_rule, sur, true, blockDim.x >> 5, image_scratch(c.g, c.bem, E, blockDim.x));
+    c.L = make_layout(E, far_rule, sur, tiles, blockDim.x >> 5, image_scratch(c.g, c.bem, E, blockDim.x));
     c.round_pts = kRound;
     c.kappa = kKappa;
     c.cnt = s_cnt;
@@ -1697,7 +1697,9 @@ static __device__ __noinline__ void stage_image_force(Ctx& c) {
                                                  &s_imgflag);
 }
 
-template <int KIND, int FORM, int FAR>
+// GIVEN: the BEM perturbation field of every particle that takes one is in
+// c.fld already (spt_accel's first pass).
+template <int KIND, int FORM, int FAR, bool GIVEN = false>
 __device__ void stage_accel(Ctx& c, double* out, int* status_flag) {
     const int E = c.E, tid = threadIdx.x;
     const double* sx = c.sp;
@@ -1706,7 +1708,7 @@ __device__ void stage_accel(Ctx& c, double* out, int* status_flag) {
     const SptGeometry& g = c.g;
 
     // 1. external field
-    if (KIND == SPT_GEOM_TIP_BEM || KIND == SPT_GEOM_WELL_BEM || KIND == SPT_GEOM_POST_BEM) {
+    if constexpr (!GIVEN && (KIND == SPT_GEOM_TIP_BEM || KIND == SPT_GEOM_WELL_BEM || KIND == SPT_GEOM_POST_BEM)) {
         // Field map (float64 adaptive form): warp w takes particles w, w + nw,
         // ... (one per lane, spread over all warps of a small group), the
         // mapped ones are evaluated here and the rest compacted into c.list;
@@ -2389,8 +2391,9 @@ trace_kernel(const __grid_constant__ SptState st, const __grid_constant__ SptTra
     if constexpr (sur) release_surrogate(c);
 }
 
-// one stage evaluation per group (spt_accel), one CTA per group
-template <int KIND, int FORM, int FAR>
+// one stage evaluation per group (spt_accel), one CTA per group; GIVEN: ax, ay,
+// az hold the perturbation field (of the particles that take one) on entry
+template <int KIND, int FORM, int FAR, bool GIVEN>
 __global__ void __launch_bounds__(kMaxThreads, 2)
 accel_kernel(const __grid_constant__ SptAccelArgs a, const __grid_constant__ SptGeometry geo,
              const __grid_constant__ SptBem bem) {
@@ -2404,7 +2407,7 @@ accel_kernel(const __grid_constant__ SptAccelArgs a, const __grid_constant__ Spt
     c.kc = a.coulomb_constant;
     c.soft2 = a.plummer_radius * a.plummer_radius;
     const int Emax = a.max_group_size;
-    bind(c, smem, Emax, FAR, nullptr, s_cnt);
+    bind(c, smem, Emax, FAR, nullptr, s_cnt, false, !GIVEN);
     init_barriers(c);
     const long long base = a.group_offset[g];
     const int E = (int)(a.group_offset[g + 1] - base);
@@ -2417,10 +2420,15 @@ accel_kernel(const __grid_constant__ SptAccelArgs a, const __grid_constant__ Spt
         c.live[i] = a.active[base + i];
         c.q[i] = a.charge[base + i];
         c.m[i] = a.mass[base + i];
+        if constexpr (GIVEN) {
+            c.fld[3 * i + 0] = a.ax[base + i];
+            c.fld[3 * i + 1] = a.ay[base + i];
+            c.fld[3 * i + 2] = a.az[base + i];
+        }
     }
     __syncthreads();
     double* out = c.kv;  // slope storage is free on this path (groups here are at most kSmallGroup)
-    stage_accel<KIND, FORM, FAR>(c, out, &s_flag);
+    stage_accel<KIND, FORM, FAR, GIVEN>(c, out, &s_flag);
     for (int i = tid; i < E; i += c.nt) {
         a.ax[base + i] = out[i];
         a.ay[base + i] = out[E + i];
@@ -2966,6 +2974,19 @@ struct TraceLaunch {
     bool warp_team;              // one group per warp (trace_warp_kernel), slope slots at `slots`
 };
 
+// Which points a field launch (spt_field.cu) evaluates: points 0 .. n-1
+// (active NULL), or of the particles group_offset[0] .. group_offset[n_groups]
+// - 1, at most n, the active ones in the geometry's valid region below its
+// handoff.
+struct FieldMask {
+    const uint8_t* active;
+    const int64_t* group_offset;
+    int n_groups;
+    SptGeometry g;
+};
+int launch_field(const double* x, const double* y, const double* z, long long n, const SptBem& b,
+                 const FieldMask& mask, double* ex, double* ey, double* ez, cudaStream_t st);
+
 // Shared memory and grid of a trace launch; returns 0 or a cudaError_t.
 template <int KIND, int FORM, int FAR>
 int trace_grid(int max_group_size, int threads, int n_groups, long long max_slots, int img_doubles, size_t* smem,
@@ -3019,15 +3040,31 @@ int trace_launch(const TraceLaunch& t, int grid, size_t smem) {
     return (int)cudaGetLastError();
 }
 
-template <int KIND, int FORM, int FAR>
+template <int KIND, int FORM, int FAR, bool GIVEN = false>
 int accel_launch(const SptAccelArgs* a, const SptGeometry* g, const SptBem& bem, cudaStream_t stream) {
-    const Layout L = make_layout(a->max_group_size, FAR, false, true, kMaxWarps,
+    const Layout L = make_layout(a->max_group_size, FAR, false, !GIVEN, kMaxWarps,
                                  image_scratch(*g, bem, a->max_group_size, kMaxThreads));
-    auto kern = accel_kernel<KIND, FORM, FAR>;
+    auto kern = accel_kernel<KIND, FORM, FAR, GIVEN>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.bytes);
     if (e != cudaSuccess) return (int)e;
     kern<<<a->n_groups, kMaxThreads, L.bytes, stream>>>(*a, *g, bem);
     return (int)cudaGetLastError();
+}
+
+// The float64 form of a BEM geometry in two launches: the field of all
+// particles at once into ax, ay, az -- one point a warp or a point split over
+// several, whatever fills the SMs, where one CTA per group leaves them idle
+// for few groups and waits for its slowest point for many -- then the groups'
+// pair sums.  Either far rule: only the first launch depends on it.
+template <int KIND>
+int accel_launch_split(const SptAccelArgs* a, const SptGeometry* g, const SptBem& bem, cudaStream_t stream) {
+    const FieldMask mask{a->active, a->group_offset, a->n_groups, *g};
+    const long long most = (long long)a->n_groups * a->max_group_size;
+    const long long n = a->n_particles > 0 && a->n_particles < most ? a->n_particles : most;
+    const int e = launch_field(a->x, a->y, a->z, n, bem, mask, a->ax, a->ay, a->az, stream);
+    if (e == -1) return (int)cudaErrorInvalidValue;
+    if (e) return e;
+    return accel_launch<KIND, SPT_FORM_FP64, SPT_FAR_REFERENCE, true>(a, g, bem, stream);
 }
 
 // Trace dispatch over the (form, far rule) instantiations of one geometry
@@ -3075,10 +3112,7 @@ int accel_dispatch(const SptAccelArgs* a, const SptGeometry* g, const SptBem& be
     constexpr bool kBem = KIND == SPT_GEOM_TIP_BEM || KIND == SPT_GEOM_WELL_BEM || KIND == SPT_GEOM_POST_BEM;
     const int far = kBem ? bem.far_rule : SPT_FAR_REFERENCE;
     if constexpr (kBem) {
-        if (a->form == SPT_FORM_FP64 && far == SPT_FAR_REFERENCE)
-            return accel_launch<KIND, SPT_FORM_FP64, SPT_FAR_REFERENCE>(a, g, bem, stream);
-        if (a->form == SPT_FORM_FP64 && far == SPT_FAR_ADAPTIVE)
-            return accel_launch<KIND, SPT_FORM_FP64, SPT_FAR_ADAPTIVE>(a, g, bem, stream);
+        if (a->form == SPT_FORM_FP64) return accel_launch_split<KIND>(a, g, bem, stream);
         if (a->form == SPT_FORM_MIXED && far == SPT_FAR_REFERENCE)
             return accel_launch<KIND, SPT_FORM_MIXED, SPT_FAR_REFERENCE>(a, g, bem, stream);
         if (a->form == SPT_FORM_MIXED && far == SPT_FAR_ADAPTIVE)

@@ -64,80 +64,6 @@ bem_field_kernel(const double* x, const double* y, const double* z, long long n,
     flush_counters(c, counters);
 }
 
-// The same in the float64 adaptive form: a CTA takes `chunk` points (8 to
-// 256: one a warp while there are few).  Every thread finds its point's cell
-// of the field map; mapped points are evaluated by the warp they sit in, the
-// others (near the surface, or no map) go to a task list that all warps of the
-// CTA draw from, one warp a point.
-template <int FORM>
-__global__ void __launch_bounds__(kMaxThreads, 2)
-field_points_kernel(const double* x, const double* y, const double* z, long long n, int chunk,
-                    const __grid_constant__ SptBem bem, double* ex, double* ey, double* ez) {
-    extern __shared__ __align__(16) double smem[];
-    __shared__ SptGeometry s_geo;
-    __shared__ double s_p[3 * kMaxThreads];
-    __shared__ int s_task[kMaxThreads];
-    __shared__ int s_n, s_next;
-    __shared__ unsigned long long s_cnt[SPT_N_COUNTERS];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) s_n = s_next = 0;
-    __syncthreads();
-    Ctx c(s_geo, bem);
-    c.nt = kMaxThreads;
-    c.nw = kMaxWarps;
-    c.cnt = s_cnt;
-    c.tiles = smem;
-    c.bpt = smem + kMaxWarps * kWarpScratchInts / 2 + 12 * warp;
-    c.fld = c.ntmp = c.bpt + 8;
-    const double* const map = field_map(bem);
-    // point of this thread: lane + 32 warp of a full chunk, fewer lanes a warp in a small one
-    const int per_warp = chunk / kMaxWarps;
-    const long long i = blockIdx.x * (long long)chunk + warp * per_warp + lane;
-    const bool in = lane < per_warp && i < n;
-    double px = 0.0, py = 0.0, pz = 0.0;
-    int leaf = -1;
-    if (in) {
-        px = x[i];
-        py = y[i];
-        pz = z[i];
-    }
-    if (map) {
-        const double rho = hypot(px, py);
-        if (in) leaf = map_find(map, rho, pz);
-        double er = 0.0, fx, fy, fz = 0.0;
-        map_field_lanes(map, leaf, rho, pz, er, fz);
-        if (leaf >= 0) {
-            rotate_rho(px, py, rho, er, fx, fy);
-            ex[i] = fx;
-            ey[i] = fy;
-            ez[i] = fz;
-        }
-    }
-    if (in && leaf < 0) {
-        s_p[tid] = px;
-        s_p[kMaxThreads + tid] = py;
-        s_p[2 * kMaxThreads + tid] = pz;
-        s_task[atomicAdd(&s_n, 1)] = tid;
-    }
-    __syncthreads();
-    const int n_direct = s_n;
-    PointCounts pts;
-    for (;;) {
-        const int t = next_task(&s_next);
-        if (t >= n_direct) break;
-        const int k = s_task[t];
-        double fx, fy, fz;
-        direct_point<FORM>(c, s_p[k], s_p[kMaxThreads + k], s_p[2 * kMaxThreads + k], pts, fx, fy, fz);
-        if (lane == 0) {
-            const long long o = blockIdx.x * (long long)chunk + (k >> 5) * per_warp + (k & 31);
-            ex[o] = fx;
-            ey[o] = fy;
-            ez[o] = fz;
-        }
-        __syncwarp();
-    }
-}
-
 // learned-form field at arbitrary points (spt_surrogate_field): 128 points
 // (one MLP tile) per CTA, through the stage kernel's surrogate_points
 constexpr int kSurChunk = 128;
@@ -687,19 +613,10 @@ int spt_bem_field(const double* x, const double* y, const double* z, int64_t n, 
                                                                                        nullptr);                  \
         return cuda_check(cudaGetLastError(), "bem_field_kernel launch");                                         \
     }
-    if (form == SPT_FORM_FP64 && far == SPT_FAR_REFERENCE) SPT_FIELD(SPT_FORM_FP64, SPT_FAR_REFERENCE)
     if (form == SPT_FORM_FP64) {
-        // chunks of 8 points (one a warp) until two CTAs on each SM are full, then larger ones
-        long long chunk = 8 * ((n + 148LL * 2 * 8 - 1) / (148LL * 2 * 8));
-        if (chunk > spt::kMaxThreads) chunk = spt::kMaxThreads;
-        const size_t smem = spt::kMaxWarps * (spt::kWarpScratchInts * 4 + 12 * 8);
-        const long long grid = (n + chunk - 1) / chunk;
-        if (grid > 0x7fffffffLL) return fail(SPT_ERR_CAPACITY, "too many points");
-        rc = set_smem(spt::field_points_kernel<SPT_FORM_FP64>, smem);
-        if (rc) return rc;
-        spt::field_points_kernel<SPT_FORM_FP64><<<(unsigned)grid, spt::kMaxThreads, smem, st>>>(x, y, z, n, (int)chunk, *b,
-                                                                                            ex, ey, ez);
-        return cuda_check(cudaGetLastError(), "field_points_kernel launch");
+        rc = spt::launch_field(x, y, z, n, *b, spt::FieldMask{}, ex, ey, ez, st);
+        if (rc == -1) return fail(SPT_ERR_CAPACITY, "too many points");
+        return cuda_check((cudaError_t)rc, "field kernel launch");
     }
     if (far == SPT_FAR_REFERENCE) SPT_FIELD(SPT_FORM_MIXED, SPT_FAR_REFERENCE)
     SPT_FIELD(SPT_FORM_MIXED, SPT_FAR_ADAPTIVE)

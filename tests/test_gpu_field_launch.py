@@ -1,0 +1,94 @@
+"""Field launches (spt_field.cu) where their work split can go wrong: point
+counts that give 1 to 64 shares a point, panel counts and sub-panels that leave
+remainders, masked and ragged groups, an offset table that starts above 0."""
+
+import ctypes
+
+import numpy as np
+import pytest
+
+from conftest import load_golden
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("needs a CUDA device", allow_module_level=True)
+
+from bem_b200 import _lib, engine  # noqa: E402
+from bem_b200.tables import BemTables  # noqa: E402
+from oracle import bem as ob  # noqa: E402
+
+import gpu_util as gu  # noqa: E402
+
+
+@pytest.mark.parametrize("n_subdiv", [1, 3, 8])
+@pytest.mark.parametrize("panels", [5, 32, 33, 97, 600])
+def test_reference_rule_at_every_share_count(panels, n_subdiv):
+    """n points of a sphere's field, against the oracle: summation order only,
+    ~sqrt(19200) roundings of terms some ten times the field, and the oracle's
+    own: 1e-11 as the parity tests of this rule."""
+    th = np.linspace(0, np.pi, panels + 1)
+    prof = np.stack([np.sin(th), np.cos(th)], -1) * 1e-6
+    prof[0, 0] = prof[-1, 0] = 0.0
+    sig = 3e7 * np.cos(th)
+    tab = BemTables(prof, sig, n_subdiv)
+    rng = np.random.default_rng(panels)
+    d, ang, ph = 10 ** rng.uniform(-2, 1, 9600), rng.uniform(0.01, np.pi, 9600), rng.uniform(0, 6.28, 9600)
+    r = 1e-6 * (1 + d)
+    pts = np.stack([r * np.sin(ang) * np.cos(ph), r * np.sin(ang) * np.sin(ph), r * np.cos(ang)], -1)
+    ref = ob.field(pts[:40], prof, sig, n_subdiv)
+    for n in (1, 2, 7, 40, 151, 1200, 9600):
+        got = engine.bem_field(tab, pts[:n]).cpu().numpy()[:40]
+        m = len(got)
+        assert (np.abs(got - ref[:m]).max(axis=-1) / np.linalg.norm(ref[:m], axis=-1)).max() < 1e-11
+
+
+def _geometry(kind):
+    g = load_golden(dict(post="trace_post", well="trace_well")[kind])
+    spec = dict(kind=kind + "_bem", E_gun=float(g["E_gun"]), R=float(g["R"]), profile=g["profile"], sigma=g["sigma"],
+                n_subdiv=int(g["n_subdiv"]), z_handoff=float(g["z_handoff"]), kill_z_below=0.0)
+    spec.update(dict(L=float(g["L"]), z0=float(g["z0"])) if kind == "post" else dict(H=float(g["H"])))
+    return gu.device_geometry(spec)
+
+
+@pytest.mark.parametrize("rule", ["reference", "adaptive"])
+@pytest.mark.parametrize("kind", ["post", "well"])
+def test_stage_of_ragged_groups_is_its_groups_alone(kind, rule):
+    """Groups of 1, 2, 31, 33 and 256 in one call, with inactive particles,
+    particles inside the conductor and above the handoff, against each group's
+    own call (other shares a point: 1e-12 of each acceleration), and through
+    an offset table that starts at the second group with n_particles left 0."""
+    geo = _geometry(kind)
+    sizes = [1, 2, 31, 33, 256]
+    n = sum(sizes)
+    rng = np.random.default_rng(4)
+    R = geo.R
+    top = geo.L if kind == "post" else 0.0
+    pos = np.stack([rng.uniform(-R, R, n), rng.uniform(-R, R, n), top + R * 10 ** rng.uniform(-3, 0.5, n)], -1)
+    pos[::7, 2] = -2.0 * R if kind == "well" else 0.5 * top       # inside the conductor (mostly)
+    pos[::11, 2] = 1.1 * geo.z_handoff
+    act = (rng.random(n) < 0.7).astype(np.uint8)
+    q, m = np.full(n, gu.Q_E), np.full(n, gu.M_E)
+    whole = engine.accel(geo, pos, act, q, m, sizes, gu.CM, 1e-12, far_rule=rule).cpu().numpy()
+    assert np.all(whole[act == 0] == 0.0)
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    for a, b in zip(off[:-1], off[1:]):
+        one = engine.accel(geo, pos[a:b], act[a:b], q[a:b], m[a:b], [b - a], gu.CM, 1e-12, far_rule=rule).cpu().numpy()
+        np.testing.assert_allclose(whole[a:b], one, rtol=0, atol=1e-12 * np.linalg.norm(one, axis=-1).max())
+    t = lambda v, d=torch.float64: torch.as_tensor(np.ascontiguousarray(v), dtype=d, device="cuda")
+    x, y, z, tq, tm = t(pos[:, 0]), t(pos[:, 1]), t(pos[:, 2]), t(q), t(m)
+    ta, to = t(act, torch.uint8), t(off, torch.int64)
+    out = torch.full((3, n), 7.0, dtype=torch.float64, device="cuda")
+    a = _lib.SptAccelArgs()
+    a.n_groups, a.max_group_size = len(sizes) - 1, 256
+    a.group_offset = to.data_ptr() + 8
+    a.x, a.y, a.z, a.active, a.charge, a.mass = (v.data_ptr() for v in (x, y, z, ta, tq, tm))
+    a.charge_to_mass, a.coulomb_constant, a.plummer_radius = gu.CM, engine.COULOMB_CONSTANT, 1e-12
+    a.ax, a.ay, a.az = (out[k].data_ptr() for k in range(3))
+    view, s = geo.bem_tables("cuda").view(rule), geo.to_struct()
+    _lib.check(_lib.lib().spt_accel(ctypes.byref(a), ctypes.byref(s), ctypes.byref(view),
+                                    ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "spt_accel")
+    got = out.T.cpu().numpy()
+    np.testing.assert_array_equal(got[:1], 7.0)
+    np.testing.assert_allclose(got[1:], whole[1:], rtol=0, atol=1e-12 * np.linalg.norm(whole, axis=-1).max())
