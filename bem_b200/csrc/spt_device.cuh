@@ -1034,36 +1034,50 @@ __device__ __forceinline__ void closest_point(Ctx& c, int k, bool frame) {
         double best = INFINITY;
         int bs = 0x7fffffff;
         if (b.blk) {
+            const int nblk = (nseg + SPT_BLOCK_SEGS - 1) / SPT_BLOCK_SEGS;
+            // The on-surface offset below needs a distance under 1e-9 of the
+            // closest segment's length.  Where no segment is within 1e-8 of its
+            // length (runs out of reach by their rigorous bounds, the others'
+            // segments one by one), the closest segment plays no further part,
+            // and the evaluation point is the point itself -- the offset path's
+            // rho + 0 and z + 0 bit for bit (z = 0 excepted: there the sign of
+            // the zero would follow the normal).
+            if (!frame && z != 0.0) {
+                bool hit = false;
+                for (int q0 = 0; q0 < nblk; q0 += 32) {
+                    const bool cand = q0 + lane < nblk &&
+                                      !(blk_lower(b, q0 + lane, rho, z) > 1e-8 * blk_lmax(b, q0 + lane));
+                    for (unsigned cm = __ballot_sync(0xffffffffu, cand); cm; cm &= cm - 1) {
+                        const int s = (q0 + __ffs(cm) - 1) * SPT_BLOCK_SEGS + lane;
+                        double proj, dist;
+                        if (s < nseg) {
+                            seg_near(b, s, rho, z, proj, dist);
+                            hit |= !(dist > 1e-8 * segf(b, 4, s));
+                        }
+                    }
+                }
+                if (!__any_sync(0xffffffffu, hit)) {
+                    if (lane == 0) {
+                        P[8 * k + 3] = rho;
+                        P[8 * k + 4] = z;
+                    }
+                    return;
+                }
+            }
             // the run with the smallest lower bound gives an upper bound of the
             // minimum; only runs whose lower bound does not exceed it are scanned
             // (each lane still takes its segments in increasing order)
-            const int nblk = (nseg + SPT_BLOCK_SEGS - 1) / SPT_BLOCK_SEGS;
-            double lbm = INFINITY, lmx = 0.0;
+            double lbm = INFINITY;
             int qm = 0;
             for (int q = lane; q < nblk; q += 32) {
                 const double lb = blk_lower(b, q, rho, z);
                 if (lb < lbm) { lbm = lb; qm = q; }
-                lmx = fmax(lmx, blk_lmax(b, q));
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 const double ol = __shfl_xor_sync(0xffffffffu, lbm, o);
                 const int oq = __shfl_xor_sync(0xffffffffu, qm, o);
                 if (ol < lbm || (ol == lbm && oq < qm)) { lbm = ol; qm = oq; }
-                lmx = fmax(lmx, __shfl_xor_sync(0xffffffffu, lmx, o));
-            }
-            // Every segment at least 2e-9 x the longest segment away (the run
-            // bounds are rigorous lower bounds): the on-surface offset below
-            // (distance^2 < (1e-9 L)^2) cannot apply, the closest segment
-            // plays no further part, and the evaluation point is the point
-            // itself -- the offset path's rho + 0 and z + 0 bit for bit (z = 0
-            // excepted: there the sign of the zero would follow the normal).
-            if (!frame && z != 0.0 && lbm > 2e-9 * lmx) {
-                if (lane == 0) {
-                    P[8 * k + 3] = rho;
-                    P[8 * k + 4] = z;
-                }
-                return;
             }
             double ub = INFINITY;
             if (qm * SPT_BLOCK_SEGS + lane < nseg) ub = seg_dist2(b, qm * SPT_BLOCK_SEGS + lane, rho, z);
@@ -1132,6 +1146,7 @@ __device__ __forceinline__ void near_point(Ctx& c, int k, unsigned long long& n_
     const int nseg = b.n_seg;
     {
         const double re = P[8 * k + 3], ze = P[8 * k + 4];
+        const double inv = re > 0.0 ? 1.0 / re : 0.0;
         double acc_r = 0.0, acc_z = 0.0;
         const int nblk = (nseg + SPT_BLOCK_SEGS - 1) / SPT_BLOCK_SEGS;
         for (int q0 = 0; q0 < nblk; q0 += 32) {
@@ -1146,30 +1161,37 @@ __device__ __forceinline__ void near_point(Ctx& c, int k, unsigned long long& n_
             double proj = 0.0, dist = 0.0;
             const bool nr = (s < nseg) && seg_near(b, s, re, ze, proj, dist);
             unsigned mask = __ballot_sync(0xffffffffu, nr);
+            // the sinh map's limits and intervals, by every near segment's lane at once
+            double lo = 0.0, hi = 0.0;
+            if (nr) {
+                const double Ls = segf(b, 4, s);
+                dist = fmax(dist, 1e-15 * Ls);
+                lo = asinh(-proj / dist);
+                hi = asinh((Ls - proj) / dist);
+            }
             while (mask) {
                 const int j = __ffs(mask) - 1;
                 mask &= mask - 1;
                 const int sg = s0 + j;
-                const double sp = __shfl_sync(0xffffffffu, proj, j);
-                const double Ls = segf(b, 4, sg);
-                const double d = fmax(__shfl_sync(0xffffffffu, dist, j), 1e-15 * Ls);
-                const double lo = asinh(-sp / d), hi = asinh((Ls - sp) / d);
-                const int cnt = max(1, (int)ceil((hi - lo) / 0.5));
-                const double width = (hi - lo) / cnt;
-                const double half = 0.5 * (hi - lo) / cnt;
+                const double sp = __shfl_sync(0xffffffffu, proj, j), d = __shfl_sync(0xffffffffu, dist, j);
+                const double v0 = __shfl_sync(0xffffffffu, lo, j), span = __shfl_sync(0xffffffffu, hi, j) - v0;
+                const int cnt = max(1, (int)ceil(span / 0.5));
+                const double width = span / cnt, half = 0.5 * width;
+                const double iL = 1.0 / segf(b, 4, sg);
                 const double p0r = segf(b, 0, sg), p0z = segf(b, 1, sg), ur = segf(b, 5, sg), uz = segf(b, 6, sg);
-                const double sg0 = segf(b, 9, sg), sg1 = segf(b, 10, sg);
+                const double sg0 = segf(b, 9, sg), dsg = (segf(b, 10, sg) - sg0) * iL;
                 for (int qn = lane; qn < cnt * 8; qn += 32) {
                     const int iv = qn >> 3, gi = qn & 7;
-                    const double v = lo + (iv + 0.5 * (b.gauss8_x[gi] + 1.0)) * width;
-                    const double sl = sp + d * sinh(v);
-                    const double sr = p0r + sl * ur, sz = p0z + sl * uz;
-                    const double dens = sg0 + (sl / Ls) * (sg1 - sg0);
-                    const double w = dens * (2.0 * kPi * sr) * d * cosh(v) * half * b.gauss8_w[gi];
+                    // sinh and cosh of the node from one exponential: sinh's rounding is 1e-16 of d, and
+                    // the node is at least d from the point
+                    const double ev = exp(fma(iv + 0.5 * (b.gauss8_x[gi] + 1.0), width, v0)), em = rcp_pos(ev);
+                    const double sl = fma(0.5 * d, ev - em, sp);
+                    const double sr = fma(sl, ur, p0r), sz = fma(sl, uz, p0z);
+                    const double w = fma(sl, dsg, sg0) * (2.0 * kPi * sr) * (0.5 * d * (ev + em)) * half * b.gauss8_w[gi];
                     double er, ez;
-                    ring_field(re, ze - sz, sr, er, ez);
-                    acc_r += w * er;
-                    acc_z += w * ez;
+                    ring_field_far<true>(re, inv, ze - sz, sr, er, ez);
+                    acc_r = fma(w, er, acc_r);
+                    acc_z = fma(w, ez, acc_z);
                 }
                 if (lane == 0) { n_near += 1; n_ring_near += (unsigned long long)cnt * 8; }
             }

@@ -128,10 +128,37 @@ static __device__ __noinline__ void ring_axis_taylor(double rho, double z, doubl
     ez = z / (4.0 * kPi * ax15) + 3.0 * rho2 * z * (3.0 * a2 - 2.0 * z2) / (16.0 * kPi * ax35);
 }
 
-// Ring field close to the ring (p = d2 / D < 1e-3), out of line: rare in a far
-// sum, and on another path than every interleaved evaluation.
-static __device__ __noinline__ void ring_close(double rho, double z, double a, double& er, double& ez) {
-    ring_field(rho, z, a, er, ez);
+// a^2 - rho^2 + z^2 in the reference's rounding (bem/axisymmetric.py:262): near
+// a surface it cancels to ~(rho - a) rho, and its rounding (1e-13 of the field
+// at 10 pm) is part of what traces of ill-conditioned particles reproduce.
+__device__ __forceinline__ double ring_a(double rho, double z2, double a) {
+    return __dadd_rn(__dadd_rn(__dmul_rn(a, a), -__dmul_rn(rho, rho)), z2);
+}
+
+// Ring field close to the ring (p = d2 / D < 1e-3): the DLMF 19.12 series (of
+// which six terms leave 1e-19 there), one reciprocal for every quotient.
+__device__ __forceinline__ void ring_close(double rho, double inv_rho, double a, double z, double D, double d2,
+                                           double& er, double& ez) {
+    const double inv = rcp_pos(D * d2), inv_d2 = D * inv, p = d2 * (d2 * inv);
+    const double L = -0.5 * log(p);
+    auto h6 = [&](const double* c) {
+        double v = c[5];
+#pragma unroll
+        for (int n = 4; n >= 0; --n) v = fma(v, p, c[n]);
+        return v;
+    };
+    const double K = fma(L, h6(kSerK), h6(kSerKd));
+    const double E = fma(0.5 * p, fma(L, h6(kSerE), h6(kSerEd)), 1.0);
+    const double g = sqrt_pos(d2 * inv) * (1.0 / (4.0 * kPi * kPi));  // 1 / (4 pi^2 sqrt(D))
+    er = fma(-ring_a(rho, __dmul_rn(z, z), a) * inv_d2, E, K) * (g * inv_rho);
+    ez = 2.0 * z * E * inv_d2 * g;
+}
+
+// The same out of line: rare in a far sum, and on another path than every
+// interleaved evaluation.
+static __device__ __noinline__ void ring_close_cold(double rho, double inv_rho, double a, double z, double D,
+                                                    double d2, double& er, double& ez) {
+    ring_close(rho, inv_rho, a, z, D, d2, er, ez);
 }
 
 // Ring field for the far-quadrature sum, 1/rho supplied by the caller (constant
@@ -148,6 +175,7 @@ static __device__ __noinline__ void ring_close(double rho, double z, double a, d
 // either).  Five square roots and one reciprocal, against eight and two of the
 // AGM run to convergence on d2 / D: the far sums are bound by these
 // instructions (96 M rings of one 1500-point call: 11.4 -> 6.7 ms).
+template <bool NEAR = false>
 __device__ __forceinline__ void ring_field_far(double rho, double inv_rho, double z, double a, double& er,
                                                double& ez) {
     const double z2 = z * z, s = rho + a, t = rho - a;
@@ -157,7 +185,8 @@ __device__ __forceinline__ void ring_field_far(double rho, double inv_rho, doubl
         return;
     }
     if (d2 < 1e-3 * D) {
-        ring_close(rho, z, a, er, ez);
+        if constexpr (NEAR) ring_close(rho, inv_rho, a, z, D, d2, er, ez);
+        else ring_close_cold(rho, inv_rho, a, z, D, d2, er, ez);
         return;
     }
     const double r1 = sqrt_pos(D), r2 = sqrt_pos(d2);
@@ -174,7 +203,8 @@ __device__ __forceinline__ void ring_field_far(double rho, double inv_rho, doubl
     S = fma(fma(0.25, e2, 2.0) * t4, t4, S);
     const double Q = (D - S) * (inv * m);
     const double F = im * fma(e2, fma(e2, 9.0 / 64.0, 0.25), 1.0);
-    er = fma(-fma(-s, t, z2), Q, 1.0) * (F * inv_rho * (1.0 / (8.0 * kPi)));  // a^2 - rho^2 = -(rho + a)(rho - a)
+    const double A = NEAR ? ring_a(rho, __dmul_rn(z, z), a) : fma(-s, t, z2);  // a^2 - rho^2 = -(rho + a)(rho - a)
+    er = fma(-A, Q, 1.0) * (F * inv_rho * (1.0 / (8.0 * kPi)));
     ez = z * Q * (F * (1.0 / (4.0 * kPi)));
 }
 

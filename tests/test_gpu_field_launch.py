@@ -92,3 +92,33 @@ def test_stage_of_ragged_groups_is_its_groups_alone(kind, rule):
     got = out.T.cpu().numpy()
     np.testing.assert_array_equal(got[:1], 7.0)
     np.testing.assert_allclose(got[1:], whole[1:], rtol=0, atol=1e-12 * np.linalg.norm(whole, axis=-1).max())
+
+
+def test_on_surface_offset_around_its_threshold():
+    """Points 0 to a few 1e-8 panel lengths from a panel, both sides (the
+    offset acts below 1e-9, the scan that skips it from 1e-8), with the run
+    bounds and without (every segment scanned): the same bits."""
+    g = load_golden("sigma_c1")
+    prof = g["profile"]
+    tab = BemTables(prof, g["sigma"], 8)
+    rows = []
+    for k in (3, 60, 99, 100, 500):
+        t = prof[k + 1] - prof[k]
+        L = np.hypot(*t)
+        nrm = np.array([-t[1], t[0]]) / L
+        for f in (0.0, 0.3e-9, 0.999e-9, 1.001e-9, 3e-9, 0.99e-8, 1.01e-8, 5e-8, 1e-3, 0.5):
+            for u in (0.0, 0.4, 1.0):
+                p = prof[k] + u * t + f * L * nrm
+                rows += [[p[0], 0.0, p[1]], [0.6 * p[0], 0.8 * p[0], p[1]]]
+    pts = np.array(rows)
+    x, y, z = (torch.as_tensor(np.ascontiguousarray(pts[:, k]), device="cuda") for k in range(3))
+    out = []
+    for bounds in (True, False):
+        view = tab.view("reference", bounds=bounds)
+        e = [torch.empty_like(x) for _ in range(3)]
+        _lib.check(_lib.lib().spt_bem_field(x.data_ptr(), y.data_ptr(), z.data_ptr(), len(pts), ctypes.byref(view), 0,
+                                            e[0].data_ptr(), e[1].data_ptr(), e[2].data_ptr(),
+                                            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "spt_bem_field")
+        out.append(torch.stack(e, -1).cpu().numpy())
+    assert np.isfinite(out[0]).all()
+    np.testing.assert_array_equal(out[0], out[1])
