@@ -185,13 +185,15 @@ struct Layout {
     bool big;                 // slopes/y0/nw in global memory
 };
 
-// Segments per chunk of the adaptive far rule (8 runs of SPT_BLOCK_SEGS).
-// Each warp classifies and sums its own rounds in a private scratch of
-// kWarpScratchInts ints: three segment lists of kWarpChunk entries, the
-// near masks of the first (kWarpChunk bytes) and four run lists.
+// The adaptive far rule classifies 32 runs of SPT_BLOCK_SEGS segments at a time
+// (a lane each) and the segments of up to kWarpChunk / SPT_BLOCK_SEGS of them
+// before their nodes are summed.  Each warp keeps its lists in a private
+// scratch of kWarpScratchInts ints: four segment lists and the near masks of
+// the first (kWarpChunk bytes each: a segment by its place among the runs at
+// hand), four run lists and the bits of the runs that cluster expansions cover.
 constexpr int kWarpChunk = 256;
-constexpr int kWarpScratchInts = 3 * kWarpChunk + kWarpChunk / 4 + 4 * (kWarpChunk / SPT_BLOCK_SEGS) +
-                                  SPT_MAX_CLUSTER_RUNS / 32;
+constexpr int kWarpRuns = 32;
+constexpr int kWarpScratchInts = 5 * kWarpChunk / 4 + 4 * kWarpRuns + SPT_MAX_CLUSTER_RUNS / 32;
 static_assert(kWarpScratchInts % 2 == 0, "per-warp scratch keeps 8-byte alignment");
 
 // Shared-memory layout of one CTA for groups of up to E particles.  The far
@@ -572,7 +574,7 @@ __device__ void far_round(Ctx& c, int r0, int np_, int n_tiles, int segs_per_til
                         if (p < np_ && in[j] && !c.nflag[p * 256 + sl[j]]) {
                             const double dz = pz[p] - zq[j];
                             double er, ez;
-                            ring_field_far(pr[p], pinv[p], dz, rq[j], er, ez);
+                            ring_field_far<false, false>(pr[p], pinv[p], dz, rq[j], er, ez);
                             tr_ = fma(wq[j], er, tr_);
                             tz_ = fma(wq[j], ez, tz_);
                             ++far_evals;
@@ -765,8 +767,17 @@ __device__ __forceinline__ void rotate_rho(double x, double y, double rho, doubl
     }
 }
 
-constexpr int kWarpRuns = kWarpChunk / SPT_BLOCK_SEGS;
-static_assert(kWarpRuns <= 32, "one lane classifies each run of a chunk");
+// Gauss-8 nodes of each whole panel (rho, z, w rows), kept with the field map:
+// panels PANEL8_FROM to PANEL8_TO x ratio4 lengths away.  At two lengths its
+// error (8.1^-16) is that of the reference's 32 sub-panel nodes, at a quarter
+// of the ring evaluations; up to twice ratio4 it replaces the whole-panel
+// Gauss-4, whose error at ratio4 = 8 (32^-8, 1e-12) is the adaptive rule's
+// largest.
+constexpr double kPanel8From = 2.0, kPanel8To = 2.0;
+__device__ __forceinline__ const double* panel8(const SptBem& b) {
+    const double* map = field_map(b);
+    return map ? map + (size_t)__ldg(map + 3) : nullptr;
+}
 
 template <int NP, int NQ, bool MIX>
 __device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& far_evals,
@@ -776,9 +787,9 @@ __device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& f
     const int nseg = b.n_seg, nps = b.nodes_per_seg;
     double* P = c.bpt;
     int* scratch = reinterpret_cast<int*>(c.tiles) + warp * kWarpScratchInts;
-    int* lists = scratch;                                                    // L0 | L1 | L2, kWarpChunk each
-    unsigned char* mask = reinterpret_cast<unsigned char*>(scratch + 3 * kWarpChunk);  // near masks of L0
-    int* R2 = scratch + 3 * kWarpChunk + kWarpChunk / 4;
+    unsigned char* lists = reinterpret_cast<unsigned char*>(scratch);  // L0 | L1 | L2 | L8, kWarpChunk each
+    unsigned char* mask = lists + 4 * kWarpChunk;                      // near masks of L0
+    int* R2 = scratch + 5 * kWarpChunk / 4;
     int* R3 = R2 + kWarpRuns;
     int* M = R3 + kWarpRuns;
     int* Mcls = M + kWarpRuns;
@@ -813,7 +824,8 @@ __device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& f
         const int nt = b.cluster_terms, rec_len = nt + 2;
         // the covering clusters' heads, listed first (the segment lists are free
         // until the chunk loop) and then expanded in one lane-parallel pass
-        int* const heads = lists;
+        int* const heads = scratch;
+        static_assert(SPT_MAX_CLUSTER_RUNS <= kWarpChunk, "the heads fit the segment lists");
         int n_heads = 0;
         for (int qb = 0; qb < n_run; qb += 32) {
             const int q = qb + lane;
@@ -848,12 +860,16 @@ __device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& f
         }
         __syncwarp();
     }
-    for (int c0 = 0; c0 < nseg; c0 += kWarpChunk) {
-        const int q0 = c0 / SPT_BLOCK_SEGS;
-        const int nr = min(kWarpRuns, (nseg - c0 + SPT_BLOCK_SEGS - 1) / SPT_BLOCK_SEGS);
+    const double* p8 = panel8(b);
+    const double* p8r = p8;
+    const double* p8z = p8 + 8 * (size_t)nseg;
+    const double* p8w = p8 + 16 * (size_t)nseg;
+    // the segment tests read ratio4 as the distance from which whole-panel Gauss-4 serves
+    const double r4s = p8 ? kPanel8To * r4 : r4;
+    for (int q0 = 0; q0 < n_run; q0 += kWarpRuns) {
         const int q = q0 + lane;
-        int cls = -1;  // 3 run rule, 2 Gauss-2 on every segment, 1 no near segment, 0 full test
-        if (lane < nr && !(use_cl && ((covered[q >> 5] >> (q & 31)) & 1u))) {
+        int cls = -1;  // 3 run rule, 2 Gauss-2 on every segment, 1 no segment below ratio4, 0 full test
+        if (q < n_run && !(use_cl && ((covered[q >> 5] >> (q & 31)) & 1u))) {
             cls = 0;
             if (b.blk) {
                 double lb = INFINITY;
@@ -863,7 +879,7 @@ __device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& f
                     lb >= b.ratio_run * __ldg(b.blk + 4 * b.blk_stride + q))
                     cls = 3;
                 else if (lb >= r2 * lm) cls = 2;
-                else if (lb >= r4 * lm) cls = 1;
+                else if (lb >= r4s * lm) cls = 1;
             }
         }
         const unsigned b3 = __ballot_sync(0xffffffffu, cls == 3);
@@ -872,12 +888,16 @@ __device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& f
         if (cls == 3) R3[__popc(b3 & lt)] = q;
         if (cls == 2) R2[__popc(b2 & lt)] = q;
         if (cls == 0 || cls == 1) { M[__popc(bm & lt)] = q; Mcls[__popc(bm & lt)] = cls; }
-        const int nR2 = __popc(b2), nR3 = __popc(b3), nm = __popc(bm);
+        int nR2 = __popc(b2), nR3 = __popc(b3);
+        const int nm = __popc(bm);
         __syncwarp();
+        // the M runs, as many at a time as the lists hold; the R2 and R3 runs with the first
+        for (int m0 = 0; m0 < nm || m0 == 0; m0 += kWarpChunk / SPT_BLOCK_SEGS, nR2 = nR3 = 0) {
         // segment classification of the M runs, one run at a time (lane = segment)
-        int n0 = 0, n1 = 0, n2 = 0;
-        for (int mi = 0; mi < nm; ++mi) {
+        int n0 = 0, n1 = 0, n2 = 0, n8 = 0;
+        for (int mi = m0; mi < min(nm, m0 + kWarpChunk / SPT_BLOCK_SEGS); ++mi) {
             const int sg = M[mi] * SPT_BLOCK_SEGS + lane;
+            const unsigned char at = (unsigned char)((mi - m0) * SPT_BLOCK_SEGS + lane);
             int lvl = 3;
             unsigned m = 0;
             if (sg < nseg) {
@@ -890,26 +910,35 @@ __device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& f
                     dmin = fmin(dmin, dist);
                 }
                 if (mc == 1) m = 0, lvl = dmin < r2 * L ? 1 : 2;
+                else if (p8 && dmin >= kPanel8From * L) lvl = dmin < r4s * L ? 4 : (dmin < r2 * L ? 1 : 2);
                 else lvl = dmin < r4 * L ? 0 : (dmin < r2 * L ? 1 : 2);
             }
             const unsigned v0 = __ballot_sync(0xffffffffu, lvl == 0);
             const unsigned v1 = __ballot_sync(0xffffffffu, lvl == 1);
             const unsigned v2 = __ballot_sync(0xffffffffu, lvl == 2);
+            const unsigned v8 = __ballot_sync(0xffffffffu, lvl == 4);
             if (lvl == 0) {
                 const int pos = n0 + __popc(v0 & lt);
-                lists[pos] = sg;
+                lists[pos] = at;
                 mask[pos] = (unsigned char)m;
             } else if (lvl == 1) {
-                lists[kWarpChunk + n1 + __popc(v1 & lt)] = sg;
+                lists[kWarpChunk + n1 + __popc(v1 & lt)] = at;
             } else if (lvl == 2) {
-                lists[2 * kWarpChunk + n2 + __popc(v2 & lt)] = sg;
+                lists[2 * kWarpChunk + n2 + __popc(v2 & lt)] = at;
+            } else if (lvl == 4) {
+                lists[3 * kWarpChunk + n8 + __popc(v8 & lt)] = at;
             }
             n0 += __popc(v0);
             n1 += __popc(v1);
             n2 += __popc(v2);
+            n8 += __popc(v8);
         }
         __syncwarp();
-        const int e0 = n0 * nps, e1 = e0 + 4 * n1, e2 = e1 + 2 * n2;
+        auto listed = [&](int list, int k) {  // segment k of a list
+            const int v = lists[list * kWarpChunk + k];
+            return M[m0 + v / SPT_BLOCK_SEGS] * SPT_BLOCK_SEGS + v % SPT_BLOCK_SEGS;
+        };
+        const int e0 = n0 * nps, e8 = e0 + 8 * n8, e1 = e8 + 4 * n1, e2 = e1 + 2 * n2;
         const int e3 = e2 + 2 * SPT_BLOCK_SEGS * nR2, e4 = e3 + SPT_RUN_NODES * nR3;
         for (int q0i = lane; q0i < e4; q0i += 32 * NQ) {
             double rq[NQ], zq[NQ], wq[NQ];
@@ -926,17 +955,23 @@ __device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& f
                     // padding lane: any valid node, not accumulated
                 } else if (qq < e0) {
                     const int li = qq / nps;
-                    src = (size_t)lists[li] * nps + (qq - li * nps);
+                    src = (size_t)listed(0, li) * nps + (qq - li * nps);
                     tr = b.node;
                     tz = b.node + b.node_stride;
                     tw = b.node + 2 * b.node_stride;
                     mk[j] = mask[li];
-                } else if (qq < e1) {
+                } else if (qq < e8) {
                     const int i = qq - e0;
-                    src = (size_t)lists[kWarpChunk + (i >> 2)] * 6 + (i & 3);
+                    src = (size_t)listed(3, i >> 3) * 8 + (i & 7);
+                    tr = p8r;
+                    tz = p8z;
+                    tw = p8w;
+                } else if (qq < e1) {
+                    const int i = qq - e8;
+                    src = (size_t)listed(1, i >> 2) * 6 + (i & 3);
                 } else if (qq < e2) {
                     const int i = qq - e1;
-                    src = (size_t)lists[2 * kWarpChunk + (i >> 1)] * 6 + 4 + (i & 1);
+                    src = (size_t)listed(2, i >> 1) * 6 + 4 + (i & 1);
                 } else if (qq < e3) {
                     const int i = qq - e2;
                     const int sgi = R2[i / (2 * SPT_BLOCK_SEGS)] * SPT_BLOCK_SEGS + ((i & (2 * SPT_BLOCK_SEGS - 1)) >> 1);
@@ -978,7 +1013,7 @@ __device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& f
                             }
                         } else {
                             double er, ez;
-                            ring_field_far(pr[p], pinv[p], dz, rq[j], er, ez);
+                            ring_field_far<false, true>(pr[p], pinv[p], dz, rq[j], er, ez);
                             ar[p] = fma(wq[j], er, ar[p]);
                             az[p] = fma(wq[j], ez, az[p]);
                         }
@@ -988,6 +1023,7 @@ __device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& f
             }
         }
         __syncwarp();  // the lists are rewritten by the next chunk
+        }
     }
     // fixed-order warp reduction; lane 0 writes the round's fields
     bool redo = false;
@@ -1139,6 +1175,7 @@ static __device__ void bem_closest(Ctx& c, int n, bool frame) {
 // B for one record k, by one warp: the near-segment sinh quadrature
 // (bem/axisymmetric.py:566-600); lane 0 ends with near_r in record slot 7 and
 // near_z in ntmp[3k + 2].
+template <bool FAST>
 __device__ __forceinline__ void near_point(Ctx& c, int k, unsigned long long& n_near, unsigned long long& n_ring_near) {
     const SptBem& b = c.bem;
     const int lane = threadIdx.x & 31;
@@ -1182,14 +1219,24 @@ __device__ __forceinline__ void near_point(Ctx& c, int k, unsigned long long& n_
                 const double sg0 = segf(b, 9, sg), dsg = (segf(b, 10, sg) - sg0) * iL;
                 for (int qn = lane; qn < cnt * 8; qn += 32) {
                     const int iv = qn >> 3, gi = qn & 7;
-                    // sinh and cosh of the node from one exponential: sinh's rounding is 1e-16 of d, and
-                    // the node is at least d from the point
-                    const double ev = exp(fma(iv + 0.5 * (b.gauss8_x[gi] + 1.0), width, v0)), em = rcp_pos(ev);
-                    const double sl = fma(0.5 * d, ev - em, sp);
+                    // A node's place is rounded at ulp(rho), 1e-10 of its distance at a picometre, so the
+                    // reference rule takes sinh as accurate as the reference's; the adaptive rule takes sinh and
+                    // cosh from one exponential (sinh to 1e-16 of d, and the node is at least d from the point).
+                    const double v = fma(iv + 0.5 * (b.gauss8_x[gi] + 1.0), width, v0);
+                    double sh, ch;
+                    if constexpr (FAST) {
+                        const double ev = exp(v), em = rcp_pos(ev);
+                        sh = 0.5 * (ev - em);
+                        ch = 0.5 * (ev + em);
+                    } else {
+                        sh = sinh(v);
+                        ch = sqrt_pos(fma(sh, sh, 1.0));
+                    }
+                    const double sl = fma(d, sh, sp);
                     const double sr = fma(sl, ur, p0r), sz = fma(sl, uz, p0z);
-                    const double w = fma(sl, dsg, sg0) * (2.0 * kPi * sr) * (0.5 * d * (ev + em)) * half * b.gauss8_w[gi];
+                    const double w = fma(sl, dsg, sg0) * (2.0 * kPi * sr) * d * ch * half * b.gauss8_w[gi];
                     double er, ez;
-                    ring_field_far<true>(re, inv, ze - sz, sr, er, ez);
+                    ring_field_far<true, FAST>(re, inv, ze - sz, sr, er, ez);
                     acc_r = fma(w, er, acc_r);
                     acc_z = fma(w, ez, acc_z);
                 }
@@ -1268,7 +1315,7 @@ __device__ __forceinline__ void bem_sums(Ctx& c, int n, int* status_flag) {
                 atomicAdd(c.cnt + SPT_CNT_CLUSTER_EVALS, 1ull);
             }
         } else {
-            near_point(c, k, n_near, n_ring_near);
+            near_point<FAR == SPT_FAR_ADAPTIVE>(c, k, n_near, n_ring_near);
         }
     }
     count_add(c, SPT_CNT_NEAR_PAIRS, n_near);
@@ -1601,7 +1648,7 @@ __device__ void bem_points_fused(Ctx& c, int n) {
     for (int k = threadIdx.x >> 5; k < n; k = next_task(&s_task)) {
         closest_point(c, k, false);
         __syncwarp();
-        near_point(c, k, n_near, n_ring_near);
+        near_point<true>(c, k, n_near, n_ring_near);
         __syncwarp();
         far_point<FORM>(c, k, far_evals, cl_evals);
         if (lane == 0) {
@@ -2535,7 +2582,7 @@ __device__ __forceinline__ void direct_point(Ctx& c, double x, double y, double 
     __syncwarp();
     closest_point(c, 0, false);
     __syncwarp();
-    near_point(c, 0, n.n_near, n.n_ring_near);
+    near_point<true>(c, 0, n.n_near, n.n_ring_near);
     __syncwarp();
     far_point<FORM>(c, 0, n.far_evals, n.cl_evals);
     __syncwarp();

@@ -179,8 +179,8 @@ field_quad_kernel(const double* x, const double* y, const double* z, long long n
                 const bool on0 = !((m >> __umulhi((unsigned)k, nps_inv)) & 1u);
                 const bool on1 = k1 != k && !((m >> __umulhi((unsigned)k1, nps_inv)) & 1u);
                 double er0, ez0, er1, ez1;
-                ring_field_far(rho, inv, zz - z0, r0, er0, ez0);
-                ring_field_far(rho, inv, zz - z1, r1, er1, ez1);
+                ring_field_far<false, false>(rho, inv, zz - z0, r0, er0, ez0);
+                ring_field_far<false, false>(rho, inv, zz - z1, r1, er1, ez1);
                 if (on0) {
                     ar = fma(w0, er0, ar);
                     az = fma(w0, ez0, az);
@@ -193,7 +193,7 @@ field_quad_kernel(const double* x, const double* y, const double* z, long long n
         }
         ar = warp_sum(ar);
         az = warp_sum(az);
-        if (part == 0) near_point(c, 0, n_near, n_ring);
+        if (part == 0) near_point<false>(c, 0, n_near, n_ring);
     }
     if (in_cta > 1) {
         // partial sums to the first rank's shared memory

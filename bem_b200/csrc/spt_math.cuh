@@ -128,17 +128,25 @@ static __device__ __noinline__ void ring_axis_taylor(double rho, double z, doubl
     ez = z / (4.0 * kPi * ax15) + 3.0 * rho2 * z * (3.0 * a2 - 2.0 * z2) / (16.0 * kPi * ax35);
 }
 
-// a^2 - rho^2 + z^2 in the reference's rounding (bem/axisymmetric.py:262): near
-// a surface it cancels to ~(rho - a) rho, and its rounding (1e-13 of the field
-// at 10 pm) is part of what traces of ill-conditioned particles reproduce.
-__device__ __forceinline__ double ring_a(double rho, double z2, double a) {
-    return __dadd_rn(__dadd_rn(__dmul_rn(a, a), -__dmul_rn(rho, rho)), z2);
+// Ring field close to the ring (p = d2 / D < 1e-3), the operations of
+// ring_field with its series branch: near a surface a^2 - rho^2 + z^2 cancels
+// to ~(rho - a) rho, and its rounding (1e-13 of the field at 10 pm) is part of
+// what the reference rule's traces of ill-conditioned particles reproduce.
+__device__ __forceinline__ void ring_close(double rho, double z, double a, double D, double d2, double& er,
+                                           double& ez) {
+    const double z2 = z * z, a2 = a * a, rho2 = rho * rho;
+    const double p = d2 / D, L = -0.5 * log(p);
+    const double K = fma(L, horner10(kSerK, p), horner10(kSerKd, p));
+    const double E = fma(0.5 * p, fma(L, horner10(kSerE, p), horner10(kSerEd, p)), 1.0);
+    const double sD = sqrt(D);
+    er = (K - (a2 - rho2 + z2) * E / d2) / (4.0 * kPi * kPi * rho * sD);
+    ez = z * E / (2.0 * kPi * kPi * sD * d2);
 }
 
-// Ring field close to the ring (p = d2 / D < 1e-3): the DLMF 19.12 series (of
-// which six terms leave 1e-19 there), one reciprocal for every quotient.
-__device__ __forceinline__ void ring_close(double rho, double inv_rho, double a, double z, double D, double d2,
-                                           double& er, double& ez) {
+// The same for the adaptive rule: six terms (what is left out is below 1e-19)
+// and one reciprocal for every quotient.
+__device__ __forceinline__ void ring_close_fast(double rho, double inv_rho, double z, double a, double D, double d2,
+                                                double& er, double& ez) {
     const double inv = rcp_pos(D * d2), inv_d2 = D * inv, p = d2 * (d2 * inv);
     const double L = -0.5 * log(p);
     auto h6 = [&](const double* c) {
@@ -148,17 +156,22 @@ __device__ __forceinline__ void ring_close(double rho, double inv_rho, double a,
         return v;
     };
     const double K = fma(L, h6(kSerK), h6(kSerKd));
-    const double E = fma(0.5 * p, fma(L, h6(kSerE), h6(kSerEd)), 1.0);
+    const double E = fma(0.5 * p, fma(L, h6(kSerE), h6(kSerEd)), 1.0) * inv_d2;
     const double g = sqrt_pos(d2 * inv) * (1.0 / (4.0 * kPi * kPi));  // 1 / (4 pi^2 sqrt(D))
-    er = fma(-ring_a(rho, __dmul_rn(z, z), a) * inv_d2, E, K) * (g * inv_rho);
-    ez = 2.0 * z * E * inv_d2 * g;
+    const double A = __dadd_rn(__dadd_rn(__dmul_rn(a, a), -__dmul_rn(rho, rho)), __dmul_rn(z, z));
+    er = fma(-A, E, K) * (g * inv_rho);
+    ez = 2.0 * z * E * g;
 }
 
-// The same out of line: rare in a far sum, and on another path than every
+// Both out of line for the far sums: rare there, and on another path than every
 // interleaved evaluation.
-static __device__ __noinline__ void ring_close_cold(double rho, double inv_rho, double a, double z, double D,
-                                                    double d2, double& er, double& ez) {
-    ring_close(rho, inv_rho, a, z, D, d2, er, ez);
+static __device__ __noinline__ void ring_close_cold(double rho, double z, double a, double D, double d2, double& er,
+                                                    double& ez) {
+    ring_close(rho, z, a, D, d2, er, ez);
+}
+static __device__ __noinline__ void ring_close_fast_cold(double rho, double inv_rho, double z, double a, double D,
+                                                         double d2, double& er, double& ez) {
+    ring_close_fast(rho, inv_rho, z, a, D, d2, er, ez);
 }
 
 // Ring field for the far-quadrature sum, 1/rho supplied by the caller (constant
@@ -175,7 +188,9 @@ static __device__ __noinline__ void ring_close_cold(double rho, double inv_rho, 
 // either).  Five square roots and one reciprocal, against eight and two of the
 // AGM run to convergence on d2 / D: the far sums are bound by these
 // instructions (96 M rings of one 1500-point call: 11.4 -> 6.7 ms).
-template <bool NEAR = false>
+// NEAR: a near panel's node (close rings are common, in line, and a^2 - rho^2
+// as the reference forms it); FAST: the adaptive rule's close rings.
+template <bool NEAR, bool FAST>
 __device__ __forceinline__ void ring_field_far(double rho, double inv_rho, double z, double a, double& er,
                                                double& ez) {
     const double z2 = z * z, s = rho + a, t = rho - a;
@@ -185,8 +200,10 @@ __device__ __forceinline__ void ring_field_far(double rho, double inv_rho, doubl
         return;
     }
     if (d2 < 1e-3 * D) {
-        if constexpr (NEAR) ring_close(rho, inv_rho, a, z, D, d2, er, ez);
-        else ring_close_cold(rho, inv_rho, a, z, D, d2, er, ez);
+        if constexpr (NEAR && FAST) ring_close_fast(rho, inv_rho, z, a, D, d2, er, ez);
+        else if constexpr (NEAR) ring_close(rho, z, a, D, d2, er, ez);
+        else if constexpr (FAST) ring_close_fast_cold(rho, inv_rho, z, a, D, d2, er, ez);
+        else ring_close_cold(rho, z, a, D, d2, er, ez);
         return;
     }
     const double r1 = sqrt_pos(D), r2 = sqrt_pos(d2);
@@ -203,7 +220,7 @@ __device__ __forceinline__ void ring_field_far(double rho, double inv_rho, doubl
     S = fma(fma(0.25, e2, 2.0) * t4, t4, S);
     const double Q = (D - S) * (inv * m);
     const double F = im * fma(e2, fma(e2, 9.0 / 64.0, 0.25), 1.0);
-    const double A = NEAR ? ring_a(rho, __dmul_rn(z, z), a) : fma(-s, t, z2);  // a^2 - rho^2 = -(rho + a)(rho - a)
+    const double A = NEAR ? a * a - rho * rho + z2 : fma(-s, t, z2);  // a^2 - rho^2 = -(rho + a)(rho - a)
     er = fma(-A, Q, 1.0) * (F * inv_rho * (1.0 / (8.0 * kPi)));
     ez = z * Q * (F * (1.0 / (4.0 * kPi)));
 }
@@ -211,7 +228,7 @@ __device__ __forceinline__ void ring_field_far(double rho, double inv_rho, doubl
 // ring_field_far out of line, for the rare float64 terms of a float32 sum.
 static __device__ __noinline__ void ring_field_far_cold(double rho, double inv_rho, double z, double a, double& er,
                                                         double& ez) {
-    ring_field_far(rho, inv_rho, z, a, er, ez);
+    ring_field_far<false, false>(rho, inv_rho, z, a, er, ez);
 }
 
 // ---------------------------------------------------------------------------

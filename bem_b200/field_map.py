@@ -8,7 +8,8 @@ its highest two Chebyshev orders are below TAIL of its largest coefficient
 (sampled by the direct sum with tighter thresholds than the adaptive rule's
 own), and divided otherwise; near a panel (closer than two of its lengths)
 and behind the surface there are no cells, and points there take the direct
-sum.  Not in the reference.
+sum, with the Gauss-8 panel nodes that are kept beside the map for it.  Not
+in the reference.
 """
 
 import ctypes
@@ -34,6 +35,19 @@ DCT[0] *= 0.5
 MONO = np.zeros((N, N))
 for _k in range(N):
     MONO[_k, : _k + 1] = np.polynomial.chebyshev.cheb2poly(np.eye(N)[_k])[: _k + 1]
+
+
+def panel_nodes(profile, sigma, n):
+    """[3, n_seg * n]: the n-point Gauss rule over each whole segment, as
+    (rho_q, z_q, area_q * sigma_q), segment-major."""
+    x, w = np.polynomial.legendre.leggauss(n)
+    t = 0.5 * (x + 1.0)
+    p0, tan = profile[:-1], profile[1:] - profile[:-1]
+    rho = p0[:, 0:1] + t * tan[:, 0:1]
+    z = p0[:, 1:2] + t * tan[:, 1:2]
+    area = 2.0 * np.pi * rho * (np.linalg.norm(tan, axis=-1)[:, None] * 0.5 * w)
+    dens = sigma[:-1, None] + t * (sigma[1:, None] - sigma[:-1, None])
+    return np.stack([rho.ravel(), z.ravel(), (area * dens).ravel()])
 
 
 def link_tables(leaves, divided):
@@ -128,11 +142,14 @@ def build(tables):
         unit = _lib.MAP_UNIT
         start = -(-base.numel() // unit) * unit
         rec_at = -(-(_lib.MAP_HEADER + tab.size // 2) // 8) * 8
-        out = torch.zeros(start + rec_at + n_kept * _lib.MAP_REC, dtype=torch.float64, device=dev)
+        p8_at = rec_at + n_kept * _lib.MAP_REC
+        p8 = panel_nodes(prof, tables.sigma, 8)
+        out = torch.zeros(start + p8_at + p8.size, dtype=torch.float64, device=dev)
         out[: base.numel()] = base
-        out[start: start + 3] = t64([1.0 / side, z_lo, float(rec_at)])
+        out[start: start + 4] = t64([1.0 / side, z_lo, float(rec_at), float(p8_at)])
+        out[start + p8_at:] = t64(p8.reshape(-1))
         out[start + _lib.MAP_HEADER: start + _lib.MAP_HEADER + tab.size // 2] = torch.as_tensor(
             tab.reshape(-1), device=dev).view(torch.float64)
-        out[start + rec_at:] = torch.cat(records).reshape(-1)
+        out[start + rec_at: start + p8_at] = torch.cat(records).reshape(-1)
         torch.cuda.current_stream(dev).synchronize()
     return out, (_lib.MAP_TAG << 16) | (start // unit)

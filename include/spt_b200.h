@@ -217,7 +217,9 @@ typedef struct {
  * of a quadtree over the (rho, z) half plane that hold the perturbation field
  * as polynomials of SPT_MAP_N coefficients in each coordinate.  Layout, in
  * doubles: a header of SPT_MAP_HEADER (1 / side of the root square, its lowest
- * z, the offset of the cell records; its lowest rho is 0), int32 tables of 64
+ * z, the offset of the cell records, the offset of the panels' Gauss-8 nodes --
+ * rows rho, z, w of 8 n_seg, segment-major, w = area * density --; the root's
+ * lowest rho is 0), int32 tables of 64
  * entries (three quadtree levels each, entry 8 * z index + rho index: a cell's
  * number, -1 for none, or -2 - the number of the next table), then one record
  * of SPT_MAP_REC per cell: centre rho, centre z, 1 / half-width, 5 unused, and

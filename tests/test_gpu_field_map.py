@@ -32,7 +32,7 @@ def _direct(tab, pts):
 def _cells(tab):
     m, tag = tab.field_map()
     m = m[(tag & 0xFFFF) * _lib.MAP_UNIT:].cpu().numpy()
-    rec = m[int(m[2]):].reshape(-1, _lib.MAP_REC)
+    rec = m[int(m[2]):int(m[3])].reshape(-1, _lib.MAP_REC)
     return rec[:, 0], rec[:, 1], 1.0 / rec[:, 2]
 
 
