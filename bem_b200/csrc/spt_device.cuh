@@ -195,6 +195,9 @@ constexpr int kWarpChunk = 256;
 constexpr int kWarpRuns = 32;
 constexpr int kWarpScratchInts = 5 * kWarpChunk / 4 + 4 * kWarpRuns + SPT_MAX_CLUSTER_RUNS / 32;
 static_assert(kWarpScratchInts % 2 == 0, "per-warp scratch keeps 8-byte alignment");
+// Shared slots of the points that several warps share (bem_points_direct).
+constexpr int kSplitPoints = kMaxWarps / 2;
+constexpr int kSplitDoubles = kSplitPoints * 256;  // per point: 4 slots x 2 components x 32 lanes
 
 // Shared-memory layout of one CTA for groups of up to E particles.  The far
 // rule decides the big region: node tiles for the reference rule (the TMA
@@ -240,7 +243,7 @@ __host__ __device__ inline Layout make_layout(int E, int far_rule, bool want_sur
     for (int cap = kTileNodes; cap >= 256; cap >>= 1) {
         o = base;
         L.tile_cap = tiles ? cap : 0;
-        L.tiles = o; o += tiles ? 2 * 3 * cap : (lists ? warps * kWarpScratchInts / 2 : 0);
+        L.tiles = o; o += tiles ? 2 * 3 * cap : (lists ? warps * (kWarpScratchInts / 2) + kSplitDoubles : 0);
         L.red = o; o += kMaxWarps * 3 * kRound;
         L.ints = o;
         L.total_doubles = o + (n_ints + 1) / 2;
@@ -288,7 +291,8 @@ struct Ctx {
     double* base;    // dynamic smem
     Layout L;
     double *y0, *nw_, *sp, *kp, *kv, *tb, *td, *q, *m, *cps, *fld, *img, *bpt, *tiles, *red, *imgs;
-    double* ntmp;    // near sums' E_z per record (stride 3): fld, or img while fld holds mapped fields
+    double* ntmp;    // reference rule: near sums' E_z per record (stride 3)
+    double* wrec;    // adaptive rule: this warp's record (8 doubles)
     int* live;
     int* list;
     unsigned char* nflag;
@@ -351,6 +355,7 @@ __device__ inline void bind(Ctx& c, double* smem, int E, int far_rule, double* s
     c.imgs = smem + L.imgs;
     c.tiles = smem + L.tiles;
     c.red = smem + L.red;
+    c.wrec = c.red + 8 * (threadIdx.x >> 5);  // (the adaptive rule has no block reduction)
     int* ib = reinterpret_cast<int*>(smem + L.ints);
     c.live = ib + L.live_off;
     c.list = ib + L.list_off;
@@ -393,13 +398,16 @@ __device__ __forceinline__ double seg_dist2(const SptBem& b, int s, double rq, d
 }
 
 // near test of bem/axisymmetric.py:566-570 -> (near, projection, distance)
+// FAST (the adaptive rule): a branch-free root, exact to the last bit or two.
+template <bool FAST = false>
 __device__ __forceinline__ bool seg_near(const SptBem& b, int s, double re, double ze, double& proj, double& dist) {
     const double p0r = segf(b, 0, s), p0z = segf(b, 1, s), L = segf(b, 4, s), ur = segf(b, 5, s), uz = segf(b, 6, s);
     const double dr = re - p0r, dz = ze - p0z;
     const double along = dr * ur + dz * uz;
     proj = fmin(fmax(along, 0.0), L);
     const double ar = dr - proj * ur, az = dz - proj * uz;
-    dist = sqrt(ar * ar + az * az);
+    if constexpr (FAST) dist = sqrt_pos(fmax(fma(ar, ar, az * az), 1e-300));
+    else dist = sqrt(ar * ar + az * az);
     return dist < L;
 }
 
@@ -409,7 +417,8 @@ __device__ __forceinline__ bool seg_near(const SptBem& b, int s, double re, doub
 // largest segment length.
 __device__ __forceinline__ double blk_lower(const SptBem& b, int q, double r, double z) {
     const double cr = __ldg(b.blk + q), cz = __ldg(b.blk + b.blk_stride + q), rad = __ldg(b.blk + 2 * b.blk_stride + q);
-    const double dc = sqrt((r - cr) * (r - cr) + (z - cz) * (z - cz));
+    const double dr = r - cr, dz = z - cz;
+    const double dc = sqrt_pos(fmax(fma(dr, dr, dz * dz), 1e-300));
     return dc - rad - 1e-9 * (dc + rad);
 }
 __device__ __forceinline__ double blk_lmax(const SptBem& b, int q) { return __ldg(b.blk + 3 * b.blk_stride + q); }
@@ -593,22 +602,6 @@ __device__ void far_round(Ctx& c, int r0, int np_, int n_tiles, int segs_per_til
     round_reduce<NP, MIX>(c, r0, np_, ar, az, fr, fz, kr, kz, sa);
 }
 
-// Adaptive far sum (SPT_FAR_ADAPTIVE) for points r0..r0+np_-1 of the list,
-// computed by ONE warp (each warp of the CTA takes its own rounds; nothing
-// here waits on another warp).  Segments are taken kWarpChunk at a time
-// (kWarpRuns runs of SPT_BLOCK_SEGS).  The warp classifies the chunk's runs by
-// the smallest lower-bound distance over the round's points: flagged runs at
-// least ratio_run arclengths away take the 8-point rule over the whole run
-// (list R3), runs whose every segment is at least ratio2 lengths away take
-// Gauss-2 on each segment (R2), the rest (M) are classified segment by
-// segment -- below ratio4 lengths the reference nodes, with an 8-bit mask of
-// the points for which the segment is near (they skip it), below ratio2
-// Gauss-4, else Gauss-2 (lists L0, L1, L2 in the warp's own shared scratch).
-// The flattened node list L0 | L1 | L2 | R2 | R3 is then evaluated by the
-// warp's lanes, NQ nodes in flight per lane, nodes read through L1/L2.
-// Without run bounds every run is in M.  Lane 0 ends with the round's
-// fields in record slots 5, 6 (near parts included); returns, in every lane,
-// whether a float32 sum (MIX) was ill-conditioned (kappa test).
 // Recurrence constants of the Legendre polynomials, P_(n+1) = a_n u P_n - b_n P_(n-1).
 static __device__ __constant__ double kLegA[64] = {
 #define SPT_LA(n) (2.0 * (n) + 1.0) / ((n) + 1.0)
@@ -645,13 +638,14 @@ __device__ __forceinline__ void cluster_field(const double* rec, int nt, double 
     const double u = dz * ir, s = rho * ir, x = __ldg(rec + 1) * ir;
     double p0 = 1.0, p1 = u, d0 = 0.0, d1 = 1.0;
     double A = __ldg(rec + 2), B = 0.0;
-    double xn = x;
+    double xn = x, n1 = 2.0;  // n + 1, as a double: conversions are slower than the sum
     auto term = [&](int n, double moment) {
         const double m = moment * xn;
-        A = fma((double)(n + 1) * m, p1, A);
+        A = fma(n1 * m, p1, A);
         B = fma(m, d1, B);
         const double p2 = fma(kLegA[n] * u, p1, -kLegB[n] * p0);
-        const double d2 = fma((double)(2 * n + 1), p1, d0);
+        const double d2 = fma(fma(2.0, n1, -1.0), p1, d0);
+        n1 += 1.0;
         p0 = p1;
         p1 = p2;
         d0 = d1;
@@ -771,55 +765,105 @@ __device__ __forceinline__ void rotate_rho(double x, double y, double rho, doubl
 // panels PANEL8_FROM to PANEL8_TO x ratio4 lengths away.  At two lengths its
 // error (8.1^-16) is that of the reference's 32 sub-panel nodes, at a quarter
 // of the ring evaluations; up to twice ratio4 it replaces the whole-panel
-// Gauss-4, whose error at ratio4 = 8 (32^-8, 1e-12) is the adaptive rule's
-// largest.
+// Gauss-4, whose error at ratio4 = 8 is 32^-8 = 1e-12, and Gauss-4 serves to
+// twice ratio2 (Gauss-2 at 300 lengths was the rule's largest error, 2e-12 near
+// the corner of the 3000-panel well; 2e-13 at 600).
 constexpr double kPanel8From = 2.0, kPanel8To = 2.0;
 __device__ __forceinline__ const double* panel8(const SptBem& b) {
     const double* map = field_map(b);
     return map ? map + (size_t)__ldg(map + 3) : nullptr;
 }
 
-template <int NP, int NQ, bool MIX>
-__device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& far_evals,
-                                  unsigned long long& cl_evals) {
+// Sums of one point's direct evaluation.  Its ring evaluations come in rounds
+// of one per lane, and each round adds to one of four slots of its lane: near
+// quadrature and cluster expansions by their number, round % 4, the far nodes
+// of a chunk by quarters.  So one warp can take all rounds, or 2 or 4 warps a
+// share of the slots each, and the result -- the slots added per lane, then the
+// lanes -- is the same to the bit.
+struct PointSums {
+    double r[4], z[4];
+    int round, share, shares;  // next round's number; this warp's share of 1, 2 or 4
+    __device__ PointSums(int share_, int shares_) : round(0), share(share_), shares(shares_) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) r[k] = z[k] = 0.0;
+    }
+    // whether the next round is this warp's (alike in every lane)
+    __device__ __forceinline__ bool mine() const { return (round & (shares - 1)) == share; }
+    __device__ __forceinline__ void add(double er, double ez) {
+        const int k = round & 3;  // a branch the whole warp takes
+        if (k == 0) { r[0] += er; z[0] += ez; }
+        else if (k == 1) { r[1] += er; z[1] += ez; }
+        else if (k == 2) { r[2] += er; z[2] += ez; }
+        else { r[3] += er; z[3] += ez; }
+    }
+    // the far rounds' quarters: slot 0 is the current quarter's, and four turns bring every slot home
+    __device__ __forceinline__ void turn(double er, double ez) {
+        const double r0 = r[0] + er, z0 = z[0] + ez;
+        r[0] = r[1]; r[1] = r[2]; r[2] = r[3]; r[3] = r0;
+        z[0] = z[1]; z[1] = z[2]; z[2] = z[3]; z[3] = z0;
+    }
+    // the whole sums, in lane 0
+    __device__ __forceinline__ void total(double& er, double& ez) const {
+        er = warp_sum((r[0] + r[1]) + (r[2] + r[3]));
+        ez = warp_sum((z[0] + z[1]) + (z[2] + z[3]));
+    }
+};
+
+// Counters of a warp's direct evaluations, and their sum into the CTA's.
+struct PointCounts {
+    unsigned long long n_near = 0, n_ring_near = 0, far_evals = 0, cl_evals = 0;
+};
+__device__ __forceinline__ void count_points(Ctx& c, const PointCounts& n) {
+    count_add(c, SPT_CNT_NEAR_PAIRS, n.n_near);
+    count_add(c, SPT_CNT_RING_NEAR, n.n_ring_near);
+    count_add(c, SPT_CNT_RING_FAR, n.far_evals);
+    count_add(c, SPT_CNT_CLUSTER_EVALS, n.cl_evals);
+}
+
+// Adaptive far sum (SPT_FAR_ADAPTIVE) at (re, ze), by one warp (nothing here
+// waits on another warp).  Cluster expansions cover the runs of their clusters.
+// The other runs are classified 32 at a time by their lower-bound distance:
+// flagged runs at least ratio_run arclengths away take the 8-point rule over
+// the whole run (list R3), runs whose every segment is at least ratio2 lengths
+// away Gauss-2 on each segment (R2), the rest (M) are classified segment by
+// segment -- the reference nodes (near segments masked), Gauss-8 where the
+// panel nodes are given, Gauss-4, or Gauss-2 (lists L0, L8, L1, L2 in the
+// warp's own shared scratch).  The flattened node list is then evaluated by the
+// lanes, nodes read through L1/L2.  Without run bounds every run is in M.
+//
+// MIX false: float64, one ring evaluation in flight per lane (every copy in
+// flight is an inlined copy of the ring kernel, and the trace kernels are bound
+// by instruction fetch), into S.  MIX true: float32 Kahan sums, four in flight;
+// mr, mz, mabs return them and the sum of |terms| in lane 0.
+template <bool MIX>
+__device__ void far_adaptive_warp(Ctx& c, double re, double ze, PointSums& S, PointCounts& cnt, double& mr, double& mz,
+                                  double& mabs) {
+    constexpr int NQ = MIX ? 4 : 1;
     const SptBem& b = c.bem;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nseg = b.n_seg, nps = b.nodes_per_seg;
-    double* P = c.bpt;
     int* scratch = reinterpret_cast<int*>(c.tiles) + warp * kWarpScratchInts;
     unsigned char* lists = reinterpret_cast<unsigned char*>(scratch);  // L0 | L1 | L2 | L8, kWarpChunk each
-    unsigned char* mask = lists + 4 * kWarpChunk;                      // near masks of L0
+    unsigned char* mask = lists + 4 * kWarpChunk;                      // near flags of L0
     int* R2 = scratch + 5 * kWarpChunk / 4;
     int* R3 = R2 + kWarpRuns;
     int* M = R3 + kWarpRuns;
     int* Mcls = M + kWarpRuns;
     unsigned* covered = reinterpret_cast<unsigned*>(Mcls + kWarpRuns);  // runs summed by cluster expansions
-    double pr[NP], pinv[NP], pz[NP], ar[NP], az[NP];
-    float fr[NP], fz[NP], kr[NP], kz[NP], prf[NP], pinvf[NP];
-    float sa[NP];
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        const int k = r0 + (p < np_ ? p : 0);
-        pr[p] = P[8 * k + 3];
-        pinv[p] = pr[p] > 0.0 ? 1.0 / pr[p] : 0.0;
-        pz[p] = P[8 * k + 4];
-        ar[p] = 0.0;
-        az[p] = 0.0;
-        fr[p] = fz[p] = kr[p] = kz[p] = sa[p] = 0.0f;
-        prf[p] = (float)pr[p];
-        pinvf[p] = (float)pinv[p];
-    }
-    const double r4 = b.ratio4, r2 = b.ratio2;
+    const double inv = re > 0.0 ? 1.0 / re : 0.0;
+    double cr_ = 0.0, cz_ = 0.0;                                // mixed form: the float64 expansions
+    float fr = 0.f, fz = 0.f, kr = 0.f, kz = 0.f, sa = 0.f;     // mixed form: Kahan sums, sum of |float32 terms|
+    const float ref = (float)re, invf = (float)inv;
     const double* cr = b.coarse;
     const double* cz = b.coarse + b.coarse_stride;
     const double* cw = b.coarse + 2 * b.coarse_stride;
     const bool run_rule = b.blk && b.run_nodes && b.ratio_run > 0.0;
     const unsigned lt = (1u << lane) - 1u;
-    // Cluster expansions (one point per task): lane = run; the run is covered
-    // by its highest ancestor cluster that is at least kappa radii away, and
-    // the lane of the cluster's first run adds that cluster's expansion.
+    // Cluster expansions: lane = run; the run is covered by its highest
+    // ancestor cluster that is at least kappa radii away, and the lane of the
+    // cluster's first run lists that cluster.
     const int n_run = (nseg + SPT_BLOCK_SEGS - 1) / SPT_BLOCK_SEGS;
-    const bool use_cl = NP == 1 && b.blk && b.clusters && b.cluster_kappa > 0.0 && n_run <= SPT_MAX_CLUSTER_RUNS;
+    const bool use_cl = b.blk && b.clusters && b.cluster_kappa > 0.0 && n_run <= SPT_MAX_CLUSTER_RUNS;
     if (use_cl) {
         const int nt = b.cluster_terms, rec_len = nt + 2;
         // the covering clusters' heads, listed first (the segment lists are free
@@ -835,8 +879,8 @@ __device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& f
                 for (int l = 0; l < b.cluster_levels; ++l) {
                     const int i = off + (q >> l);
                     const double* rec = b.clusters + (size_t)i * rec_len;
-                    const double dz = pz[0] - __ldg(rec);
-                    if (pr[0] * pr[0] + dz * dz >= b.cluster_kappa * b.cluster_kappa * __ldg(rec + 1) * __ldg(rec + 1)) {
+                    const double dz = ze - __ldg(rec);
+                    if (re * re + dz * dz >= b.cluster_kappa * b.cluster_kappa * __ldg(rec + 1) * __ldg(rec + 1)) {
                         lv = l;
                         idx = i;
                     }
@@ -851,29 +895,37 @@ __device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& f
             n_heads += __popc(hm);
         }
         __syncwarp();
-        for (int hh = lane; hh < n_heads; hh += 32) {
-            double er, ez;
-            cluster_field(b.clusters + (size_t)heads[hh] * rec_len, nt, pr[0], pz[0], er, ez);
-            ar[0] += er;
-            az[0] += ez;
-            ++cl_evals;
+        for (int h0 = 0; h0 < n_heads; h0 += 32, ++S.round) {
+            if (!S.mine()) continue;
+            double er = 0.0, ez = 0.0;
+            if (h0 + lane < n_heads) {
+                cluster_field(b.clusters + (size_t)heads[h0 + lane] * rec_len, nt, re, ze, er, ez);
+                ++cnt.cl_evals;
+            }
+            if (MIX) {
+                cr_ += er;
+                cz_ += ez;
+            } else {
+                S.add(er, ez);
+            }
         }
         __syncwarp();
     }
+    // floor(q / nps) = umulhi(q, nps_inv) for q below kWarpChunk nps <= 65536
+    const unsigned nps_inv = 0xffffffffu / (unsigned)nps + 1u;
     const double* p8 = panel8(b);
     const double* p8r = p8;
     const double* p8z = p8 + 8 * (size_t)nseg;
     const double* p8w = p8 + 16 * (size_t)nseg;
     // the segment tests read ratio4 as the distance from which whole-panel Gauss-4 serves
-    const double r4s = p8 ? kPanel8To * r4 : r4;
+    const double r4 = b.ratio4, r4s = p8 ? kPanel8To * r4 : r4, r2 = p8 ? kPanel8To * b.ratio2 : b.ratio2;
     for (int q0 = 0; q0 < n_run; q0 += kWarpRuns) {
         const int q = q0 + lane;
         int cls = -1;  // 3 run rule, 2 Gauss-2 on every segment, 1 no segment below ratio4, 0 full test
         if (q < n_run && !(use_cl && ((covered[q >> 5] >> (q & 31)) & 1u))) {
             cls = 0;
             if (b.blk) {
-                double lb = INFINITY;
-                for (int p = 0; p < np_; ++p) lb = fmin(lb, blk_lower(b, q, P[8 * (r0 + p) + 3], P[8 * (r0 + p) + 4]));
+                const double lb = blk_lower(b, q, re, ze);
                 const double lm = blk_lmax(b, q);
                 if (run_rule && __ldg(b.blk + 5 * b.blk_stride + q) != 0.0 &&
                     lb >= b.ratio_run * __ldg(b.blk + 4 * b.blk_stride + q))
@@ -899,17 +951,13 @@ __device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& f
             const int sg = M[mi] * SPT_BLOCK_SEGS + lane;
             const unsigned char at = (unsigned char)((mi - m0) * SPT_BLOCK_SEGS + lane);
             int lvl = 3;
-            unsigned m = 0;
+            bool m = false;
             if (sg < nseg) {
                 const int mc = Mcls[mi];
                 const double L = segf(b, 4, sg);
-                double dmin = INFINITY;
-                for (int p = 0; p < np_; ++p) {
-                    double proj, dist;
-                    if (seg_near(b, sg, P[8 * (r0 + p) + 3], P[8 * (r0 + p) + 4], proj, dist)) m |= 1u << p;
-                    dmin = fmin(dmin, dist);
-                }
-                if (mc == 1) m = 0, lvl = dmin < r2 * L ? 1 : 2;
+                double proj, dmin;
+                m = seg_near<true>(b, sg, re, ze, proj, dmin) && mc == 0;
+                if (mc == 1) lvl = dmin < r2 * L ? 1 : 2;
                 else if (p8 && dmin >= kPanel8From * L) lvl = dmin < r4s * L ? 4 : (dmin < r2 * L ? 1 : 2);
                 else lvl = dmin < r4 * L ? 0 : (dmin < r2 * L ? 1 : 2);
             }
@@ -940,9 +988,16 @@ __device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& f
         };
         const int e0 = n0 * nps, e8 = e0 + 8 * n8, e1 = e8 + 4 * n1, e2 = e1 + 2 * n2;
         const int e3 = e2 + 2 * SPT_BLOCK_SEGS * nR2, e4 = e3 + SPT_RUN_NODES * nR3;
-        for (int q0i = lane; q0i < e4; q0i += 32 * NQ) {
+        const int rounds = (e4 + 32 * NQ - 1) / (32 * NQ);
+#pragma unroll 1
+        for (int quarter = 0; quarter < (MIX ? 1 : 4); ++quarter) {
+        double tr_ = 0.0, tz_ = 0.0;
+        const bool own = MIX || (quarter & (S.shares - 1)) == S.share;
+        const int first = MIX ? 0 : rounds * quarter / 4, last = MIX ? rounds : (own ? rounds * (quarter + 1) / 4 : first);
+#pragma unroll 1
+        for (int rd = first; rd < last; ++rd) {
+            const int q0i = rd * 32 * NQ + lane;
             double rq[NQ], zq[NQ], wq[NQ];
-            unsigned mk[NQ];
             bool in[NQ];
 #pragma unroll
             for (int j = 0; j < NQ; ++j) {
@@ -950,16 +1005,15 @@ __device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& f
                 in[j] = qq < e4;
                 size_t src = 0;
                 const double *tr = cr, *tz = cz, *tw = cw;
-                mk[j] = 0;
                 if (!in[j]) {
                     // padding lane: any valid node, not accumulated
                 } else if (qq < e0) {
-                    const int li = qq / nps;
+                    const int li = (int)__umulhi((unsigned)qq, nps_inv);
                     src = (size_t)listed(0, li) * nps + (qq - li * nps);
                     tr = b.node;
                     tz = b.node + b.node_stride;
                     tw = b.node + 2 * b.node_stride;
-                    mk[j] = mask[li];
+                    in[j] = !mask[li];  // near segments are the near quadrature's
                 } else if (qq < e8) {
                     const int i = qq - e0;
                     src = (size_t)listed(3, i >> 3) * 8 + (i & 7);
@@ -988,66 +1042,48 @@ __device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& f
                 zq[j] = __ldg(tz + src);
                 wq[j] = __ldg(tw + src);
             }
-#pragma unroll
-            for (int p = 0; p < NP; ++p) {
+            if constexpr (MIX) {
 #pragma unroll
                 for (int j = 0; j < NQ; ++j) {
-                    if (p < np_ && in[j] && !((mk[j] >> p) & 1u)) {
-                        const double dz = pz[p] - zq[j];
-                        if (MIX) {
-                            float er, ez;
-                            if (ring_far_f(prf[p], pinvf[p], (float)(pr[p] - rq[j]), (float)(pr[p] + rq[j]), (float)dz,
-                                           (float)rq[j], er, ez)) {
-                                const float w = (float)wq[j];
-                                kahan_add(fr[p], kr[p], w * er);
-                                kahan_add(fz[p], kz[p], w * ez);
-                                sa[p] += fabsf(w * er) + fabsf(w * ez);
-                            } else {
-                                // close to the ring: the term in float64, summed like the others
-                                double e64r, e64z;
-                                ring_field_far_cold(pr[p], 1.0 / pr[p], dz, rq[j], e64r, e64z);
-                                const float ter = (float)(wq[j] * e64r), tez = (float)(wq[j] * e64z);
-                                kahan_add(fr[p], kr[p], ter);
-                                kahan_add(fz[p], kz[p], tez);
-                                sa[p] += fabsf(ter) + fabsf(tez);
-                            }
-                        } else {
-                            double er, ez;
-                            ring_field_far<false, true>(pr[p], pinv[p], dz, rq[j], er, ez);
-                            ar[p] = fma(wq[j], er, ar[p]);
-                            az[p] = fma(wq[j], ez, az[p]);
-                        }
-                        ++far_evals;
+                    if (!in[j]) continue;
+                    const double dz = ze - zq[j];
+                    float er, ez;
+                    if (ring_far_f(ref, invf, (float)(re - rq[j]), (float)(re + rq[j]), (float)dz, (float)rq[j], er, ez)) {
+                        const float w = (float)wq[j];
+                        kahan_add(fr, kr, w * er);
+                        kahan_add(fz, kz, w * ez);
+                        sa += fabsf(w * er) + fabsf(w * ez);
+                    } else {
+                        // close to the ring: the term in float64, summed like the others
+                        double e64r, e64z;
+                        ring_field_far_cold(re, inv, dz, rq[j], e64r, e64z);
+                        const float ter = (float)(wq[j] * e64r), tez = (float)(wq[j] * e64z);
+                        kahan_add(fr, kr, ter);
+                        kahan_add(fz, kz, tez);
+                        sa += fabsf(ter) + fabsf(tez);
                     }
+                    ++cnt.far_evals;
                 }
+            } else {
+                double er = 0.0, ez = 0.0;
+                if (in[0]) {
+                    ring_field_far<false, true>(re, inv, ze - zq[0], rq[0], er, ez);
+                    ++cnt.far_evals;
+                }
+                tr_ = fma(wq[0], er, tr_);
+                tz_ = fma(wq[0], ez, tz_);
             }
+        }
+        if (!MIX) S.turn(tr_, tz_);
         }
         __syncwarp();  // the lists are rewritten by the next chunk
         }
     }
-    // fixed-order warp reduction; lane 0 writes the round's fields
-    bool redo = false;
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        if (MIX) {
-            ar[p] += (double)fr[p] - (double)kr[p];
-            az[p] += (double)fz[p] - (double)kz[p];
-        }
-        const double vr = warp_sum(ar[p]);
-        const double vz = warp_sum(az[p]);
-        const double va = MIX ? warp_sum((double)sa[p]) : 0.0;
-        if (lane == 0 && p < np_) {
-            const int k = r0 + p;
-            const double er = vr + P[8 * k + 7], ez = vz + c.ntmp[3 * k + 2];
-            P[8 * k + 5] = er;
-            P[8 * k + 6] = ez;
-            if (MIX) {
-                const double tz = ez + c.g.E_gun;
-                if (!(va <= c.kappa * sqrt(er * er + tz * tz))) redo = true;
-            }
-        }
+    if (MIX) {
+        mr = warp_sum(cr_ + ((double)fr - (double)kr));
+        mz = warp_sum(cz_ + ((double)fz - (double)kz));
+        mabs = warp_sum((double)sa);
     }
-    return __shfl_sync(0xffffffffu, redo, 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -1059,10 +1095,10 @@ __device__ bool far_adaptive_warp(Ctx& c, int r0, int np_, unsigned long long& f
 // also the closest segment, its parameter t and the distance, for the
 // surrogate's inputs.
 // One warp, record k.
-__device__ __forceinline__ void closest_point(Ctx& c, int k, bool frame) {
+__device__ __forceinline__ void closest_point(Ctx& c, double* P, int k, bool frame) {
     const SptBem& b = c.bem;
     const int lane = threadIdx.x & 31;
-    double* P = c.bpt;  // record k: [0]x [1]y [2]z [3]rho_e [4]z_e [5]ax [6]ay [7]near_r ; near_z in ntmp
+    // record k: [0]x [1]y [2]z [3]rho_e [4]z_e [5]ax [6]ay [7]near_r ; near_z in ntmp
     const int nseg = b.n_seg;
     {
         const double x = P[8 * k + 0], y = P[8 * k + 1], z = P[8 * k + 2];
@@ -1087,7 +1123,7 @@ __device__ __forceinline__ void closest_point(Ctx& c, int k, bool frame) {
                         const int s = (q0 + __ffs(cm) - 1) * SPT_BLOCK_SEGS + lane;
                         double proj, dist;
                         if (s < nseg) {
-                            seg_near(b, s, rho, z, proj, dist);
+                            seg_near<true>(b, s, rho, z, proj, dist);
                             hit |= !(dist > 1e-8 * segf(b, 4, s));
                         }
                     }
@@ -1167,24 +1203,21 @@ __device__ __forceinline__ void closest_point(Ctx& c, int k, bool frame) {
 
 static __device__ void bem_closest(Ctx& c, int n, bool frame) {
     // one warp per point
-    for (int k = threadIdx.x >> 5; k < n; k += c.nw) closest_point(c, k, frame);
+    for (int k = threadIdx.x >> 5; k < n; k += c.nw) closest_point(c, c.bpt, k, frame);
     __syncthreads();
 }
 
 
-// B for one record k, by one warp: the near-segment sinh quadrature
-// (bem/axisymmetric.py:566-600); lane 0 ends with near_r in record slot 7 and
-// near_z in ntmp[3k + 2].
+// B at (re, ze), by one warp: the near-segment sinh quadrature
+// (bem/axisymmetric.py:566-600) into S.  FAST (the adaptive rule): in rounds;
+// else every node into slot 0, in the reference rule's order.
 template <bool FAST>
-__device__ __forceinline__ void near_point(Ctx& c, int k, unsigned long long& n_near, unsigned long long& n_ring_near) {
+__device__ __forceinline__ void near_sums(Ctx& c, double re, double ze, PointSums& S, PointCounts& n) {
     const SptBem& b = c.bem;
     const int lane = threadIdx.x & 31;
-    double* P = c.bpt;
     const int nseg = b.n_seg;
     {
-        const double re = P[8 * k + 3], ze = P[8 * k + 4];
         const double inv = re > 0.0 ? 1.0 / re : 0.0;
-        double acc_r = 0.0, acc_z = 0.0;
         const int nblk = (nseg + SPT_BLOCK_SEGS - 1) / SPT_BLOCK_SEGS;
         for (int q0 = 0; q0 < nblk; q0 += 32) {
           // runs that may hold a near segment (every run without the bounds table)
@@ -1196,15 +1229,21 @@ __device__ __forceinline__ void near_point(Ctx& c, int k, unsigned long long& n_
             const int s0 = (q0 + jq) * SPT_BLOCK_SEGS;
             const int s = s0 + lane;
             double proj = 0.0, dist = 0.0;
-            const bool nr = (s < nseg) && seg_near(b, s, re, ze, proj, dist);
+            const bool nr = (s < nseg) && seg_near<FAST>(b, s, re, ze, proj, dist);
             unsigned mask = __ballot_sync(0xffffffffu, nr);
             // the sinh map's limits and intervals, by every near segment's lane at once
             double lo = 0.0, hi = 0.0;
             if (nr) {
                 const double Ls = segf(b, 4, s);
                 dist = fmax(dist, 1e-15 * Ls);
-                lo = asinh(-proj / dist);
-                hi = asinh((Ls - proj) / dist);
+                if constexpr (FAST) {  // the limits to 1e-16 absolute, as v is used
+                    const double id = rcp_pos(dist), a = proj * id, e = (Ls - proj) * id;
+                    lo = -log(a + sqrt_pos(fma(a, a, 1.0)));
+                    hi = log(e + sqrt_pos(fma(e, e, 1.0)));
+                } else {
+                    lo = asinh(-proj / dist);
+                    hi = asinh((Ls - proj) / dist);
+                }
             }
             while (mask) {
                 const int j = __ffs(mask) - 1;
@@ -1213,11 +1252,13 @@ __device__ __forceinline__ void near_point(Ctx& c, int k, unsigned long long& n_
                 const double sp = __shfl_sync(0xffffffffu, proj, j), d = __shfl_sync(0xffffffffu, dist, j);
                 const double v0 = __shfl_sync(0xffffffffu, lo, j), span = __shfl_sync(0xffffffffu, hi, j) - v0;
                 const int cnt = max(1, (int)ceil(span / 0.5));
-                const double width = span / cnt, half = 0.5 * width;
-                const double iL = 1.0 / segf(b, 4, sg);
+                const double width = FAST ? span * rcp_pos((double)cnt) : span / cnt, half = 0.5 * width;
+                const double iL = FAST ? rcp_pos(segf(b, 4, sg)) : 1.0 / segf(b, 4, sg);
                 const double p0r = segf(b, 0, sg), p0z = segf(b, 1, sg), ur = segf(b, 5, sg), uz = segf(b, 6, sg);
                 const double sg0 = segf(b, 9, sg), dsg = (segf(b, 10, sg) - sg0) * iL;
-                for (int qn = lane; qn < cnt * 8; qn += 32) {
+                for (int q0 = 0; q0 < cnt * 8; q0 += 32, ++S.round) {
+                    const int qn = q0 + lane;
+                    if ((FAST && !S.mine()) || qn >= cnt * 8) continue;
                     const int iv = qn >> 3, gi = qn & 7;
                     // A node's place is rounded at ulp(rho), 1e-10 of its distance at a picometre, so the
                     // reference rule takes sinh as accurate as the reference's; the adaptive rule takes sinh and
@@ -1237,44 +1278,57 @@ __device__ __forceinline__ void near_point(Ctx& c, int k, unsigned long long& n_
                     const double w = fma(sl, dsg, sg0) * (2.0 * kPi * sr) * d * ch * half * b.gauss8_w[gi];
                     double er, ez;
                     ring_field_far<true, FAST>(re, inv, ze - sz, sr, er, ez);
-                    acc_r = fma(w, er, acc_r);
-                    acc_z = fma(w, ez, acc_z);
+                    if constexpr (FAST) {
+                        S.add(w * er, w * ez);
+                    } else {
+                        S.r[0] = fma(w, er, S.r[0]);
+                        S.z[0] = fma(w, ez, S.z[0]);
+                    }
                 }
-                if (lane == 0) { n_near += 1; n_ring_near += (unsigned long long)cnt * 8; }
+                if (lane == 0 && S.share == 0) { n.n_near += 1; n.n_ring_near += (unsigned long long)cnt * 8; }
             }
           }
-        }
-        acc_r = warp_sum(acc_r);
-        acc_z = warp_sum(acc_z);
-        if (lane == 0) {
-            P[8 * k + 7] = acc_r;
-            c.ntmp[3 * k + 2] = acc_z;
         }
     }
 }
 
-// Adaptive far rule for record k, by this warp: float32 first in the mixed
-// form, float64 again when its sum is ill-conditioned.  The float64 tile is
-// the float64 form's, so with every sum redone the mixed form reproduces it.
-// Ring evaluations each lane keeps in flight in the float64 adaptive far sum.
-// One: every in-flight evaluation is an inlined copy of the ring kernel, and
-// the trace kernel is bound by instruction fetch, not by the latency the
-// copies would hide (whole C1 traces, 1184 groups: 8 in flight 8.9 M, 4 in
-// flight 12.1 M, 2 in flight 15.4 M, 1 in flight 18.3 M particle-steps/s).
-#ifndef SPT_FAR_NQ_FP64
-#define SPT_FAR_NQ_FP64 1
-#endif
+// The same for record k of the reference rule: lane 0 ends with near_r in slot
+// 7 and near_z in ntmp[3k + 2].
+__device__ __forceinline__ void near_point(Ctx& c, double* P, int k, PointCounts& n) {
+    PointSums S(0, 1);
+    near_sums<false>(c, P[8 * k + 3], P[8 * k + 4], S, n);
+    const double r = warp_sum(S.r[0]), z = warp_sum(S.z[0]);
+    if ((threadIdx.x & 31) == 0) {
+        P[8 * k + 7] = r;
+        c.ntmp[3 * k + 2] = z;
+    }
+}
 
+// The adaptive rule's near and far sums at (re, ze) into S.  The mixed form
+// sums in float32 first, and in float64 again when that sum is ill-conditioned
+// (its sum of |terms| above kappa times the whole field); it takes all rounds,
+// and its float64 sums are the float64 form's.
 template <int FORM>
-__device__ __forceinline__ void far_point(Ctx& c, int k, unsigned long long& fe, unsigned long long& ce) {
+__device__ __forceinline__ void adaptive_sums(Ctx& c, double re, double ze, PointSums& S, PointCounts& n) {
+    double mr, mz, mabs;
+    near_sums<true>(c, re, ze, S, n);
     if constexpr (FORM == SPT_FORM_FP64) {
-        far_adaptive_warp<1, SPT_FAR_NQ_FP64, false>(c, k, 1, fe, ce);
+        far_adaptive_warp<false>(c, re, ze, S, n, mr, mz, mabs);
     } else {
-        // float32 tiles keep 4 ring evaluations in flight per lane (8 spill at
-        // 128 registers; more resident warps supply the parallelism instead)
-        if (far_adaptive_warp<1, 4, true>(c, k, 1, fe, ce)) {
+        const int round = S.round;
+        double nr, nz;
+        S.total(nr, nz);
+        far_adaptive_warp<true>(c, re, ze, S, n, mr, mz, mabs);
+        const double er = nr + mr, tz = (nz + mz) + c.g.E_gun;
+        bool redo = !(mabs <= c.kappa * sqrt(er * er + tz * tz));
+        redo = __shfl_sync(0xffffffffu, redo, 0);
+        if (redo) {
             if ((threadIdx.x & 31) == 0) atomicAdd(c.cnt + SPT_CNT_FP64_ROUNDS, 1ull);
-            far_adaptive_warp<1, 8, false>(c, k, 1, fe, ce);
+            S.round = round;
+            far_adaptive_warp<false>(c, re, ze, S, n, mr, mz, mabs);
+        } else if ((threadIdx.x & 31) == 0) {
+            S.r[0] += mr;
+            S.z[0] += mz;
         }
     }
 }
@@ -1299,47 +1353,44 @@ __device__ __forceinline__ void bem_sums(Ctx& c, int n, int* status_flag) {
     const int nseg = b.n_seg;
     const int nps = b.nodes_per_seg;
     if (n <= 0) return;
-    // Adaptive rule with a field map: the map gives the points its cells hold
-    // (phases B and C then leave them out).
+    // adaptive rule with a field map: the map gives the points its cells hold
     const double* const map = FAR == SPT_FAR_ADAPTIVE ? field_map(b) : nullptr;
-    auto mapped = [&](int k) { return map && map_find(map, P[8 * k + 3], P[8 * k + 4]) >= 0; };
-    // B: near-segment sinh quadrature (one warp per point)
-    unsigned long long n_near = 0, n_ring_near = 0;
-    for (int k = warp; k < n; k += c.nw) {
-        if (mapped(k)) {
+    PointCounts cnt;
+    bool ok = true;
+    if constexpr (FAR == SPT_FAR_ADAPTIVE) {
+        // B + C: one point per warp task, taken dynamically
+        __shared__ int s_far_task;
+        __syncthreads();
+        if (tid == 0) s_far_task = c.nw;
+        __syncthreads();
+        for (int k = warp; k < n; k = next_task(&s_far_task)) {
+            const double re = P[8 * k + 3], ze = P[8 * k + 4];
+            const int leaf = map ? map_find(map, re, ze) : -1;
             double er, ez;
-            map_field(map, map_find(map, P[8 * k + 3], P[8 * k + 4]), P[8 * k + 3], P[8 * k + 4], er, ez);
+            if (leaf >= 0) {
+                map_field(map, leaf, re, ze, er, ez);
+                if (lane == 0) ++cnt.cl_evals;
+            } else {
+                PointSums S(0, 1);
+                adaptive_sums<FORM>(c, re, ze, S, cnt);
+                S.total(er, ez);
+            }
             if (lane == 0) {
                 P[8 * k + 5] = er;
                 P[8 * k + 6] = ez;
-                atomicAdd(c.cnt + SPT_CNT_CLUSTER_EVALS, 1ull);
             }
-        } else {
-            near_point<FAR == SPT_FAR_ADAPTIVE>(c, k, n_near, n_ring_near);
+            __syncwarp();
         }
-    }
-    count_add(c, SPT_CNT_NEAR_PAIRS, n_near);
-    count_add(c, SPT_CNT_RING_NEAR, n_ring_near);
-    __syncthreads();
-
-    // C: far sum.  Adaptive rule: rounds of up to c.round_pts points, each
-    // owned by one warp (as many rounds as warps where the points allow, so
-    // no warp waits for another until the end).  Reference rule: rounds over
-    // TMA-staged node tiles shared by the whole CTA; the round's point count
-    // selects how many nodes each thread keeps in flight.
-    unsigned long long far_evals = 0;
-    bool ok = true;
-    if constexpr (FAR == SPT_FAR_ADAPTIVE) {
-        // one point per warp task, taken dynamically
-        __shared__ int s_far_task;
-        if (tid == 0) s_far_task = c.nw;
         __syncthreads();
-        unsigned long long cl_evals = 0;
-        for (int k = warp; k < n; k = next_task(&s_far_task))
-            if (!mapped(k)) far_point<FORM>(c, k, far_evals, cl_evals);
-        count_add(c, SPT_CNT_CLUSTER_EVALS, cl_evals);
-        __syncthreads();
+        count_points(c, cnt);
     } else {
+        // B: near-segment sinh quadrature (one warp per point)
+        for (int k = warp; k < n; k += c.nw) near_point(c, P, k, cnt);
+        count_points(c, cnt);
+        __syncthreads();
+        // C: far sum, rounds over TMA-staged node tiles shared by the whole CTA;
+        // the round's point count selects how many nodes each thread keeps in flight
+        unsigned long long far_evals = 0;
         const int tile_cap = c.L.tile_cap;
         const int segs_per_tile = min(tile_cap / nps, 256);
         const int n_tiles = (nseg + segs_per_tile - 1) / segs_per_tile;
@@ -1367,9 +1418,9 @@ __device__ __forceinline__ void bem_sums(Ctx& c, int n, int* status_flag) {
                 }
             }
         }
+        count_add(c, SPT_CNT_RING_FAR, far_evals);
     }
     if (!ok && tid == 0) *status_flag = SPT_GROUP_TIMEOUT;
-    count_add(c, SPT_CNT_RING_FAR, far_evals);
 }
 
 // D: rotate E_rho of records [0, n) into (x, y) (record slots 5, 6, 7 = ex, ey, ez)
@@ -1630,13 +1681,105 @@ __device__ void surrogate_points(Ctx& c, int n, int* status_flag) {
     bem_rotate(c, n, false);
 }
 
-// BEM field of the n points listed in c.bpt (x, y, z at slots 0..2 of each
-// 8-double record): the reference's evaluation, phases A-D.
+// Direct field of the point (x, y, z) by this warp, or its share of it: on-surface
+// offset, near quadrature and adaptive far sum into S.  Uses the warp's own
+// record c.wrec.
+template <int FORM>
+__device__ __forceinline__ void direct_sums(Ctx& c, double x, double y, double z, PointSums& S, PointCounts& n) {
+    double* const P = c.wrec;
+    if ((threadIdx.x & 31) == 0) {
+        P[0] = x;
+        P[1] = y;
+        P[2] = z;
+    }
+    __syncwarp();
+    closest_point(c, P, 0, false);
+    __syncwarp();
+    adaptive_sums<FORM>(c, P[3], P[4], S, n);
+    __syncwarp();
+}
+
+// The same for the whole point, rotated; lane 0 returns it.
+template <int FORM>
+__device__ __forceinline__ void direct_point(Ctx& c, double x, double y, double z, PointCounts& n, double& ex,
+                                             double& ey, double& ez) {
+    PointSums S(0, 1);
+    direct_sums<FORM>(c, x, y, z, S, n);
+    double er;
+    S.total(er, ez);
+    rotate_rho(x, y, hypot(x, y), er, ex, ey);
+}
+
+// Direct points of a CTA with fewer points than half its warps: each point's
+// rounds are shared by 2 or 4 warps (a point is a chain of ~15 rounds of one
+// ring evaluation per lane, 20 us on one warp, and the CTA waits for it).  A
+// warp leaves its slots, lane by lane, in `part`; after a barrier the point's
+// warp adds them as PointSums::total does.
+__device__ __forceinline__ int split_shares(int n, int warps) {
+    return 4 * n <= warps ? 4 : (2 * n <= warps ? 2 : 1);
+}
+__device__ __forceinline__ void split_store(const PointSums& S, double* part) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if ((k & (S.shares - 1)) == S.share) {
+            part[64 * k + lane] = S.r[k];
+            part[64 * k + 32 + lane] = S.z[k];
+        }
+}
+__device__ __forceinline__ void split_total(const double* part, double& er, double& ez) {
+    const int lane = threadIdx.x & 31;
+    const double* p = part + lane;
+    er = warp_sum((p[0] + p[64]) + (p[128] + p[192]));
+    ez = warp_sum((p[32] + p[96]) + (p[160] + p[224]));
+}
+
+// BEM field of the particles c.list[0..n) into c.fld, float64 adaptive form:
+// one point a warp task, or its shares while there are few points.
+__device__ __forceinline__ void bem_points_direct(Ctx& c, int n) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, E = c.E;
+    const double* sp = c.sp;
+    double* const part = c.tiles + (size_t)c.nw * (kWarpScratchInts / 2);
+    __shared__ int s_task;
+    const int shares = split_shares(n, c.nw);
+    if (threadIdx.x == 0) s_task = c.nw;
+    __syncthreads();
+    PointCounts cnt;
+    auto store = [&](int i, double er, double ez) {  // lane 0
+        double ex, ey;
+        rotate_rho(sp[i], sp[E + i], hypot(sp[i], sp[E + i]), er, ex, ey);
+        c.fld[3 * i + 0] = ex;
+        c.fld[3 * i + 1] = ey;
+        c.fld[3 * i + 2] = ez;
+    };
+    for (int t = warp; t < n * shares; t = next_task(&s_task)) {
+        const int k = t / shares, i = c.list[k];
+        PointSums S(t - k * shares, shares);
+        direct_sums<SPT_FORM_FP64>(c, sp[i], sp[E + i], sp[2 * E + i], S, cnt);
+        if (shares == 1) {
+            double er, ez;
+            S.total(er, ez);
+            if (lane == 0) store(i, er, ez);
+        } else {
+            split_store(S, part + 256 * k);
+        }
+    }
+    if (shares > 1) {
+        __syncthreads();
+        for (int k = warp; k < n; k += c.nw) {
+            double er, ez;
+            split_total(part + 256 * k, er, ez);
+            if (lane == 0) store(c.list[k], er, ez);
+        }
+    }
+    count_points(c, cnt);
+    __syncthreads();
+}
+
 // BEM field of the records [0, n) with the adaptive far rule, each point one
 // warp task from start to end -- closest segment and on-surface offset, near
 // quadrature, far sum, rotation -- taken dynamically from a CTA counter, so
-// the only barrier is the one at the end.  Same arithmetic as the phased
-// path (bem_closest, bem_sums, bem_rotate).
+// the only barrier is the one at the end.
 template <int FORM>
 __device__ void bem_points_fused(Ctx& c, int n) {
     const int lane = threadIdx.x & 31;
@@ -1644,35 +1787,24 @@ __device__ void bem_points_fused(Ctx& c, int n) {
     __shared__ int s_task;
     if (threadIdx.x == 0) s_task = c.nw;
     __syncthreads();
-    unsigned long long n_near = 0, n_ring_near = 0, far_evals = 0, cl_evals = 0;
+    PointCounts cnt;
     for (int k = threadIdx.x >> 5; k < n; k = next_task(&s_task)) {
-        closest_point(c, k, false);
-        __syncwarp();
-        near_point<true>(c, k, n_near, n_ring_near);
-        __syncwarp();
-        far_point<FORM>(c, k, far_evals, cl_evals);
+        double ex, ey, ez;
+        direct_point<FORM>(c, P[8 * k + 0], P[8 * k + 1], P[8 * k + 2], cnt, ex, ey, ez);
         if (lane == 0) {
-            const double x = P[8 * k + 0], y = P[8 * k + 1];
-            const double rho = hypot(x, y);
-            const double e_rho = P[8 * k + 5], e_z = P[8 * k + 6];
-            double ex = 0.0, ey = 0.0;
-            if (rho != 0.0) {
-                ex = e_rho * (x / rho);
-                ey = e_rho * (y / rho);
-            }
             P[8 * k + 5] = ex;
             P[8 * k + 6] = ey;
-            P[8 * k + 7] = e_z;
+            P[8 * k + 7] = ez;
         }
         __syncwarp();
     }
-    count_add(c, SPT_CNT_NEAR_PAIRS, n_near);
-    count_add(c, SPT_CNT_RING_NEAR, n_ring_near);
-    count_add(c, SPT_CNT_RING_FAR, far_evals);
-    count_add(c, SPT_CNT_CLUSTER_EVALS, cl_evals);
+    count_points(c, cnt);
     __syncthreads();
 }
 
+// BEM field of the n points listed in c.bpt (x, y, z at slots 0..2 of each
+// 8-double record): the reference's evaluation, phases A-D, or the adaptive
+// rule's one task per point.
 template <int FORM, int FAR>
 __device__ void bem_points(Ctx& c, int n, bool scatter, int* status_flag) {
     if constexpr (FAR == SPT_FAR_ADAPTIVE) {
@@ -1778,12 +1910,12 @@ __device__ void stage_accel(Ctx& c, double* out, int* status_flag) {
 
     // 1. external field
     if constexpr (!GIVEN && (KIND == SPT_GEOM_TIP_BEM || KIND == SPT_GEOM_WELL_BEM || KIND == SPT_GEOM_POST_BEM)) {
-        // Field map (float64 adaptive form): warp w takes particles w, w + nw,
+        // Field map (float64 and mixed forms): warp w takes particles w, w + nw,
         // ... (one per lane, spread over all warps of a small group), the
         // mapped ones are evaluated here and the rest compacted into c.list;
         // without a map every particle that needs the field is listed.
         const double* map = nullptr;
-        if constexpr (FORM == SPT_FORM_FP64 && FAR == SPT_FAR_ADAPTIVE) map = field_map(c.bem);
+        if constexpr (FORM != SPT_FORM_SURROGATE && FAR == SPT_FAR_ADAPTIVE) map = field_map(c.bem);
         for (int i = tid; i < 3 * E; i += c.nt) c.fld[i] = 0.0;
         __shared__ int s_wcount[kMaxWarps + 1];
         int n_list = 0;
@@ -1827,15 +1959,19 @@ __device__ void stage_accel(Ctx& c, double* out, int* status_flag) {
             if (need) {
                 const int pos = n_list + s_wcount[tid >> 5] + __popc(bal & ((1u << (tid & 31)) - 1u));
                 c.list[pos] = i;
-                c.bpt[8 * pos + 0] = sx[i];
-                c.bpt[8 * pos + 1] = sy[i];
-                c.bpt[8 * pos + 2] = sz[i];
+                if constexpr (!(FORM == SPT_FORM_FP64 && FAR == SPT_FAR_ADAPTIVE)) {
+                    c.bpt[8 * pos + 0] = sx[i];
+                    c.bpt[8 * pos + 1] = sy[i];
+                    c.bpt[8 * pos + 2] = sz[i];
+                }
             }
             n_list += s_wcount[c.nw];
             __syncthreads();
         }
         if (n_list > 0) {
-            c.ntmp = map ? c.img : c.fld;
+            if constexpr (FORM == SPT_FORM_FP64 && FAR == SPT_FAR_ADAPTIVE) {
+                bem_points_direct(c, n_list);
+            } else {
             if constexpr (FORM == SPT_FORM_SURROGATE)
                 surrogate_points<FAR>(c, n_list, status_flag);
             else
@@ -1846,6 +1982,7 @@ __device__ void stage_accel(Ctx& c, double* out, int* status_flag) {
                 c.fld[3 * i + 0] = c.bpt[8 * k + 5];
                 c.fld[3 * i + 1] = c.bpt[8 * k + 6];
                 c.fld[3 * i + 2] = c.bpt[8 * k + 7];
+            }
             }
         }
         __syncthreads();
@@ -2531,12 +2668,12 @@ accel_kernel(const __grid_constant__ SptAccelArgs a, const __grid_constant__ Spt
 
 constexpr int kWarpSlotComps = 54;  // y0 6, 5th-order solution 6, stage velocities 21, stage accelerations 21
 constexpr int kWarpSlotDoubles = kWarpSlotComps * 32;
-// per-warp shared doubles: BEM record 8, near-sum scratch 4, stage positions
-// and charges 4 x 32, sphere images 4 x 32, BEM fields 3 x 32, live flags 32 ints
-constexpr int kWarpTeamDoubles = 8 + 4 + 4 * 32 + 4 * 32 + 3 * 32 + 16;
+// per-warp shared doubles: BEM record 8, stage positions and charges 4 x 32,
+// sphere images 4 x 32, BEM fields 3 x 32, live flags 32 ints
+constexpr int kWarpTeamDoubles = 8 + 4 * 32 + 4 * 32 + 3 * 32 + 16;
 
 __host__ __device__ inline size_t warp_team_smem(int warps) {
-    return (size_t)warps * ((size_t)kWarpScratchInts * 4 + (size_t)kWarpTeamDoubles * 8);
+    return (size_t)warps * ((size_t)kWarpScratchInts * 4 + (size_t)kWarpTeamDoubles * 8) + kSplitDoubles * 8;
 }
 
 __device__ __forceinline__ double warp_min_all(double v) {
@@ -2547,13 +2684,12 @@ __device__ __forceinline__ double warp_min_all(double v) {
 
 // per-warp shared region of warp w
 struct WarpTeam {
-    double *rec, *nfld, *sx, *sy, *sz, *q, *img, *fld;
+    double *rec, *sx, *sy, *sz, *q, *img, *fld;
     int* live;
     __device__ WarpTeam(double* smem, int nw, int w) {
         double* t = smem + (size_t)nw * kWarpScratchInts / 2 + (size_t)w * kWarpTeamDoubles;
         rec = t;
-        nfld = t + 8;
-        sx = t + 12;
+        sx = t + 8;
         sy = sx + 32;
         sz = sy + 32;
         q = sz + 32;
@@ -2563,65 +2699,58 @@ struct WarpTeam {
     }
 };
 
-// Direct field of the point (x, y, z) by this warp (closest segment, near
-// quadrature, adaptive far sum, rotation); lane 0 returns it.  Uses the
-// warp's own record c.bpt and near sum c.ntmp.
-struct PointCounts {
-    unsigned long long n_near = 0, n_ring_near = 0, far_evals = 0, cl_evals = 0;
-};
-
-template <int FORM>
-__device__ __forceinline__ void direct_point(Ctx& c, double x, double y, double z, PointCounts& n, double& ex,
-                                             double& ey, double& ez) {
-    double* const P = c.bpt;
-    if ((threadIdx.x & 31) == 0) {
-        P[0] = x;
-        P[1] = y;
-        P[2] = z;
-    }
-    __syncwarp();
-    closest_point(c, 0, false);
-    __syncwarp();
-    near_point<true>(c, 0, n.n_near, n.n_ring_near);
-    __syncwarp();
-    far_point<FORM>(c, 0, n.far_evals, n.cl_evals);
-    __syncwarp();
-    rotate_rho(x, y, hypot(x, y), P[5], ex, ey);
-    ez = P[6];
-    __syncwarp();
-}
-
-__device__ __forceinline__ void count_points(Ctx& c, const PointCounts& n) {
-    count_add(c, SPT_CNT_NEAR_PAIRS, n.n_near);
-    count_add(c, SPT_CNT_RING_NEAR, n.n_ring_near);
-    count_add(c, SPT_CNT_RING_FAR, n.far_evals);
-    count_add(c, SPT_CNT_CLUSTER_EVALS, n.cl_evals);
-}
-
-// The CTA's BEM task pool of one stage: entries (warp << 5 | particle),
-// drawn one per warp task; every warp calls, between the barriers that close
-// the appends and open the next stage.
-template <int FORM>
+// The CTA's BEM task pool of one stage: entries (warp << 5 | particle), drawn
+// one per warp task, or each shared by 2 or 4 warps while there are few; every
+// warp calls, between the barriers that close the appends and open the next
+// stage.  Shared points' slots end in `part` (pool_totals adds them).
 __device__ __forceinline__ void pool_bem_points(Ctx& c, double* smem, const int* entries, int count, int* next,
-                                                PointCounts& n) {
+                                                double* part, PointCounts& n) {
     const int lane = threadIdx.x & 31;
+    const int shares = split_shares(count, c.nw);
     for (;;) {
         int t = 0;
         if (lane == 0) t = atomicAdd(next, 1);
         t = __shfl_sync(0xffffffffu, t, 0);
-        if (t >= count) break;
-        const int e = entries[t];
+        if (t >= count * shares) break;
+        const int e = entries[t / shares];
         const WarpTeam own(smem, c.nw, e >> 5);
         const int k = e & 31;
-        double ex, ey, ez;
-        direct_point<FORM>(c, own.sx[k], own.sy[k], own.sz[k], n, ex, ey, ez);
-        if (lane == 0) {
-            own.fld[3 * k + 0] = ex;
-            own.fld[3 * k + 1] = ey;
-            own.fld[3 * k + 2] = ez;
+        PointSums S(t & (shares - 1), shares);
+        direct_sums<SPT_FORM_FP64>(c, own.sx[k], own.sy[k], own.sz[k], S, n);
+        if (shares == 1) {
+            double er, ez, ex, ey;
+            S.total(er, ez);
+            if (lane == 0) {
+                rotate_rho(own.sx[k], own.sy[k], hypot(own.sx[k], own.sy[k]), er, ex, ey);
+                own.fld[3 * k + 0] = ex;
+                own.fld[3 * k + 1] = ey;
+                own.fld[3 * k + 2] = ez;
+            }
+        } else {
+            split_store(S, part + 256 * (t / shares));
         }
         __syncwarp();
     }
+}
+
+// The shared points of this warp's own group (after the barrier).
+__device__ __forceinline__ void pool_totals(Ctx& c, const WarpTeam& w, const int* entries, int count,
+                                            const double* part) {
+    if (split_shares(count, c.nw) == 1) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int t = 0; t < count; ++t) {
+        if ((entries[t] >> 5) != warp) continue;
+        const int k = entries[t] & 31;
+        double er, ez, ex, ey;
+        split_total(part + 256 * t, er, ez);
+        if (lane == 0) {
+            rotate_rho(w.sx[k], w.sy[k], hypot(w.sx[k], w.sy[k]), er, ex, ey);
+            w.fld[3 * k + 0] = ex;
+            w.fld[3 * k + 1] = ey;
+            w.fld[3 * k + 2] = ez;
+        }
+    }
+    __syncwarp();
 }
 
 // The rest of a stage for this warp's group, after the pool: images, pair
@@ -2733,8 +2862,8 @@ trace_warp_kernel(const __grid_constant__ SptState st, const __grid_constant__ S
     c.nw = nw;
     c.tiles = smem;  // far-rule scratch of every warp (far_adaptive_warp takes its own by warp index)
     const WarpTeam w(smem, nw, warp);
-    c.bpt = w.rec;
-    c.fld = c.ntmp = w.nfld;
+    c.wrec = w.rec;
+    double* const part = smem + (warp_team_smem(nw) / 8 - kSplitDoubles);
     const double* const map = field_map(bem);
     PointCounts pts;
     c.live = w.live;
@@ -2932,8 +3061,9 @@ trace_warp_kernel(const __grid_constant__ SptState st, const __grid_constant__ S
             }
             const int n_direct = s_pool_n[pp];
             if (n_direct > 0) {  // alike in every thread
-                pool_bem_points<FORM>(c, smem, s_pool[pp], n_direct, &s_pool_next[pp], pts);
+                pool_bem_points(c, smem, s_pool[pp], n_direct, &s_pool_next[pp], part, pts);
                 __syncthreads();
+                pool_totals(c, w, s_pool[pp], n_direct, part);
             }
             if (run) {
                 double ax, ay, az;

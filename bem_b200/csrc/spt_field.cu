@@ -24,8 +24,8 @@ __device__ __forceinline__ bool field_wanted(const FieldMask& m, long long i, do
     return bem_valid<SPT_GEOM_POST_BEM>(x, y, z, m.g);
 }
 
-// The adaptive rule: a CTA takes `chunk` points (8 to 256: one a warp while
-// there are few).  Every thread finds its point's cell
+// The adaptive rule: a CTA takes `chunk` points (1 to 256: fewer than its warps
+// while that leaves SMs free, so that a point's direct sums are shared).  Every thread finds its point's cell
 // of the field map; mapped points are evaluated by the warp they sit in, the
 // others (near the surface, or no map) go to a task list that all warps of the
 // CTA draw from, one warp a point.
@@ -35,7 +35,7 @@ field_points_kernel(const double* x, const double* y, const double* z, long long
                     double* ez) {
     extern __shared__ __align__(16) double smem[];
     __shared__ SptGeometry s_geo;
-    __shared__ double s_p[3 * kMaxThreads];
+    __shared__ double s_p[3 * kMaxThreads], s_rec[kMaxWarps][8];
     __shared__ int s_task[kMaxThreads];
     __shared__ int s_n, s_next;
     __shared__ unsigned long long s_cnt[SPT_N_COUNTERS];
@@ -47,15 +47,14 @@ field_points_kernel(const double* x, const double* y, const double* z, long long
     c.nw = kMaxWarps;
     c.cnt = s_cnt;
     c.tiles = smem;
-    c.bpt = smem + kMaxWarps * kWarpScratchInts / 2 + 12 * warp;
-    c.fld = c.ntmp = c.bpt + 8;
+    c.wrec = s_rec[warp];
     const double* const map = field_map(bem);
     // point of this thread: lane + 32 warp of a full chunk, fewer lanes a warp in a small one
-    const int per_warp = chunk / kMaxWarps;
+    const int per_warp = (chunk + kMaxWarps - 1) / kMaxWarps;
     long long end;
     const long long first = field_range(mask, n, end) + blockIdx.x * (long long)chunk;
     const long long i = first + warp * per_warp + lane;
-    bool in = lane < per_warp && i < end;
+    bool in = lane < per_warp && warp * per_warp + lane < chunk && i < end;
     double px = 0.0, py = 0.0, pz = 0.0;
     int leaf = -1;
     if (in) {
@@ -83,21 +82,37 @@ field_points_kernel(const double* x, const double* y, const double* z, long long
         s_task[atomicAdd(&s_n, 1)] = tid;
     }
     __syncthreads();
-    const int n_direct = s_n;
+    const int n_direct = s_n, shares = chunk < kMaxWarps ? split_shares(n_direct, kMaxWarps) : 1;
+    double* const part = smem + kMaxWarps * (kWarpScratchInts / 2);
     PointCounts pts;
+    auto store = [&](int k, double er, double fz) {  // lane 0
+        double fx, fy;
+        rotate_rho(s_p[k], s_p[kMaxThreads + k], hypot(s_p[k], s_p[kMaxThreads + k]), er, fx, fy);
+        const long long o = first + (k >> 5) * per_warp + (k & 31);
+        ex[o] = fx;
+        ey[o] = fy;
+        ez[o] = fz;
+    };
     for (;;) {
         const int t = next_task(&s_next);
-        if (t >= n_direct) break;
-        const int k = s_task[t];
-        double fx, fy, fz;
-        direct_point<SPT_FORM_FP64>(c, s_p[k], s_p[kMaxThreads + k], s_p[2 * kMaxThreads + k], pts, fx, fy, fz);
-        if (lane == 0) {
-            const long long o = first + (k >> 5) * per_warp + (k & 31);
-            ex[o] = fx;
-            ey[o] = fy;
-            ez[o] = fz;
+        if (t >= n_direct * shares) break;
+        const int k = s_task[t / shares];
+        PointSums S(t & (shares - 1), shares);
+        direct_sums<SPT_FORM_FP64>(c, s_p[k], s_p[kMaxThreads + k], s_p[2 * kMaxThreads + k], S, pts);
+        if (shares == 1) {
+            double er, fz;
+            S.total(er, fz);
+            if (lane == 0) store(k, er, fz);
+        } else {
+            split_store(S, part + 256 * (t / shares));
         }
-        __syncwarp();
+    }
+    if (shares == 1) return;
+    __syncthreads();
+    for (int t = warp; t < n_direct; t += kMaxWarps) {
+        double er, fz;
+        split_total(part + 256 * t, er, fz);
+        if (lane == 0) store(s_task[t], er, fz);
     }
 }
 
@@ -129,7 +144,7 @@ field_quad_kernel(const double* x, const double* y, const double* z, long long n
     c.nw = kMaxWarps;
     c.cnt = s_cnt;
     c.bpt = s_rec[slot];  // the record of the point, shared by its warps
-    c.fld = c.ntmp = c.bpt + 8;
+    c.ntmp = c.bpt + 8;
     // (a CTA of the cluster may write to another's shared memory only once that one has started)
     if (ranks > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     double px = 0.0, py = 0.0, pz = 0.0;
@@ -140,7 +155,7 @@ field_quad_kernel(const double* x, const double* y, const double* z, long long n
         pz = z[i];
         in = field_wanted(mask, i, px, py, pz);
     }
-    unsigned long long n_near = 0, n_ring = 0;
+    PointCounts cnt;
     if (in && sub == 0) {
         if (lane == 0) {
             c.bpt[0] = px;
@@ -149,7 +164,7 @@ field_quad_kernel(const double* x, const double* y, const double* z, long long n
             c.bpt[7] = c.ntmp[2] = 0.0;
         }
         __syncwarp();
-        closest_point(c, 0, false);
+        closest_point(c, c.bpt, 0, false);
         __syncwarp();
     }
     if (in_cta > 1) __syncthreads();
@@ -193,7 +208,7 @@ field_quad_kernel(const double* x, const double* y, const double* z, long long n
         }
         ar = warp_sum(ar);
         az = warp_sum(az);
-        if (part == 0) near_point<false>(c, 0, n_near, n_ring);
+        if (part == 0) near_point(c, c.bpt, 0, cnt);
     }
     if (in_cta > 1) {
         // partial sums to the first rank's shared memory
@@ -237,10 +252,11 @@ int launch_field(const double* x, const double* y, const double* z, long long n,
                  const FieldMask& mask, double* ex, double* ey, double* ez, cudaStream_t st) {
     constexpr long long kWarps = 148 * 2 * kMaxWarps;  // resident warps: two CTAs of 128 registers a thread on each SM
     if (b.far_rule == SPT_FAR_ADAPTIVE) {
-        // chunks of 8 points (one a warp) until the SMs are full, then larger ones
-        long long chunk = 8 * ((n + kWarps - 1) / kWarps);
+        // 1, 2, 4 points a CTA while every CTA finds a place at once, then chunks of 8 a resident warp
+        constexpr long long kCtas = 148 * 2;
+        long long chunk = n <= kCtas ? 1 : (n <= 2 * kCtas ? 2 : (n <= 4 * kCtas ? 4 : 8 * ((n + kWarps - 1) / kWarps)));
         if (chunk > kMaxThreads) chunk = kMaxThreads;
-        const size_t smem = kMaxWarps * (kWarpScratchInts * 4 + 12 * 8);
+        const size_t smem = kMaxWarps * (kWarpScratchInts * 4) + (chunk < kMaxWarps ? kSplitDoubles * 8 : 0);
         const long long grid = (n + chunk - 1) / chunk;
         if (grid > 0x7fffffffLL) return -1;
         const cudaError_t e = cudaFuncSetAttribute(field_points_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

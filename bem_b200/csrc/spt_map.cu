@@ -74,25 +74,19 @@ map_cells_kernel(const double* cells, const __grid_constant__ SptBem bem, const 
     c.nw = kMaxWarps;
     c.cnt = s_cnt;
     c.tiles = smem;
-    c.bpt = smem + kMaxWarps * kWarpScratchInts / 2 + 12 * warp;
-    c.fld = c.ntmp = c.bpt + 8;
     __syncthreads();
-    unsigned long long fe = 0, ce = 0;
+    PointCounts cnt;
     for (;;) {
         const int t = next_task(&s_next);
         if (t >= kMapN2) break;
-        double* P = c.bpt;
+        // rho: row i, z: row j; no panel is near
+        PointSums S(0, 1);
+        double er, ez, mr, mz, mabs;
+        far_adaptive_warp<false>(c, rc + h * s_x[t / N], zc + h * s_x[t % N], S, cnt, mr, mz, mabs);
+        S.total(er, ez);
         if (lane == 0) {
-            P[3] = rc + h * s_x[t / N];  // rho: row i
-            P[4] = zc + h * s_x[t % N];
-            P[7] = 0.0;                  // no near panel
-            c.ntmp[2] = 0.0;
-        }
-        __syncwarp();
-        far_point<SPT_FORM_FP64>(c, 0, fe, ce);
-        if (lane == 0) {
-            s_f[t] = P[5];
-            s_f[kMapN2 + t] = P[6];
+            s_f[t] = er;
+            s_f[kMapN2 + t] = ez;
         }
         __syncwarp();
     }
@@ -175,7 +169,7 @@ extern "C" int spt_map_cells(const double* cells, int32_t n, const SptBem* b, co
     if (rc) return rc;
     if (b->far_rule != SPT_FAR_ADAPTIVE || !b->node || !b->coarse || b->nodes_per_seg <= 0 || b->reserved)
         return fail(SPT_ERR_ARG, "spt_map_cells: needs the adaptive far rule's tables, without a map");
-    const size_t smem = spt::kMaxWarps * (spt::kWarpScratchInts * 4 + 12 * 8);
+    const size_t smem = spt::kMaxWarps * spt::kWarpScratchInts * 4;
     spt::map_cells_kernel<<<(unsigned)n, spt::kMaxThreads, smem, static_cast<cudaStream_t>(stream)>>>(
         cells, *b, cheb, dct, mono, rec, tail);
     return cuda_check(cudaGetLastError(), "map_cells_kernel launch");

@@ -156,10 +156,11 @@ typedef struct {
      * ratio4 >= 1 (coarse segments are never near), ratio2 >= ratio4. */
     int32_t far_rule;
     /* 0, or SPT_MAP_TAG << 16 | u: a field map (spt_map_cells) starts u *
-     * SPT_MAP_UNIT doubles after `clusters`.  The float64 form of the adaptive
-     * far rule reads the field of the points its cells hold from it; the
-     * other points, forms and rule sum directly.  The map stands for the
-     * field itself: it takes precedence over the thresholds below. */
+     * SPT_MAP_UNIT doubles after `clusters`.  With the adaptive far rule the
+     * float64 form, the mixed form's stages and the learned form's exact sums
+     * read the field of the points its cells hold from it; the other points
+     * and the reference rule sum directly.  The map stands for the field
+     * itself: it takes precedence over the thresholds below. */
     int32_t reserved;
     double ratio4;
     double ratio2;
