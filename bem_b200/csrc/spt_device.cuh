@@ -180,7 +180,7 @@ struct Layout {
     int red;                  // kMaxWarps * 3 * kRound (far-round reduction: E_rho, E_z, sum of |terms|)
     int ints;                 // int region start (in doubles)
     int total_doubles;
-    int live_off, list_off, flags_off;  // in ints from ints start
+    int live_off, list_off, lidx_off, flags_off;  // in ints from ints start
     size_t bytes;
     bool big;                 // slopes/y0/nw in global memory
 };
@@ -206,12 +206,15 @@ constexpr int kSplitDoubles = kSplitPoints * 256;  // per point: 4 slots x 2 com
 // warp of a CTA of `warps` warps.  want_tiles false: neither (paths that
 // evaluate no far sum).
 __host__ __device__ inline Layout make_layout(int E, int far_rule, bool want_sur = false, bool want_tiles = true,
-                                              int warps = kMaxWarps, int img_doubles = 0) {
+                                              int warps = kMaxWarps, int img_doubles = 0, bool slopes = true) {
     Layout L;
     const bool big = E > kSmallGroup;
     int o = 0;
     L.big = big;
-    if (!big) {
+    if (!slopes) {  // one stage only: its result
+        L.y0 = L.nw = L.kp = 0;
+        L.kv = o; o += 3 * E;
+    } else if (!big) {
         L.y0 = o; o += 6 * E;
         L.nw = o; o += 6 * E;
         L.kp = o; o += 21 * E;
@@ -237,7 +240,7 @@ __host__ __device__ inline Layout make_layout(int E, int far_rule, bool want_sur
     }
     o = (o + 1) & ~1;  // 16-byte alignment for the TMA tiles
     const int base = o;
-    const int n_ints = 2 * E + kRound * 256 / 4 + 4;  // live, list, near flags (bytes) packed in ints
+    const int n_ints = 3 * E + kRound * 256 / 4 + 4;  // live, list, live list, near flags (bytes), redo flag, live count
     const bool tiles = want_tiles && far_rule == SPT_FAR_REFERENCE;
     const bool lists = want_tiles && far_rule != SPT_FAR_REFERENCE;
     for (int cap = kTileNodes; cap >= 256; cap >>= 1) {
@@ -252,7 +255,8 @@ __host__ __device__ inline Layout make_layout(int E, int far_rule, bool want_sur
     }
     L.live_off = 0;
     L.list_off = E;
-    L.flags_off = 2 * E;
+    L.lidx_off = 2 * E;
+    L.flags_off = 3 * E;
     return L;
 }
 
@@ -295,6 +299,8 @@ struct Ctx {
     double* wrec;    // adaptive rule: this warp's record (8 doubles)
     int* live;
     int* list;
+    int* lidx;       // live particles in order
+    int* nl;         // and their number
     unsigned char* nflag;
     uint64_t* bars;
     uint32_t phase[3];          // parity of the next phase to wait for on bars[0..2] (identical in every thread)
@@ -321,12 +327,12 @@ __device__ __forceinline__ void count_add(Ctx& c, int k, unsigned long long v) {
 }
 
 __device__ inline void bind(Ctx& c, double* smem, int E, int far_rule, double* slot, unsigned long long* s_cnt,
-                            bool sur = false, bool tiles = true) {
+                            bool sur = false, bool tiles = true, bool slopes = true) {
     c.base = smem;
     c.E = E;
     c.nt = blockDim.x;
     c.nw = blockDim.x >> 5;
-    c.L = make_layout(E, far_rule, sur, tiles, blockDim.x >> 5, image_scratch(c.g, c.bem, E, blockDim.x));
+    c.L = make_layout(E, far_rule, sur, tiles, blockDim.x >> 5, image_scratch(c.g, c.bem, E, blockDim.x), slopes);
     c.round_pts = kRound;
     c.kappa = kKappa;
     c.cnt = s_cnt;
@@ -359,8 +365,10 @@ __device__ inline void bind(Ctx& c, double* smem, int E, int far_rule, double* s
     int* ib = reinterpret_cast<int*>(smem + L.ints);
     c.live = ib + L.live_off;
     c.list = ib + L.list_off;
+    c.lidx = ib + L.lidx_off;
     c.nflag = reinterpret_cast<unsigned char*>(ib + L.flags_off);
     c.redo = ib + L.flags_off + kRound * 256 / 4;  // first spare int after the near-flag bytes
+    c.nl = c.redo + 1;
     c.bars = reinterpret_cast<uint64_t*>(smem + L.total_doubles + 1);
     for (int k = threadIdx.x; k < SPT_N_COUNTERS; k += blockDim.x) s_cnt[k] = 0;
     if (L.sur >= 0) {
@@ -1253,36 +1261,35 @@ __device__ __forceinline__ void near_sums(Ctx& c, double re, double ze, PointSum
                 const double v0 = __shfl_sync(0xffffffffu, lo, j), span = __shfl_sync(0xffffffffu, hi, j) - v0;
                 const int cnt = max(1, (int)ceil(span / 0.5));
                 const double width = FAST ? span * rcp_pos((double)cnt) : span / cnt, half = 0.5 * width;
-                const double iL = FAST ? rcp_pos(segf(b, 4, sg)) : 1.0 / segf(b, 4, sg);
+                
                 const double p0r = segf(b, 0, sg), p0z = segf(b, 1, sg), ur = segf(b, 5, sg), uz = segf(b, 6, sg);
-                const double sg0 = segf(b, 9, sg), dsg = (segf(b, 10, sg) - sg0) * iL;
+                const double sg0 = segf(b, 9, sg), dsg = FAST ? (segf(b, 10, sg) - sg0) * rcp_pos(segf(b, 4, sg)) : 0.0;
                 for (int q0 = 0; q0 < cnt * 8; q0 += 32, ++S.round) {
                     const int qn = q0 + lane;
                     if ((FAST && !S.mine()) || qn >= cnt * 8) continue;
                     const int iv = qn >> 3, gi = qn & 7;
-                    // A node's place is rounded at ulp(rho), 1e-10 of its distance at a picometre, so the
-                    // reference rule takes sinh as accurate as the reference's; the adaptive rule takes sinh and
-                    // cosh from one exponential (sinh to 1e-16 of d, and the node is at least d from the point).
                     const double v = fma(iv + 0.5 * (b.gauss8_x[gi] + 1.0), width, v0);
-                    double sh, ch;
-                    if constexpr (FAST) {
-                        const double ev = exp(v), em = rcp_pos(ev);
-                        sh = 0.5 * (ev - em);
-                        ch = 0.5 * (ev + em);
-                    } else {
-                        sh = sinh(v);
-                        ch = sqrt_pos(fma(sh, sh, 1.0));
-                    }
-                    const double sl = fma(d, sh, sp);
-                    const double sr = fma(sl, ur, p0r), sz = fma(sl, uz, p0z);
-                    const double w = fma(sl, dsg, sg0) * (2.0 * kPi * sr) * d * ch * half * b.gauss8_w[gi];
                     double er, ez;
-                    ring_field_far<true, FAST>(re, inv, ze - sz, sr, er, ez);
                     if constexpr (FAST) {
+                        // sinh and cosh from one exponential (sinh to 1e-16 of d, and the node is at least d from
+                        // the point)
+                        const double ev = exp(v), em = rcp_pos(ev);
+                        const double sl = fma(0.5 * d, ev - em, sp);
+                        const double sr = fma(sl, ur, p0r), sz = fma(sl, uz, p0z);
+                        const double w = fma(sl, dsg, sg0) * (2.0 * kPi * sr) * (0.5 * d * (ev + em)) * half * b.gauss8_w[gi];
+                        ring_field_far<true, true>(re, inv, ze - sz, sr, er, ez);
                         S.add(w * er, w * ez);
                     } else {
-                        S.r[0] = fma(w, er, S.r[0]);
-                        S.z[0] = fma(w, ez, S.z[0]);
+                        // the reference's own operations: a node's place is rounded at ulp(rho), 1e-10 of its
+                        // distance at a picometre, and a^2 - rho^2 + z^2 cancels (1e-12 of the field at 0.1 nm
+                        // from a 2 um wall), so traces of ill-conditioned particles follow this rounding
+                        const double sl = sp + d * sinh(v);
+                        const double sr = p0r + sl * ur, sz = p0z + sl * uz;
+                        const double dens = sg0 + (sl / segf(b, 4, sg)) * (segf(b, 10, sg) - sg0);
+                        const double w = dens * (2.0 * kPi * sr) * d * cosh(v) * half * b.gauss8_w[gi];
+                        ring_field(re, ze - sz, sr, er, ez);
+                        S.r[0] += w * er;
+                        S.z[0] += w * ez;
                     }
                 }
                 if (lane == 0 && S.share == 0) { n.n_near += 1; n.n_ring_near += (unsigned long long)cnt * 8; }
@@ -1818,52 +1825,113 @@ __device__ void bem_points(Ctx& c, int n, bool scatter, int* status_flag) {
     bem_rotate(c, n, scatter);
 }
 
-// Softened pair sum over the live sources of the group (forces.py:16-29):
-// sum_j k q_i q_j (r_i - r_j) / (|r_i - r_j|^2 + a^2)^1.5, sources given by
-// src(j, x, y, z, q).  float64: the reference's operation order.  Mixed
-// form: separations are taken in float64 (nearby particles far from the
-// origin), then the rest in float32 with Kahan-compensated sums.
-template <bool MIX, typename SRC>
-__device__ __forceinline__ void pair_sum(const Ctx& c, int E, int j0, int jstep, double xi, double yi, double zi,
-                                         double qk, SRC src, double& fx, double& fy, double& fz,
-                                         double* sabs = nullptr) {
-    // sources j0, j0 + jstep, ... (the callers split one target's sources over
-    // the lanes of a warp and add the partial sums)
-    if (!MIX) {
-        double ax = 0.0, ay = 0.0, az = 0.0;
-        for (int j = j0; j < E; j += jstep) {
-            if (!c.live[j]) continue;
-            double x, y, z, q;
-            src(j, x, y, z, q);
-            const double dx = xi - x, dy = yi - y, dz = zi - z;
-            const double r2 = (dx * dx + dy * dy) + dz * dz + c.soft2;
-            const double r3 = r2 * sqrt(r2);
-            const double cf = qk * q / r3;
-            ax = fma(cf, dx, ax);
-            ay = fma(cf, dy, ay);
-            az = fma(cf, dz, az);
+// Softened pair sum over the live sources of the group (forces.py:16-29), mixed
+// form: sum_j k q_i q_j (r_i - r_j) / (|r_i - r_j|^2 + a^2)^1.5, sources given
+// by src(j, x, y, z, q).  Separations are taken in float64 (nearby particles
+// far from the origin), then the rest in float32 with Kahan-compensated sums.
+template <typename SRC>
+__device__ __forceinline__ void pair_sum(const Ctx& c, int nl, int j0, int jstep, double xi, double yi, double zi,
+                                         double qk, SRC src, double& fx, double& fy, double& fz, double& sabs) {
+    // live sources j0, j0 + jstep, ... (the callers split one target's sources
+    // over the lanes of a warp and add the partial sums)
+    float ax = 0.f, ay = 0.f, az = 0.f, cx = 0.f, cy = 0.f, cz = 0.f, sa = 0.f;
+    const float soft2 = (float)c.soft2;
+    for (int jj = j0; jj < nl; jj += jstep) {
+        double x, y, z, q;
+        src(c.lidx[jj], x, y, z, q);
+        const float dx = (float)(xi - x), dy = (float)(yi - y), dz = (float)(zi - z);
+        const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, soft2)));
+        const float rs = rsqrtf(r2);
+        const float cf = (float)(qk * q) * (rs * rs * rs);
+        kahan_add(ax, cx, cf * dx);
+        kahan_add(ay, cy, cf * dy);
+        kahan_add(az, cz, cf * dz);
+        sa += fabsf(cf * dx) + fabsf(cf * dy) + fabsf(cf * dz);
+    }
+    sabs += sa;
+    fx = (double)ax - (double)cx;
+    fy = (double)ay - (double)cy;
+    fz = (double)az - (double)cz;
+}
+
+// The indices of the live particles, in order, and their number, into c.lidx
+// and c.nl: by the first warp; a barrier follows before they are read.
+__device__ __forceinline__ void list_live(Ctx& c) {
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x;
+    int n = 0;
+    for (int base = 0; base < c.E; base += 32) {
+        const bool on = base + lane < c.E && c.live[base + lane];
+        const unsigned m = __ballot_sync(0xffffffffu, on);
+        if (on) c.lidx[n + __popc(m & ((1u << lane) - 1u))] = base + lane;
+        n += __popc(m);
+    }
+    if (lane == 0) {
+        c.nl[0] = n;
+        if (n == 0) c.lidx[0] = 0;
+    }
+}
+
+// 1 / sqrt(x)^3 times q, for positive normal x: the hardware's 20-bit estimate
+// and one third-order Newton step (the next term is 5 e^3 / 16 < 1e-17).
+__device__ __forceinline__ double pair_coef(double x, double q) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-(x * y), y, 1.0);
+    y = fma(y * e, fma(0.375, e, 0.5), y);
+    return (q * y) * (y * y);
+}
+
+// Float64 pair sums of one target (forces.py:16-191): the softened Coulomb
+// force of the live sources and of their images, in one loop over the live
+// list (the sources share dx, dy and their loads, and nothing in the loop
+// branches, so that iterations overlap; the sums apart took a square root and
+// a division with their special cases for each of up to four sets, one
+// iteration after the other).  SETS: 1 Coulomb only; 2 and the plane image
+// (z -> plane - z, -q); 4 and, in the apex frame, the sphere image and its
+// plane image (forces.py:101-191), from img.  `zc` is subtracted from z for
+// the images, `plane` the mirror sum of z + z'.
+struct PairForces {
+    double cx = 0.0, cy = 0.0, cz = 0.0;      // Coulomb
+    double ax = 0.0, ay = 0.0, az = 0.0;      // sphere images
+    double bx = 0.0, by = 0.0, bz = 0.0;      // plane images
+    double dx = 0.0, dy = 0.0, dz = 0.0;      // plane images of the sphere images
+};
+template <int SETS, typename SRC, typename IMG>
+__device__ __forceinline__ void pair_forces(int n, int j0, int jstep, double xi, double yi, double zi, double qk,
+                                            double soft2, double zc, double plane, SRC src, IMG img, PairForces& f) {
+    const double zl = zi - zc;
+#pragma unroll 2
+    for (int jj = j0; jj < n; jj += jstep) {
+        double x, y, z, q;
+        const int j = src(jj, x, y, z, q);
+        const double dx = xi - x, dy = yi - y, dz = zi - z, qq = qk * q;
+        const double r = fma(dx, dx, dy * dy);
+        const double c = pair_coef(fma(dz, dz, r) + soft2, qq);
+        f.cx = fma(c, dx, f.cx);
+        f.cy = fma(c, dy, f.cy);
+        f.cz = fma(c, dz, f.cz);
+        if constexpr (SETS >= 2) {
+            const double ez = zl - (plane - (z - zc));
+            const double b = pair_coef(fma(ez, ez, r) + soft2, -qq);
+            f.bx = fma(b, dx, f.bx);
+            f.by = fma(b, dy, f.by);
+            f.bz = fma(b, ez, f.bz);
         }
-        fx = ax; fy = ay; fz = az;
-    } else {
-        float ax = 0.f, ay = 0.f, az = 0.f, cx = 0.f, cy = 0.f, cz = 0.f, sa = 0.f;
-        const float soft2 = (float)c.soft2;
-        for (int j = j0; j < E; j += jstep) {
-            if (!c.live[j]) continue;
-            double x, y, z, q;
-            src(j, x, y, z, q);
-            const float dx = (float)(xi - x), dy = (float)(yi - y), dz = (float)(zi - z);
-            const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, soft2)));
-            const float rs = rsqrtf(r2);
-            const float cf = (float)(qk * q) * (rs * rs * rs);
-            kahan_add(ax, cx, cf * dx);
-            kahan_add(ay, cy, cf * dy);
-            kahan_add(az, cz, cf * dz);
-            sa += fabsf(cf * dx) + fabsf(cf * dy) + fabsf(cf * dz);
+        if constexpr (SETS >= 4) {
+            double ix, iy, iz, iq;
+            img(j, ix, iy, iz, iq);
+            const double ux = xi - ix, uy = yi - iy, uz = zl - iz, vz = zl - (plane - iz), uq = qk * iq;
+            const double ur = fma(ux, ux, uy * uy);
+            const double a = pair_coef(fma(uz, uz, ur) + soft2, uq);
+            f.ax = fma(a, ux, f.ax);
+            f.ay = fma(a, uy, f.ay);
+            f.az = fma(a, uz, f.az);
+            const double d = pair_coef(fma(vz, vz, ur) + soft2, -uq);
+            f.dx = fma(d, ux, f.dx);
+            f.dy = fma(d, uy, f.dy);
+            f.dz = fma(d, vz, f.dz);
         }
-        if (sabs) *sabs += sa;
-        fx = (double)ax - (double)cx;
-        fy = (double)ay - (double)cy;
-        fz = (double)az - (double)cz;
     }
 }
 
@@ -2015,86 +2083,101 @@ __device__ void stage_accel(Ctx& c, double* out, int* status_flag) {
         __syncthreads();
     }
 
-    // 3. per particle: field + pair sums.  Each target's sources are split
-    // over T lanes of a warp (T = 256 / E rounded down to a power of two, at
-    // most 32), whose partial sums are added with shuffles.  Mixed form: the
-    // sums run in float32 first; a target whose sum of |float32 terms| / m
-    // exceeds kappa times its whole acceleration is summed again in float64.
+    // 3. per live particle: field + pair sums over the live sources.  Each
+    // target's sources are split over T lanes of a warp (as many as the CTA has
+    // threads per live particle, a power of two, at most 32), whose partial sums
+    // are added with shuffles.  Mixed form: the sums run in float32 first; a
+    // target whose sum of |float32 terms| / m exceeds kappa times its whole
+    // acceleration is summed again in float64.
+    const int nl = c.nl[0];
+    for (int i = tid; i < E; i += c.nt)
+        if (!c.live[i]) out[i] = out[E + i] = out[2 * E + i] = 0.0;
     int T = 1;
-    while (T < 32 && T * 2 * E <= c.nt) T *= 2;
+    while (T < 32 && T * 2 * nl <= c.nt) T *= 2;
     const int per_pass = c.nt / T;
     const int sub = tid & (T - 1);
     const int lead = (tid & 31) & ~(T - 1);  // lane of the target's first sub-lane
     unsigned long long pairs = 0, redone = 0;
-    for (int base = 0; base < E; base += per_pass) {
-        const int i = base + tid / T;
-        const bool act = i < E && c.live[i];
+    const bool flat_img = KIND == SPT_GEOM_FLAT && g.has_image;
+    const double zc = (KIND == SPT_GEOM_POST_BEM) ? g.L : 0.0;
+    const double plane = flat_img ? -2.0 * g.z0 : -2.0 * (zc + g.z0);
+    for (int base = 0; base < nl; base += per_pass) {
+        const int at = base + tid / T;
+        const bool act = at < nl;
         constexpr bool mix = FORM != SPT_FORM_FP64;
-        const int ii = i < E ? i : 0;
-        const double xi = sx[ii], yi = sy[ii], zi = sz[ii];
-        const double qk = c.kc * c.q[ii];
-        // this lane's share of the target's Coulomb (fc) and image (fi) sums
-        auto pass = [&](auto f32_tag, bool on, double& fcx, double& fcy, double& fcz, double& fix, double& fiy,
-                        double& fiz, double& sabs) {
-            constexpr bool f32 = decltype(f32_tag)::value;
+        const int i = c.lidx[act ? at : 0];
+        const double xi = sx[i], yi = sy[i], zi = sz[i];
+        const double qk = c.kc * c.q[i];
+        double fcx, fcy, fcz, fix, fiy, fiz;
+        auto reduce = [&]() {
+            fcx = group_sum(fcx, T); fcy = group_sum(fcy, T); fcz = group_sum(fcz, T);
+            fix = group_sum(fix, T); fiy = group_sum(fiy, T); fiz = group_sum(fiz, T);
+        };
+        // this lane's share of the target's Coulomb (fc) and image (fi) sums (lanes without work add zeros)
+        auto pass64 = [&](bool on) {
+            PairForces f;
+            auto real = [&](int jj, double& x, double& y, double& z, double& q) {
+                const int j = c.lidx[jj];
+                x = sx[j]; y = sy[j]; z = sz[j]; q = c.q[j];
+                return j;
+            };
+            auto sphere = [&](int j, double& x, double& y, double& z, double& q) {
+                x = c.img[j]; y = c.img[E + j]; z = c.img[2 * E + j]; q = c.img[3 * E + j];
+            };
+            const int n = on ? nl : 0;
+            if constexpr (KIND == SPT_GEOM_TIP || KIND == SPT_GEOM_POST_BEM) {
+                if (three_img) pair_forces<4>(n, sub, T, xi, yi, zi, qk, c.soft2, zc, plane, real, sphere, f);
+                else pair_forces<1>(n, sub, T, xi, yi, zi, qk, c.soft2, zc, plane, real, sphere, f);
+            } else if constexpr (KIND == SPT_GEOM_FLAT) {
+                if (flat_img) pair_forces<2>(n, sub, T, xi, yi, zi, qk, c.soft2, 0.0, plane, real, sphere, f);
+                else pair_forces<1>(n, sub, T, xi, yi, zi, qk, c.soft2, 0.0, plane, real, sphere, f);
+            } else {
+                pair_forces<1>(n, sub, T, xi, yi, zi, qk, c.soft2, 0.0, plane, real, sphere, f);
+            }
+            // a lone particle has no Coulomb force, whatever the softening makes of its own term
+            fcx = E > 1 ? f.cx : 0.0; fcy = E > 1 ? f.cy : 0.0; fcz = E > 1 ? f.cz : 0.0;
+            fix = (f.ax + f.bx) + f.dx; fiy = (f.ay + f.by) + f.dy; fiz = (f.az + f.bz) + f.dz;
+        };
+        double sabs = 0.0;
+        auto pass32 = [&](bool on) {
             fcx = fcy = fcz = fix = fiy = fiz = sabs = 0.0;
             if (!on) return;
-            double* sa = f32 ? &sabs : nullptr;
-            if (E > 1) {
-                auto real = [&](int j, double& x, double& y, double& z, double& q) {
-                    x = sx[j]; y = sy[j]; z = sz[j]; q = c.q[j];
-                };
-                if constexpr (f32) pair_sum<true>(c, E, sub, T, xi, yi, zi, qk, real, fcx, fcy, fcz, sa);
-                else pair_sum<false>(c, E, sub, T, xi, yi, zi, qk, real, fcx, fcy, fcz);
-            }
-            if (KIND == SPT_GEOM_FLAT && g.has_image) {
-                const double zimg = -2.0 * g.z0;
+            auto real = [&](int j, double& x, double& y, double& z, double& q) {
+                x = sx[j]; y = sy[j]; z = sz[j]; q = c.q[j];
+            };
+            if (E > 1) pair_sum(c, nl, sub, T, xi, yi, zi, qk, real, fcx, fcy, fcz, sabs);
+            if (flat_img) {
                 auto mirror = [&](int j, double& x, double& y, double& z, double& q) {
-                    x = sx[j]; y = sy[j]; z = zimg - sz[j]; q = -c.q[j];
+                    x = sx[j]; y = sy[j]; z = plane - sz[j]; q = -c.q[j];
                 };
-                if constexpr (f32) pair_sum<true>(c, E, sub, T, xi, yi, zi, qk, mirror, fix, fiy, fiz, sa);
-                else pair_sum<false>(c, E, sub, T, xi, yi, zi, qk, mirror, fix, fiy, fiz);
+                pair_sum(c, nl, sub, T, xi, yi, zi, qk, mirror, fix, fiy, fiz, sabs);
             } else if (three_img) {
-                const double zc = (KIND == SPT_GEOM_POST_BEM) ? g.L : 0.0;
-                const double pz0 = (KIND == SPT_GEOM_POST_BEM) ? g.L + g.z0 : g.z0;
                 const double zl = zi - zc;
                 double s1x, s1y, s1z, s2x, s2y, s2z, s3x, s3y, s3z;
                 auto sphere = [&](int j, double& x, double& y, double& z, double& q) {
                     x = c.img[j]; y = c.img[E + j]; z = c.img[2 * E + j]; q = c.img[3 * E + j];
                 };
-                auto plane = [&](int j, double& x, double& y, double& z, double& q) {
-                    x = sx[j]; y = sy[j]; z = -2.0 * pz0 - (sz[j] - zc); q = -c.q[j];
+                auto mirror = [&](int j, double& x, double& y, double& z, double& q) {
+                    x = sx[j]; y = sy[j]; z = plane - (sz[j] - zc); q = -c.q[j];
                 };
-                auto plane_sphere = [&](int j, double& x, double& y, double& z, double& q) {
-                    x = c.img[j]; y = c.img[E + j]; z = -2.0 * pz0 - c.img[2 * E + j]; q = -c.img[3 * E + j];
+                auto mirror_sphere = [&](int j, double& x, double& y, double& z, double& q) {
+                    x = c.img[j]; y = c.img[E + j]; z = plane - c.img[2 * E + j]; q = -c.img[3 * E + j];
                 };
-                if constexpr (f32) {
-                    pair_sum<true>(c, E, sub, T, xi, yi, zl, qk, sphere, s1x, s1y, s1z, sa);
-                    pair_sum<true>(c, E, sub, T, xi, yi, zl, qk, plane, s2x, s2y, s2z, sa);
-                    pair_sum<true>(c, E, sub, T, xi, yi, zl, qk, plane_sphere, s3x, s3y, s3z, sa);
-                } else {
-                    pair_sum<false>(c, E, sub, T, xi, yi, zl, qk, sphere, s1x, s1y, s1z);
-                    pair_sum<false>(c, E, sub, T, xi, yi, zl, qk, plane, s2x, s2y, s2z);
-                    pair_sum<false>(c, E, sub, T, xi, yi, zl, qk, plane_sphere, s3x, s3y, s3z);
-                }
+                pair_sum(c, nl, sub, T, xi, yi, zl, qk, sphere, s1x, s1y, s1z, sabs);
+                pair_sum(c, nl, sub, T, xi, yi, zl, qk, mirror, s2x, s2y, s2z, sabs);
+                pair_sum(c, nl, sub, T, xi, yi, zl, qk, mirror_sphere, s3x, s3y, s3z, sabs);
                 fix = (s1x + s2x) + s3x;
                 fiy = (s1y + s2y) + s3y;
                 fiz = (s1z + s2z) + s3z;
             }
-            // every lane takes part in the shuffles (lanes without work add zeros)
-        };
-        auto reduce = [&](double& fcx, double& fcy, double& fcz, double& fix, double& fiy, double& fiz,
-                          double& sabs) {
-            fcx = group_sum(fcx, T); fcy = group_sum(fcy, T); fcz = group_sum(fcz, T);
-            fix = group_sum(fix, T); fiy = group_sum(fiy, T); fiz = group_sum(fiz, T);
-            sabs = group_sum(sabs, T);
         };
         if (act && sub == 0) {
-            pairs += (E > 1 ? E : 0) + ((KIND == SPT_GEOM_FLAT && g.has_image) ? E : 0) + (three_img ? 3 * E : 0);
+            pairs += (E > 1 ? E : 0) + (flat_img ? E : 0) + (three_img ? 3 * E : 0);
         }
-        double fcx, fcy, fcz, fix, fiy, fiz, sabs;
-        pass(std::integral_constant<bool, mix>{}, act, fcx, fcy, fcz, fix, fiy, fiz, sabs);
-        reduce(fcx, fcy, fcz, fix, fiy, fiz, sabs);
+        if constexpr (mix) pass32(act);
+        else pass64(act);
+        reduce();
+        sabs = group_sum(sabs, T);
         auto bem_image = [&]() {  // the BEM image force of 1b takes the place of a pair-sum image
             if (bem_img && act && sub == 0) {
                 fix = c.img[i];
@@ -2139,17 +2222,19 @@ __device__ void stage_accel(Ctx& c, double* out, int* status_flag) {
             accel_of(ax, ay, az);
             redo = mix && !(sabs / mi <= c.kappa * sqrt(ax * ax + ay * ay + az * az));
         }
-        redo = __shfl_sync(0xffffffffu, redo, lead);
-        if (mix && __any_sync(0xffffffffu, redo)) {
-            pass(std::integral_constant<bool, false>{}, act && redo, fcx, fcy, fcz, fix, fiy, fiz, sabs);
-            reduce(fcx, fcy, fcz, fix, fiy, fiz, sabs);
-            bem_image();
-            if (act && redo && sub == 0) {
-                accel_of(ax, ay, az);
-                ++redone;
+        if constexpr (mix) {
+            redo = __shfl_sync(0xffffffffu, redo, lead);
+            if (__any_sync(0xffffffffu, redo)) {
+                pass64(act && redo);
+                reduce();
+                bem_image();
+                if (act && redo && sub == 0) {
+                    accel_of(ax, ay, az);
+                    ++redone;
+                }
             }
         }
-        if (i < E && sub == 0) {
+        if (act && sub == 0) {
             out[i] = ax;
             out[E + i] = ay;
             out[2 * E + i] = az;
@@ -2436,6 +2521,7 @@ trace_kernel(const __grid_constant__ SptState st, const __grid_constant__ SptTra
             const double t = gs.t, hr = gs.hr;
             for (int i = tid; i < E; i += nt) c.live[i] = (t >= c.tb[i]) && (t < c.td[i]);
             __syncthreads();
+            list_live(c);  // (the stages' first barrier orders it)
             // seven stage evaluations through one call site of stage_accel (a second
             // inlined copy of the stage code would double the kernel's instruction footprint)
             for (int s = 0; s < 7; ++s) {
@@ -2613,7 +2699,7 @@ accel_kernel(const __grid_constant__ SptAccelArgs a, const __grid_constant__ Spt
     c.kc = a.coulomb_constant;
     c.soft2 = a.plummer_radius * a.plummer_radius;
     const int Emax = a.max_group_size;
-    bind(c, smem, Emax, FAR, nullptr, s_cnt, false, !GIVEN);
+    bind(c, smem, Emax, FAR, nullptr, s_cnt, false, !GIVEN, false);
     init_barriers(c);
     const long long base = a.group_offset[g];
     const int E = (int)(a.group_offset[g + 1] - base);
@@ -2633,7 +2719,9 @@ accel_kernel(const __grid_constant__ SptAccelArgs a, const __grid_constant__ Spt
         }
     }
     __syncthreads();
-    double* out = c.kv;  // slope storage is free on this path (groups here are at most kSmallGroup)
+    list_live(c);
+    __syncthreads();
+    double* out = c.kv;
     stage_accel<KIND, FORM, FAR, GIVEN>(c, out, &s_flag);
     for (int i = tid; i < E; i += c.nt) {
         a.ax[base + i] = out[i];
@@ -2669,7 +2757,7 @@ accel_kernel(const __grid_constant__ SptAccelArgs a, const __grid_constant__ Spt
 constexpr int kWarpSlotComps = 54;  // y0 6, 5th-order solution 6, stage velocities 21, stage accelerations 21
 constexpr int kWarpSlotDoubles = kWarpSlotComps * 32;
 // per-warp shared doubles: BEM record 8, stage positions and charges 4 x 32,
-// sphere images 4 x 32, BEM fields 3 x 32, live flags 32 ints
+// sphere images 4 x 32, BEM fields 3 x 32, live list 32 ints
 constexpr int kWarpTeamDoubles = 8 + 4 * 32 + 4 * 32 + 3 * 32 + 16;
 
 __host__ __device__ inline size_t warp_team_smem(int warps) {
@@ -2685,7 +2773,7 @@ __device__ __forceinline__ double warp_min_all(double v) {
 // per-warp shared region of warp w
 struct WarpTeam {
     double *rec, *sx, *sy, *sz, *q, *img, *fld;
-    int* live;
+    int* lidx;
     __device__ WarpTeam(double* smem, int nw, int w) {
         double* t = smem + (size_t)nw * kWarpScratchInts / 2 + (size_t)w * kWarpTeamDoubles;
         rec = t;
@@ -2695,7 +2783,7 @@ struct WarpTeam {
         q = sz + 32;
         img = q + 32;
         fld = img + 128;
-        live = reinterpret_cast<int*>(fld + 96);
+        lidx = reinterpret_cast<int*>(fld + 96);
     }
 };
 
@@ -2778,41 +2866,48 @@ __device__ __forceinline__ void stage_finish_warp(Ctx& c, const WarpTeam& w, boo
         }
         __syncwarp();
     }
-    // pair sums, one target per lane, sources in order (forces.py:16-57,
-    // 101-191), and the blended external field
+    // Pair sums (forces.py:16-57, 101-191): T lanes a target while the live
+    // particles leave lanes free (targets and sources by the live list), the
+    // partial sums added with shuffles and handed to the target's lane.
+    const unsigned lm = __ballot_sync(0xffffffffu, live);
+    const int nl = __popc(lm);
+    double fcx = 0.0, fcy = 0.0, fcz = 0.0, fix = 0.0, fiy = 0.0, fiz = 0.0;
+    if (nl > 0 && (E > 1 || three_img)) {
+        int T = 1;
+        while (T * 2 * nl <= 32 && T * 2 <= nl) T *= 2;
+        const int at = lane / T, sub = lane & (T - 1);
+        const bool on = at < nl;
+        const int i = w.lidx[on ? at : 0];
+        PairForces f;
+        auto real = [&](int jj, double& x, double& y, double& z, double& q) {
+            const int j = w.lidx[jj];
+            x = w.sx[j]; y = w.sy[j]; z = w.sz[j]; q = w.q[j];
+            return j;
+        };
+        auto sphere = [&](int j, double& x, double& y, double& z, double& q) {
+            x = w.img[j]; y = w.img[32 + j]; z = w.img[64 + j]; q = w.img[96 + j];
+        };
+        const double qk = c.kc * w.q[i];
+        const double plane = -2.0 * (zc + g.z0);
+        if (three_img)
+            pair_forces<4>(on ? nl : 0, sub, T, w.sx[i], w.sy[i], w.sz[i], qk, c.soft2, zc, plane, real, sphere, f);
+        else
+            pair_forces<1>(on ? nl : 0, sub, T, w.sx[i], w.sy[i], w.sz[i], qk, c.soft2, zc, plane, real, sphere, f);
+        const int from = __popc(lm & ((1u << lane) - 1u)) * T;  // the lane that holds this lane's target
+        auto hand = [&](double v) { return __shfl_sync(0xffffffffu, group_sum(v, T), from & 31); };
+        fcx = hand(E > 1 ? f.cx : 0.0);  // (a lone particle has no Coulomb force)
+        fcy = hand(E > 1 ? f.cy : 0.0);
+        fcz = hand(E > 1 ? f.cz : 0.0);
+        if (three_img) {
+            fix = hand((f.ax + f.bx) + f.dx);
+            fiy = hand((f.ay + f.by) + f.dy);
+            fiz = hand((f.az + f.bz) + f.dz);
+        }
+    }
     ax = ay = az = 0.0;
     unsigned long long pairs = 0;
     if (live) {
-        const double qk = c.kc * w.q[lane];
-        double fcx = 0.0, fcy = 0.0, fcz = 0.0, fix = 0.0, fiy = 0.0, fiz = 0.0;
-        if (E > 1) {
-            auto real = [&](int j, double& x, double& y, double& z, double& q) {
-                x = w.sx[j]; y = w.sy[j]; z = w.sz[j]; q = w.q[j];
-            };
-            pair_sum<false>(c, E, 0, 1, xi, yi, zi, qk, real, fcx, fcy, fcz);
-            pairs += E;
-        }
-        if (three_img) {
-            const double pz0 = g.L + g.z0;
-            const double zl = zi - zc;
-            double s1x, s1y, s1z, s2x, s2y, s2z, s3x, s3y, s3z;
-            auto sphere = [&](int j, double& x, double& y, double& z, double& q) {
-                x = w.img[j]; y = w.img[32 + j]; z = w.img[64 + j]; q = w.img[96 + j];
-            };
-            auto plane = [&](int j, double& x, double& y, double& z, double& q) {
-                x = w.sx[j]; y = w.sy[j]; z = -2.0 * pz0 - (w.sz[j] - zc); q = -w.q[j];
-            };
-            auto plane_sphere = [&](int j, double& x, double& y, double& z, double& q) {
-                x = w.img[j]; y = w.img[32 + j]; z = -2.0 * pz0 - w.img[64 + j]; q = -w.img[96 + j];
-            };
-            pair_sum<false>(c, E, 0, 1, xi, yi, zl, qk, sphere, s1x, s1y, s1z);
-            pair_sum<false>(c, E, 0, 1, xi, yi, zl, qk, plane, s2x, s2y, s2z);
-            pair_sum<false>(c, E, 0, 1, xi, yi, zl, qk, plane_sphere, s3x, s3y, s3z);
-            fix = (s1x + s2x) + s3x;
-            fiy = (s1y + s2y) + s3y;
-            fiz = (s1z + s2z) + s3z;
-            pairs += 3 * E;
-        }
+        pairs = (E > 1 ? E : 0) + (three_img ? 3 * E : 0);
         // blend(near, far) with near = where(valid, uniform + pert, 0) (bem/geometry.py:44-55, bem/fields.py:186-211)
         const double wgt = blend_weight(zi, g.z_handoff);
         const bool valid = bem_valid<KIND>(xi, yi, zi, g);
@@ -2866,7 +2961,6 @@ trace_warp_kernel(const __grid_constant__ SptState st, const __grid_constant__ S
     double* const part = smem + (warp_team_smem(nw) / 8 - kSplitDoubles);
     const double* const map = field_map(bem);
     PointCounts pts;
-    c.live = w.live;
     double* const slot = slots + ((size_t)blockIdx.x * nw + warp) * kWarpSlotDoubles + lane;
     auto ld = [&](int k) { return __ldcg(slot + 32 * k); };
     auto sto = [&](int k, double v) { __stcg(slot + 32 * k, v); };
@@ -3023,7 +3117,10 @@ trace_warp_kernel(const __grid_constant__ SptState st, const __grid_constant__ S
                 w.sx[lane] = px;
                 w.sy[lane] = py;
                 w.sz[lane] = pz;
-                w.live[lane] = live;
+                if (s == 0) {  // the live list of this attempt
+                    const unsigned lm = __ballot_sync(0xffffffffu, live);
+                    if (live) w.lidx[__popc(lm & ((1u << lane) - 1u))] = lane;
+                }
                 // the BEM field of the live particles inside the valid region
                 // with blend weight > 0: mapped points here, by their own
                 // warp, the others to the CTA's pool
@@ -3242,7 +3339,7 @@ int trace_launch(const TraceLaunch& t, int grid, size_t smem) {
 template <int KIND, int FORM, int FAR, bool GIVEN = false>
 int accel_launch(const SptAccelArgs* a, const SptGeometry* g, const SptBem& bem, cudaStream_t stream) {
     const Layout L = make_layout(a->max_group_size, FAR, false, !GIVEN, kMaxWarps,
-                                 image_scratch(*g, bem, a->max_group_size, kMaxThreads));
+                                 image_scratch(*g, bem, a->max_group_size, kMaxThreads), false);
     auto kern = accel_kernel<KIND, FORM, FAR, GIVEN>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.bytes);
     if (e != cudaSuccess) return (int)e;

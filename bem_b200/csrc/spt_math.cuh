@@ -72,6 +72,13 @@ __device__ __forceinline__ void ellip_ke(double p, double& K, double& E) {
     E = K * (1.0 - S);
 }
 
+// a^2 - rho^2 + z^2 in the reference's rounding, no contraction: it cancels near
+// the ring, and a sum that forms it otherwise (more closely, even) is off the
+// reference's by up to 5e-14 of a term.
+__device__ __forceinline__ double ring_a(double rho, double z, double a) {
+    return __dadd_rn(__dadd_rn(__dmul_rn(a, a), -__dmul_rn(rho, rho)), __dmul_rn(z, z));
+}
+
 // Field (E_rho, E_z) at (rho, z) of a unit-total-charge ring of radius a at
 // height 0 (G = 1/(4 pi r) convention), float64.  The formula and the
 // near-axis Taylor branch follow bem/axisymmetric.py:248-265.
@@ -90,7 +97,7 @@ __device__ __forceinline__ void ring_field(double rho, double z, double a, doubl
     double K, E;
     ellip_ke(d2 / D, K, E);
     const double sD = sqrt(D);
-    er = (K - (a2 - rho2 + z2) * E / d2) / (4.0 * kPi * kPi * rho * sD);
+    er = (K - ring_a(rho, z, a) * E / d2) / (4.0 * kPi * kPi * rho * sD);
     ez = z * E / (2.0 * kPi * kPi * sD * d2);
 }
 
@@ -128,23 +135,10 @@ static __device__ __noinline__ void ring_axis_taylor(double rho, double z, doubl
     ez = z / (4.0 * kPi * ax15) + 3.0 * rho2 * z * (3.0 * a2 - 2.0 * z2) / (16.0 * kPi * ax35);
 }
 
-// Ring field close to the ring (p = d2 / D < 1e-3), the operations of
-// ring_field with its series branch: near a surface a^2 - rho^2 + z^2 cancels
-// to ~(rho - a) rho, and its rounding (1e-13 of the field at 10 pm) is part of
-// what the reference rule's traces of ill-conditioned particles reproduce.
-__device__ __forceinline__ void ring_close(double rho, double z, double a, double D, double d2, double& er,
-                                           double& ez) {
-    const double z2 = z * z, a2 = a * a, rho2 = rho * rho;
-    const double p = d2 / D, L = -0.5 * log(p);
-    const double K = fma(L, horner10(kSerK, p), horner10(kSerKd, p));
-    const double E = fma(0.5 * p, fma(L, horner10(kSerE, p), horner10(kSerEd, p)), 1.0);
-    const double sD = sqrt(D);
-    er = (K - (a2 - rho2 + z2) * E / d2) / (4.0 * kPi * kPi * rho * sD);
-    ez = z * E / (2.0 * kPi * kPi * sD * d2);
-}
-
-// The same for the adaptive rule: six terms (what is left out is below 1e-19)
-// and one reciprocal for every quotient.
+// Ring field close to the ring (p = d2 / D < 1e-3), the adaptive rule's: six
+// terms of the series (what is left out is below 1e-19), one reciprocal for
+// every quotient, and a^2 - rho^2 + z^2, which cancels, in the reference's
+// rounding.
 __device__ __forceinline__ void ring_close_fast(double rho, double inv_rho, double z, double a, double D, double d2,
                                                 double& er, double& ez) {
     const double inv = rcp_pos(D * d2), inv_d2 = D * inv, p = d2 * (d2 * inv);
@@ -158,16 +152,14 @@ __device__ __forceinline__ void ring_close_fast(double rho, double inv_rho, doub
     const double K = fma(L, h6(kSerK), h6(kSerKd));
     const double E = fma(0.5 * p, fma(L, h6(kSerE), h6(kSerEd)), 1.0) * inv_d2;
     const double g = sqrt_pos(d2 * inv) * (1.0 / (4.0 * kPi * kPi));  // 1 / (4 pi^2 sqrt(D))
-    const double A = __dadd_rn(__dadd_rn(__dmul_rn(a, a), -__dmul_rn(rho, rho)), __dmul_rn(z, z));
-    er = fma(-A, E, K) * (g * inv_rho);
+    er = fma(-ring_a(rho, z, a), E, K) * (g * inv_rho);
     ez = 2.0 * z * E * g;
 }
 
-// Both out of line for the far sums: rare there, and on another path than every
-// interleaved evaluation.
-static __device__ __noinline__ void ring_close_cold(double rho, double z, double a, double D, double d2, double& er,
-                                                    double& ez) {
-    ring_close(rho, z, a, D, d2, er, ez);
+// Close rings out of line for the far sums: rare there, and on another path
+// than every interleaved evaluation.
+static __device__ __noinline__ void ring_close_cold(double rho, double z, double a, double& er, double& ez) {
+    ring_field(rho, z, a, er, ez);
 }
 static __device__ __noinline__ void ring_close_fast_cold(double rho, double inv_rho, double z, double a, double D,
                                                          double d2, double& er, double& ez) {
@@ -188,8 +180,8 @@ static __device__ __noinline__ void ring_close_fast_cold(double rho, double inv_
 // either).  Five square roots and one reciprocal, against eight and two of the
 // AGM run to convergence on d2 / D: the far sums are bound by these
 // instructions (96 M rings of one 1500-point call: 11.4 -> 6.7 ms).
-// NEAR: a near panel's node (close rings are common, in line, and a^2 - rho^2
-// as the reference forms it); FAST: the adaptive rule's close rings.
+// FAST: the adaptive rule's close rings and a^2 - rho^2; NEAR: its near panels'
+// nodes (close rings are common, in line).
 template <bool NEAR, bool FAST>
 __device__ __forceinline__ void ring_field_far(double rho, double inv_rho, double z, double a, double& er,
                                                double& ez) {
@@ -200,10 +192,9 @@ __device__ __forceinline__ void ring_field_far(double rho, double inv_rho, doubl
         return;
     }
     if (d2 < 1e-3 * D) {
-        if constexpr (NEAR && FAST) ring_close_fast(rho, inv_rho, z, a, D, d2, er, ez);
-        else if constexpr (NEAR) ring_close(rho, z, a, D, d2, er, ez);
+        if constexpr (NEAR) ring_close_fast(rho, inv_rho, z, a, D, d2, er, ez);
         else if constexpr (FAST) ring_close_fast_cold(rho, inv_rho, z, a, D, d2, er, ez);
-        else ring_close_cold(rho, z, a, D, d2, er, ez);
+        else ring_close_cold(rho, z, a, er, ez);
         return;
     }
     const double r1 = sqrt_pos(D), r2 = sqrt_pos(d2);
@@ -220,7 +211,7 @@ __device__ __forceinline__ void ring_field_far(double rho, double inv_rho, doubl
     S = fma(fma(0.25, e2, 2.0) * t4, t4, S);
     const double Q = (D - S) * (inv * m);
     const double F = im * fma(e2, fma(e2, 9.0 / 64.0, 0.25), 1.0);
-    const double A = NEAR ? a * a - rho * rho + z2 : fma(-s, t, z2);  // a^2 - rho^2 = -(rho + a)(rho - a)
+    const double A = FAST ? fma(-s, t, z2) : ring_a(rho, z, a);  // a^2 - rho^2 = -(rho + a)(rho - a)
     er = fma(-A, Q, 1.0) * (F * inv_rho * (1.0 / (8.0 * kPi)));
     ez = z * Q * (F * (1.0 / (4.0 * kPi)));
 }
