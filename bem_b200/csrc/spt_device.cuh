@@ -1962,7 +1962,7 @@ static __device__ __noinline__ void stage_image_force(Ctx& c) {
         z = sx[2 * E + i];
         q = c.live[i] ? c.q[i] : 0.0;
     };
-    spt_img::group_force<SPT_TRACE_IMAGE_MODES>(c.bem.image, ip, E, load, c.imgs, c.img, c.img + E, c.img + 2 * E,
+    spt_img::group_force<SPT_TRACE_IMAGE_MODES, false>(c.bem.image, ip, E, load, c.imgs, c.img, c.img + E, c.img + 2 * E,
                                                  &s_imgflag);
 }
 

@@ -141,8 +141,10 @@ struct ForceArgs {
     double* fz;
 };
 
+// Two CTAs an SM up to 16 modes (the reference's default): a CTA's phases are
+// chains of dependent work with barriers between, so a second one fills them.
 template <int MP>
-__global__ void __launch_bounds__(kThreads, 1) image_force_kernel(const __grid_constant__ ForceArgs a) {
+__global__ void __launch_bounds__(kThreads, MP <= 16 ? 2 : 1) image_force_kernel(const __grid_constant__ ForceArgs a) {
     extern __shared__ __align__(16) double smem[];
     __shared__ int s_flag;
     for (int g = blockIdx.x; g < a.n_groups; g += gridDim.x) {
@@ -154,7 +156,7 @@ __global__ void __launch_bounds__(kThreads, 1) image_force_kernel(const __grid_c
             z = a.z[off + i];
             q = a.active[off + i] ? a.charge[off + i] : 0.0;
         };
-        group_force<MP>(a.img, a.prm, E, load, smem, a.fx + off, a.fy + off, a.fz + off, &s_flag);
+        group_force<MP, true>(a.img, a.prm, E, load, smem, a.fx + off, a.fy + off, a.fz + off, &s_flag);
     }
 }
 
@@ -182,7 +184,12 @@ int launch_force(const spt_img::ForceArgs& a, size_t bytes, cudaStream_t st) {
     int rc = cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes),
                         "cudaFuncSetAttribute(image_force_kernel)");
     if (rc) return rc;
-    const int grid = a.n_groups < sm_count() ? a.n_groups : sm_count();
+    int per_sm = 1;
+    rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, spt_img::kThreads, bytes),
+                    "cudaOccupancyMaxActiveBlocksPerMultiprocessor(image_force_kernel)");
+    if (rc) return rc;
+    const int most = sm_count() * (per_sm < 1 ? 1 : per_sm);
+    const int grid = a.n_groups < most ? a.n_groups : most;
     k<<<grid, spt_img::kThreads, bytes, st>>>(a);
     return cuda_check(cudaGetLastError(), "image_force_kernel launch");
 }

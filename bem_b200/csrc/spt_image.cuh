@@ -79,6 +79,80 @@ __device__ __forceinline__ void toroidal(double chi, int M, double (&q)[MP + 1],
     }
 }
 
+// The same for the standalone force, whose time was the chain of divisions of
+// the downward ratios (M + 22 / eta of them, ~150 cycles each): K and E from
+// ellip_ke_fast, eta in float32 (it only chooses the recurrence and where it
+// starts), and Miller's algorithm on the values themselves, three dependent
+// operations a step,
+//   Q_{n-3/2} = (2 chi Q_{n-1/2} - Q_{n+1/2}) + (chi Q_{n-1/2} - Q_{n+1/2}) / (n - 1/2),
+// started from the same place and scaled by Q_{-1/2} at the end; the ratios
+// serve where the values would grow beyond e^600.
+template <int MP>
+__device__ __forceinline__ void toroidal_fast(double chi, int M, double (&q)[MP + 1], double& dq0) {
+    const double d = chi - 1.0, ip = spt::rcp_pos(chi + 1.0);
+    double K, E;
+    spt::ellip_ke_fast(d * ip, K, E);
+    const double root = spt::sqrt_pos(2.0 * ip);
+    const double q0 = root * K;
+    dq0 = -root * E * spt::rcp_pos(2.0 * d);
+    q[0] = q0;
+    const float df = (float)d;
+    const float eta = log1pf(df + sqrtf(df * (df + 2.0f)));
+    if ((float)M * eta <= 1.0f) {
+        double prev = q0, cur = chi * q0 - spt::sqrt_pos(2.0 * (chi + 1.0)) * E;
+        q[1] = cur;
+#pragma unroll
+        for (int n = 1; n < MP; ++n) {
+            if (n < M) {
+                const double nxt = (2.0 * n * chi * cur - (n - 0.5) * prev) * (1.0 / (n + 0.5));
+                q[n + 1] = nxt;
+                prev = cur;
+                cur = nxt;
+            }
+        }
+        return;
+    }
+    const int pad = max(kPadMin, (int)ceilf((float)kPadConst / eta));
+    if ((float)(M + pad) * eta < 600.0f) {
+        double y1 = 0.0, y = 1.0;  // Q_{n+1/2}, Q_{n-1/2} but for the scale
+        const double chi2 = 2.0 * chi;
+#pragma unroll 1
+        for (int n = M + pad; n > M; --n) {
+            const double inv = spt::rcp_pos(n - 0.5);
+            const double t = fma(inv, fma(chi, y, -y1), fma(chi2, y, -y1));
+            y1 = y;
+            y = t;
+        }
+#pragma unroll
+        for (int n = MP; n >= 1; --n) {
+            if (n <= M) {
+                q[n] = y;
+                const double t = fma(1.0 / (n - 0.5), fma(chi, y, -y1), fma(chi2, y, -y1));
+                y1 = y;
+                y = t;
+            }
+        }
+        const double scale = q0 * spt::rcp_pos(y);
+#pragma unroll
+        for (int n = 1; n <= MP; ++n)
+            if (n <= M) q[n] *= scale;
+        return;
+    }
+    double r = 0.0;
+#pragma unroll 1
+    for (int n = M + pad; n > M; --n) r = (n - 0.5) * spt::rcp_pos(2.0 * n * chi - (n + 0.5) * r);
+#pragma unroll
+    for (int n = MP; n >= 1; --n) {
+        if (n <= M) {
+            r = (n - 0.5) * spt::rcp_pos(2.0 * n * chi - (n + 0.5) * r);
+            q[n] = r;
+        }
+    }
+#pragma unroll
+    for (int n = 1; n <= MP; ++n)
+        if (n <= M) q[n] *= q[n - 1];
+}
+
 // dQ_{n-1/2}/dchi from the values (DLMF 14.10.5 at degree n - 1/2):
 // (n - 1/2)(chi Q_n - Q_{n-1}) / ((chi - 1)(chi + 1)), n >= 1.
 __device__ __forceinline__ double dq_of(int n, double chi, double qn, double qm1) {
@@ -206,7 +280,11 @@ __host__ __device__ inline long long scratch_doubles(int E, int phantoms, int P,
 //      geometry level: + the plane image for phantoms, blended with the
 //      plane image by height.
 // Phases B-D run only when some active particle needs the BEM force.
-template <int MP, class Load>
+// FAST: the standalone entry point's arithmetic and split -- toroidal_fast, four
+// rows of D at a time by eight lanes each, and in E as many warps a particle
+// as the CTA has (a batch of small groups left half of them idle).  The trace
+// keeps the operations its parity fixtures pin.
+template <int MP, bool FAST, class Load>
 __device__ void group_force(const SptImage& im, const ImgParams& a, int E, Load load, double* scratch, double* fx,
                             double* fy, double* fz, int* flag) {
     const int P = im.n_nodes, nm = im.n_max, M = max(nm, 1);
@@ -292,7 +370,8 @@ __device__ void group_force(const SptImage& im, const ImgParams& a, int E, Load 
                 if (qs == 0.0) continue;
                 const double rj = srho[j];
                 double dq0;
-                toroidal<MP>(chi_of(rp, zp, rj, sz[j]), M, q, dq0);
+                if constexpr (FAST) toroidal_fast<MP>(chi_of(rp, zp, rj, sz[j]), M, q, dq0);
+                else toroidal<MP>(chi_of(rp, zp, rj, sz[j]), M, q, dq0);
                 const double coef = qs / sqrt(rp * rj);
                 const double c1 = sc[j], s1 = ss[j];
                 double cm = 1.0, sm = 0.0;
@@ -321,6 +400,30 @@ __device__ void group_force(const SptImage& im, const ImgParams& a, int E, Load 
         }
         __syncthreads();
         // D
+        if constexpr (FAST) {
+            const int sub = lane & 7;
+            for (int r0 = 4 * warp; r0 < MPN; r0 += 4 * nw) {
+                const int row = min(r0 + (lane >> 3), MPN - 1);
+                const int m = row / P;
+                const double* arow = im.a_inv + (size_t)row * P;
+                double c = 0.0, s = 0.0;
+#pragma unroll 4
+                for (int k = sub; k < P; k += 8) {
+                    const double av = __ldg(arow + k);
+                    c += av * rhs_c[m * P + k];
+                    s += av * rhs_s[m * P + k];
+                }
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) {
+                    c += __shfl_xor_sync(0xffffffffu, c, o);
+                    s += __shfl_xor_sync(0xffffffffu, s, o);
+                }
+                if (sub == 0 && r0 + (lane >> 3) < MPN) {
+                    sig_c[row] = c;
+                    sig_s[row] = s;
+                }
+            }
+        } else
         for (int row = warp; row < MPN; row += nw) {
             const int m = row / P;
             const double* arow = im.a_inv + (size_t)row * P;
@@ -340,9 +443,74 @@ __device__ void group_force(const SptImage& im, const ImgParams& a, int E, Load 
         __syncthreads();
     }
     // E
-    for (int i = warp; i < E; i += nw) {
-        const double qi = sq[i];
+    int wpp = 1;  // warps a particle (FAST): then every warp passes the loop and its barrier once
+    if constexpr (FAST)
+        while (2 * wpp * E <= nw) wpp *= 2;
+    const int wsub = warp % wpp;
+    __shared__ double s_split[3 * 8];
+    for (int i0 = warp / wpp; wpp > 1 ? i0 < nw / wpp : i0 < E; i0 += nw / wpp) {
+        const int i = i0 < E ? i0 : 0;
+        const double qi = i0 < E ? sq[i] : 0.0;
         double f0 = 0.0, f1 = 0.0, f2 = 0.0;
+        double er = 0.0, ez = 0.0, ep = 0.0;
+        if (qi != 0.0 && wb[i] > 0.0) {
+            const double zi = sz[i], rq = srho[i];
+            const double* ci = cs + i * (nm + 1);
+            const double* si = sn + i * (nm + 1);
+            double q[MP + 1];
+            const int NQ = im.n_quad;
+            for (int k = lane + 32 * wsub; k < NQ; k += 32 * wpp) {
+                const double rk = __ldg(im.quad + k), zk = __ldg(im.quad + NQ + k);
+                const double lk = __ldg(im.quad + 2 * NQ + k), tk = __ldg(im.quad + 3 * NQ + k);
+                const int jk = (int)__ldg(im.quad + 4 * NQ + k);
+                const double chi = chi_of(rq, zi, rk, zk);
+                double dq0;
+                if constexpr (FAST) toroidal_fast<MP>(chi, M, q, dq0);
+                else toroidal<MP>(chi, M, q, dq0);
+                double SQ = 0.0, T = 0.0, SA = 0.0, c0 = 0.0;
+#pragma unroll
+                for (int m = 0; m <= MP; ++m) {
+                    if (m <= nm) {
+                        const double a0 = sig_c[m * P + jk], a1 = sig_c[m * P + jk + 1];
+                        const double b0 = sig_s[m * P + jk], b1 = sig_s[m * P + jk + 1];
+                        const double dc = (a0 + tk * (a1 - a0)) * lk;
+                        const double ds = (b0 + tk * (b1 - b0)) * lk;
+                        const double cmv = dc * ci[m] + ds * si[m];
+                        const double amv = dc * si[m] - ds * ci[m];
+                        SQ += cmv * q[m];
+                        SA += amv * (double)m * q[m];
+                        if (m == 0) c0 = cmv;
+                        else T += cmv * (m - 0.5) * (chi * q[m] - q[m - 1]);
+                    }
+                }
+                const double SD = c0 * dq0 + T / ((chi - 1.0) * (chi + 1.0));
+                const double pref = sqrt(rk / rq) / (2.0 * kPi);
+                const double dzq = zi - zk;
+                const double dchi_drho = (rq * rq - rk * rk - dzq * dzq) / (2.0 * rk * rq * rq);
+                const double dchi_dz = dzq / (rk * rq);
+                er -= pref * (-SQ / (2.0 * rq) + SD * dchi_drho);
+                ez -= pref * SD * dchi_dz;
+                ep += pref * SA;
+            }
+            er = warp_sum(er);
+            ez = warp_sum(ez);
+            ep = warp_sum(ep);
+        }
+        if (FAST && wpp > 1) {
+            if (lane == 0) {
+                s_split[3 * warp] = er;
+                s_split[3 * warp + 1] = ez;
+                s_split[3 * warp + 2] = ep;
+            }
+            __syncthreads();
+            er = ez = ep = 0.0;
+            for (int v = 0; v < wpp; ++v) {
+                er += s_split[3 * (warp - wsub + v)];
+                ez += s_split[3 * (warp - wsub + v) + 1];
+                ep += s_split[3 * (warp - wsub + v) + 2];
+            }
+            if (wsub != 0 || i0 >= E) continue;
+        }
         if (qi != 0.0) {
             const double xi = px[i], yi = py[i], zi = sz[i];
             double far0 = 0.0, far1 = 0.0, far2 = 0.0;
@@ -365,46 +533,7 @@ __device__ void group_force(const SptImage& im, const ImgParams& a, int E, Load 
             double n0 = 0.0, n1 = 0.0, n2 = 0.0;
             if (w > 0.0) {
                 const double rq = srho[i], cq = sc[i], sqn = ss[i];
-                const double* ci = cs + i * (nm + 1);
-                const double* si = sn + i * (nm + 1);
-                double er = 0.0, ez = 0.0, ep = 0.0;
-                double q[MP + 1];
-                const int NQ = im.n_quad;
-                for (int k = lane; k < NQ; k += 32) {
-                    const double rk = __ldg(im.quad + k), zk = __ldg(im.quad + NQ + k);
-                    const double lk = __ldg(im.quad + 2 * NQ + k), tk = __ldg(im.quad + 3 * NQ + k);
-                    const int jk = (int)__ldg(im.quad + 4 * NQ + k);
-                    const double chi = chi_of(rq, zi, rk, zk);
-                    double dq0;
-                    toroidal<MP>(chi, M, q, dq0);
-                    double SQ = 0.0, T = 0.0, SA = 0.0, c0 = 0.0;
-#pragma unroll
-                    for (int m = 0; m <= MP; ++m) {
-                        if (m <= nm) {
-                            const double a0 = sig_c[m * P + jk], a1 = sig_c[m * P + jk + 1];
-                            const double b0 = sig_s[m * P + jk], b1 = sig_s[m * P + jk + 1];
-                            const double dc = (a0 + tk * (a1 - a0)) * lk;
-                            const double ds = (b0 + tk * (b1 - b0)) * lk;
-                            const double cmv = dc * ci[m] + ds * si[m];
-                            const double amv = dc * si[m] - ds * ci[m];
-                            SQ += cmv * q[m];
-                            SA += amv * (double)m * q[m];
-                            if (m == 0) c0 = cmv;
-                            else T += cmv * (m - 0.5) * (chi * q[m] - q[m - 1]);
-                        }
-                    }
-                    const double SD = c0 * dq0 + T / ((chi - 1.0) * (chi + 1.0));
-                    const double pref = sqrt(rk / rq) / (2.0 * kPi);
-                    const double dzq = zi - zk;
-                    const double dchi_drho = (rq * rq - rk * rk - dzq * dzq) / (2.0 * rk * rq * rq);
-                    const double dchi_dz = dzq / (rk * rq);
-                    er -= pref * (-SQ / (2.0 * rq) + SD * dchi_drho);
-                    ez -= pref * SD * dchi_dz;
-                    ep += pref * SA;
-                }
-                er = warp_sum(er);
-                ez = warp_sum(ez);
-                ep = warp_sum(ep) / rq;
+                ep /= rq;
                 double e0 = er * cq - ep * sqn, e1 = er * sqn + ep * cq, e2 = ez;
                 const double qx = rq * cq, qy = rq * sqn;
                 double m0 = 0.0, m1 = 0.0, m2 = 0.0;

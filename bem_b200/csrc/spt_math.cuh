@@ -124,6 +124,36 @@ __device__ __forceinline__ double rcp_pos(double x) {
     return fma(y, e, y);
 }
 
+// K(1-p), E(1-p) with the steps of the far sums' ring kernel: below 1e-3 six
+// terms of the series (what is left out is below 1e-19), else three roots of
+// the AGM and its series in the last half difference (1e-17).
+__device__ __forceinline__ void ellip_ke_fast(double p, double& K, double& E) {
+    if (p < 1e-3) {
+        const double L = -0.5 * log(p);
+        auto h6 = [&](const double* c) {
+            double v = c[5];
+#pragma unroll
+            for (int n = 4; n >= 0; --n) v = fma(v, p, c[n]);
+            return v;
+        };
+        K = fma(L, h6(kSerK), h6(kSerKd));
+        E = fma(0.5 * p, fma(L, h6(kSerE), h6(kSerEd)), 1.0);
+        return;
+    }
+    const double b0 = sqrt_pos(p);
+    const double t1 = 1.0 - b0, a1 = 0.5 * (1.0 + b0), g1 = sqrt_pos(b0);
+    const double t2 = a1 - g1, a2 = 0.5 * (a1 + g1), g2 = sqrt_pos(a1 * g1);
+    const double t3 = a2 - g2, a3 = 0.5 * (a2 + g2), g3 = sqrt_pos(a2 * g2);
+    const double t4 = a3 - g3, im = rcp_pos(0.5 * (a3 + g3));
+    const double e = 0.5 * t4 * im, e2 = e * e;
+    double S = fma(0.25 * t1, t1, 0.5 * (1.0 - p));
+    S = fma(0.5 * t2, t2, S);
+    S = fma(t3, t3, S);
+    S = fma(fma(0.25, e2, 2.0) * t4, t4, S);
+    K = im * fma(e2, fma(e2, 9.0 / 64.0, 0.25), 1.0) * (0.5 * kPi);
+    E = K * (1.0 - S);
+}
+
 // Near-axis Taylor branch of the ring field (rho^2 < 1e-10 (a^2 + z^2)), out
 // of line for the same reason as ellip_ke_series.
 static __device__ __noinline__ void ring_axis_taylor(double rho, double z, double a, double& er, double& ez) {

@@ -1,0 +1,53 @@
+"""spt_image_force where its split of a group over the CTA can go wrong: groups
+of 1, 2, 3, 4 (8, 4, 2, 2 warps a particle), 5, 8, 9 and 33 (one), each alone
+and all in one ragged batch, solution and geometry level, against the oracle
+(1e-11 of the largest force, the bound of the entry point's parity tests)."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("needs a CUDA device", allow_module_level=True)
+
+from bem_b200 import geometry as bg  # noqa: E402
+from bem_b200.constants import ELEMENTARY_CHARGE  # noqa: E402
+from oracle import image_charge as oic  # noqa: E402
+
+SIZES = (1, 2, 3, 4, 5, 8, 9, 33)
+
+
+@pytest.mark.parametrize("n_max", [0, 1, 16, 20])
+@pytest.mark.parametrize("level", ["solution", "geometry"])
+def test_groups_of_every_split_match_one_by_one(level, n_max):
+    geo = bg.HemisphericalTipBEMGeometry(-1e7, 50e-9, z0=3e-9, image_n_max=n_max, sigma=np.zeros(40))
+    sol = geo.image_solution("cuda")
+    rng = np.random.default_rng(n_max)
+    n = sum(SIZES)
+    th, ph = rng.uniform(0, 1.0, n), rng.uniform(0, 6.28, n)
+    r = 50e-9 + 10 ** rng.uniform(-9.5, -6.5, n)
+    pos = np.stack([r * np.sin(th) * np.cos(ph), r * np.sin(th) * np.sin(ph), r * np.cos(th)], -1)
+    act = (rng.random(n) < 0.85).astype(np.uint8)
+    t = lambda v, d=torch.float64: torch.as_tensor(np.ascontiguousarray(v), dtype=d, device="cuda")
+    q = t(np.full(n, -ELEMENTARY_CHARGE))
+    off = np.concatenate([[0], np.cumsum(SIZES)])
+    g = geo.to_struct() if level == "geometry" else None
+    whole = sol.force(t(pos), q, t(act, torch.uint8), t(off, torch.int64), max(SIZES), geometry=g).cpu().numpy()
+    assert np.all(whole[act == 0] == 0.0)
+    for a, b in zip(off[:-1], off[1:]):
+        one = sol.force(t(pos[a:b]), q[a:b].contiguous(), t(act[a:b], torch.uint8), t([0, b - a], torch.int64),
+                        int(b - a), geometry=g).cpu().numpy()
+        # the same group, its right-hand sides perhaps in other partial sums
+        np.testing.assert_allclose(whole[a:b], one, rtol=0, atol=1e-11 * max(np.abs(one).max(), 1e-300))
+        ref = _oracle(geo, sol, pos[a:b], act[a:b], level)
+        np.testing.assert_allclose(whole[a:b], ref, rtol=0, atol=1e-11 * max(np.abs(ref).max(), 1e-300))
+
+
+def _oracle(geo, sol, pos, act, level):
+    ref = oic.ImageSolution(sol.profile, sol.n_max, A=sol.A.cpu().numpy())
+    p, q, a = pos[None], np.full((1, len(pos)), -ELEMENTARY_CHARGE), act[None].astype(bool)
+    if level == "solution":
+        return ref.image_force(p, q, a, sol.d_lo, sol.d_hi)[0]
+    return np.where(a[0][:, None], oic.geometry_image_force(ref, p, q, a, geo.z0, geo.R, z_handoff=geo.z_handoff)[0], 0.0)
