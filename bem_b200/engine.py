@@ -501,6 +501,12 @@ class TraceRecords:
         return out
 
 
+def _columns(p):
+    """The three columns of p [N, 3], contiguous: one copy for all of them (a
+    call of few points is bound by the host's launches and allocations)."""
+    return p.t().contiguous().unbind(0)
+
+
 def accel(geometry, pos, active, charge, mass, group_sizes, charge_to_mass, plummer_radius, device="cuda",
           form="fp64", coulomb_constant=COULOMB_CONSTANT, far_rule="reference"):
     """One stage evaluation through spt_accel; returns acc [N, 3] (torch)."""
@@ -509,14 +515,13 @@ def accel(geometry, pos, active, charge, mass, group_sizes, charge_to_mass, plum
     offs = np.zeros(len(sizes) + 1, dtype=np.int64)
     np.cumsum(sizes, out=offs[1:])
     d = torch.device(device)
-    p = _as_dev(pos, torch.float64, d)
-    x, y, z = (p[:, k].contiguous() for k in range(3))
+    x, y, z = _columns(_as_dev(pos, torch.float64, d))
     act = _as_dev(np.asarray(active, dtype=np.uint8) if not isinstance(active, torch.Tensor) else active.to(torch.uint8),
                   torch.uint8, d)
     q = _as_dev(charge, torch.float64, d).reshape(-1)
     m = _as_dev(mass, torch.float64, d).reshape(-1)
     off_t = torch.as_tensor(offs, device=d)
-    out = [torch.empty_like(x) for _ in range(3)]
+    out = torch.empty((3, len(x)), dtype=torch.float64, device=d)
     a = _lib.SptAccelArgs()
     a.n_groups = len(sizes)
     a.max_group_size = int(sizes.max())
@@ -535,22 +540,21 @@ def accel(geometry, pos, active, charge, mass, group_sizes, charge_to_mass, plum
     _lib.check(_lib.lib().spt_accel(ctypes.byref(a), ctypes.byref(geom),
                                     ctypes.byref(tables.view(far_rule)) if tables is not None else None,
                                     ctypes.c_void_p(stream.cuda_stream)), "spt_accel")
-    return torch.stack(out, dim=-1)
+    return out.t().contiguous()
 
 
 def bem_field(tables, points, form="fp64", far_rule="reference", **rule_kw):
     """Perturbation field of a BEM solution at points [N, 3] (spt_bem_field)."""
     view = tables.view(far_rule, **rule_kw)
     torch = _torch()
-    p = _as_dev(points, torch.float64, tables.seg.device).reshape(-1, 3)
-    x, y, z = (p[:, k].contiguous() for k in range(3))
-    out = [torch.empty_like(x) for _ in range(3)]
+    x, y, z = _columns(_as_dev(points, torch.float64, tables.seg.device).reshape(-1, 3))
+    out = torch.empty((3, x.numel()), dtype=torch.float64, device=tables.seg.device)
     stream = torch.cuda.current_stream(tables.seg.device)
     _lib.check(_lib.lib().spt_bem_field(x.data_ptr(), y.data_ptr(), z.data_ptr(), x.numel(),
                                         ctypes.byref(view), FORMS[form] if isinstance(form, str) else form,
                                         out[0].data_ptr(), out[1].data_ptr(), out[2].data_ptr(),
                                         ctypes.c_void_p(stream.cuda_stream)), "spt_bem_field")
-    return torch.stack(out, dim=-1)
+    return out.t().contiguous()
 
 
 class SurrogateBinding:
