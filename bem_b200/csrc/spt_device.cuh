@@ -2990,7 +2990,14 @@ trace_warp_kernel(const __grid_constant__ SptState st, const __grid_constant__ S
         have = false;
     };
     int pp = 0;  // the current stage's pool
+    // Single electrons are near the surface, where a point is a direct sum, in
+    // the first tenth of their attempts only.  A CTA takes its next ones together,
+    // when all it has are done: then either every warp has a direct point or
+    // none has (replaced one by one, every stage waited for somebody's).
+    const bool together = st.max_group_size == 1;
     for (;;) {
+        const bool may_take =
+            !together || !__syncthreads_or(have && status == SPT_GROUP_RUNNING && att < prm.max_attempts);
         // ready this warp's group for an attempt: take groups from the work
         // queue until one is running and within this call's attempt budget
         double hr = 0.0, next_cp = 0.0, next_out = 0.0;
@@ -2998,7 +3005,7 @@ trace_warp_kernel(const __grid_constant__ SptState st, const __grid_constant__ S
         int out_ptr = 0;
         for (;;) {
             if (!have) {
-                if (queue_empty) break;
+                if (queue_empty || !may_take) break;
                 int gi = 0;
                 if (lane == 0) gi = atomicAdd(work, 1);
                 gi = __shfl_sync(0xffffffffu, gi, 0);

@@ -345,14 +345,20 @@ int far_rule_of(const SptGeometry* g, const SptBem* b) { return is_bem(g->kind) 
 // CTA width of a trace launch: SptTraceParams.cta_threads when it is 32, 64,
 // 128 or 256, else by group size (narrow CTAs for small groups: more groups
 // per SM, fewer warps behind each barrier).  The reference far rule streams
-// 96 KiB node tiles per CTA, so it keeps 256 threads; the learned form needs
-// at least 4 warps (one per 32 TMEM lanes of its 128-row accumulator).
+// 96 KiB node tiles per CTA, so it keeps 256 threads; so does the float64
+// adaptive form for groups of 17 to 64 while four CTAs an SM hold them all, as
+// warps to spare share the direct points (512 groups of 1 to 32 on a micrometre
+// tip: 72 ms, 99 ms with 128 threads; 2000 of them 146 and 129 ms); the learned
+// form needs at least 4 warps (one per 32 TMEM lanes of its 128-row
+// accumulator).
 int trace_threads(const SptState* s, const SptTraceParams* p, int far) {
     const int want = p->cta_threads;
     int t;
     if (want == 32 || want == 64 || want == 128 || want == 256)
         t = want;
     else if (far == SPT_FAR_REFERENCE || s->max_group_size > 64)
+        t = 256;
+    else if (p->form == SPT_FORM_FP64 && s->max_group_size > 16 && s->n_groups <= 4 * 148)
         t = 256;
     else
         t = s->max_group_size > 16 ? 128 : 64;
@@ -421,9 +427,8 @@ int warp_team_grid(const SptState* s, const SptTraceParams* p, const SptGeometry
 
 // One warp-team launch: slope slots after the work-queue counter, grid
 // capped by the slots the scratch holds.  Returns kNotLaunched when the team
-// was not asked for (SPT_TEAM_AUTO) and either the groups do not fill every
-// resident warp of the launch at least once (fewer groups are spread wider by
-// one group per CTA) or the scratch holds fewer slots than a full grid.
+// was not asked for (SPT_TEAM_AUTO) and either there are too few groups or the
+// scratch holds fewer slots than a full grid.
 int run_warp_team(const SptState* s, const SptTraceParams* p, const SptGeometry* g, const SptBem* b, int far,
                   unsigned char* scratch, int64_t scratch_bytes, cudaStream_t stream, const char* who) {
     spt::TraceLaunch t{};
@@ -439,11 +444,20 @@ int run_warp_team(const SptState* s, const SptTraceParams* p, const SptGeometry*
     const long long avail = scratch_bytes > 256 ? (scratch_bytes - 256) / warp_team_slot_bytes(t.threads) : 0;
     const int full = warp_team_grid(s, p, g, b, far);
     if (p->team != SPT_TEAM_WARP) {
-        // the launch's resident CTAs, were there groups for all of them
+        // Too few groups: below three eighths of the launch's resident warps (888
+        // groups on 148 SMs), counted in groups of the largest size -- a few large
+        // groups among small ones are a chain that one CTA each shortens.
+        // Measured, CTA team / warp team: 512 groups of 32 on the post tip 133 /
+        // 196 ms, 2000 of them 452 / 232 ms; 512 single electrons 10.8 / 10.4 ms,
+        // 1024 of them 12.5 / 9.3 ms; 2000 groups of 1 to 32 on a micrometre tip
+        // 129 / 244 ms.
         SptState many = *s;
         many.n_groups = 1 << 30;
-        const long long resident = warp_team_grid(&many, p, g, b, far);
-        if ((long long)s->n_groups < resident * (t.threads / 32) || avail < full) return kNotLaunched;
+        const long long resident = warp_team_grid(&many, p, g, b, far) * (long long)(t.threads / 32);
+        long long full_groups = s->n_groups;
+        if (s->n_particles > 0 && s->n_particles / s->max_group_size < full_groups)
+            full_groups = s->n_particles / s->max_group_size;
+        if (8 * full_groups < 3 * resident || avail < full) return kNotLaunched;
     }
     if (avail < 1)
         return fail(SPT_ERR_ARG, "%s: scratch of %lld bytes holds no warp-team slot of %lld bytes", who,
