@@ -26,6 +26,7 @@ BLOCK_SEGS = 32
 RUN_NODES = 8
 MAP_TAG, MAP_UNIT, MAP_HEADER, MAP_N = 0x4D50, 64, 8, 12
 MAP_REC = 8 + 2 * MAP_N * MAP_N
+MAP_ROOT_BITS, MAP_BITS = 8, 5
 
 _d = ctypes.c_double
 _i32 = ctypes.c_int32

@@ -689,21 +689,24 @@ __device__ __forceinline__ const double* field_map(const SptBem& b) {
                                                        : nullptr;
 }
 
-// Cell that holds (rho, z), or -1: three quadtree levels per table of 64
-// entries, so a point's cell is at most ten dependent loads away; one lane
-// per point.
+// Cell that holds (rho, z), or -1: one table for the first SPT_MAP_ROOT_BITS
+// quadtree levels and tables of SPT_MAP_BITS levels below it, so a point's cell
+// is three or four dependent loads away (with three levels a table throughout it
+// was seven, at L2's latency most of a stage); one lane per point.
 __device__ __forceinline__ int map_find(const double* map, double rho, double z) {
     const double u = rho * __ldg(map), v = (z - __ldg(map + 1)) * __ldg(map);
     if (!(u < 1.0 && v >= 0.0 && v < 1.0)) return -1;
     const unsigned iu = (unsigned)(u * 1073741824.0), iv = (unsigned)(v * 1073741824.0);
     const int* tab = reinterpret_cast<const int*>(map + SPT_MAP_HEADER);
-    int node = 0;
-    for (int sh = 27; sh >= 0; sh -= 3) {
-        const int e = __ldg(tab + node * 64 + ((iv >> sh) & 7) * 8 + ((iu >> sh) & 7));
-        if (e >= -1) return e;
-        node = -2 - e;
+    constexpr int B = SPT_MAP_BITS, R = SPT_MAP_ROOT_BITS;
+    int sh = 30 - R;
+    int e = __ldg(tab + ((iv >> sh) << R) + (iu >> sh));
+    tab += 1 << (2 * R);
+    while (e < -1 && sh >= B) {
+        sh -= B;
+        e = __ldg(tab + ((size_t)(-2 - e) << (2 * B)) + (((iv >> sh) & ((1 << B) - 1)) << B) + ((iu >> sh) & ((1 << B) - 1)));
     }
-    return -1;
+    return e < -1 ? -1 : e;
 }
 
 // (E_rho, E_z) at (rho, z) of cell `leaf`, by one warp; every lane returns

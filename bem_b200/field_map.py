@@ -24,7 +24,7 @@ KAPPA = 3.0          # half-widths from the surface from which a cell is tried
 KAPPA_SURE = 12.0    # ... and taken as it is: (2 KAPPA_SURE)^-N is far below rounding
 REACH = 24.0         # half side of the root square, in radii of the profile's bounding sphere
 MAX_CELLS = 32768    # 76 MB; the levels nearest the surface are left out beyond it
-MAX_LEVEL = 29
+MAX_LEVEL = 28       # the tables' last level: MAP_ROOT_BITS + 4 MAP_BITS
 # thresholds of the samples' sums: Gauss-4 from 16 lengths, Gauss-2 from 1000,
 # the run rule from 8 arclengths, cluster expansions from 4 radii
 SAMPLE_RULE = dict(ratio4=16.0, ratio2=1000.0, ratio_run=8.0, cluster_kappa=4.0)
@@ -51,38 +51,51 @@ def panel_nodes(profile, sigma, n):
 
 
 def link_tables(leaves, divided):
-    """Lookup tables of a quadtree, int32 [n_tables, 64]: three levels a table.
-    leaves: (level, i, j, number) arrays; divided: {level: (i, j)} of the
-    divided cells.  Entry 8 * (j index) + (i index) of a table: the cell's
-    number, -1 for none, -2 - the number of the next table."""
+    """Lookup tables of a quadtree, one int32 array: a root table of the first
+    MAP_ROOT_BITS levels (4^MAP_ROOT_BITS entries, j-major), then tables of
+    MAP_BITS levels each.  leaves: (level, i, j, number) arrays; divided:
+    {level: (i, j)} of the divided cells.  An entry: the cell's number, -1 for
+    none, -2 - the number of the next table."""
+    R, B = _lib.MAP_ROOT_BITS, _lib.MAP_BITS
+    root = np.full((1 << R, 1 << R), -1, dtype=np.int32)
     ids, count = {}, 0
-    for t in range(0, MAX_LEVEL + 1, 3):
+    for t in range(R, MAX_LEVEL + 1, B):
         if t not in divided or len(divided[t][0]) == 0:
             break
         key = (divided[t][0].astype(np.int64) << 32) | divided[t][1]
         order = np.argsort(key)
         ids[t] = (key[order], count + order)
         count += len(key)
-    tab = np.full((count, 8, 8), -1, dtype=np.int32)
+    tab = np.full((count, 1 << B, 1 << B), -1, dtype=np.int32)
+    low = (1 << B) - 1
 
     def table_of(t, i, j):
         key, num = ids[t]
         return num[np.searchsorted(key, (i.astype(np.int64) << 32) | j)]
 
-    for t in list(ids)[1:]:
+    for t in ids:
         i, j = divided[t]
-        tab[table_of(t - 3, i >> 3, j >> 3), j & 7, i & 7] = -2 - table_of(t, i, j)
+        if t == R:
+            root[j, i] = -2 - table_of(t, i, j)
+        else:
+            tab[table_of(t - B, i >> B, j >> B), j & low, i & low] = -2 - table_of(t, i, j)
     lv, li, lj, num = leaves
     for level in np.unique(lv):
         m = lv == level
         i, j, n = li[m], lj[m], num[m]
-        t = (level - 1) // 3 * 3
-        up, rest = level - t, 3 - (level - t)
+        if level <= R:  # few: coarse cells far from the surface
+            w = 1 << (R - level)
+            for a, b, k in zip(i, j, n):
+                root[b * w:(b + 1) * w, a * w:(a + 1) * w] = k
+            continue
+        t = R + (level - R - 1) // B * B
+        up = level - t
         node = table_of(t, i >> up, j >> up)
+        rest = B - up
         for dj in range(1 << rest):
             for di in range(1 << rest):
-                tab[node, ((j << rest) + dj) & 7, ((i << rest) + di) & 7] = n
-    return tab.reshape(count, 64)
+                tab[node, ((j << rest) + dj) & low, ((i << rest) + di) & low] = n
+    return np.concatenate([root.reshape(-1), tab.reshape(-1)])
 
 
 def build(tables):
@@ -149,7 +162,7 @@ def build(tables):
         out[start: start + 4] = t64([1.0 / side, z_lo, float(rec_at), float(p8_at)])
         out[start + p8_at:] = t64(p8.reshape(-1))
         out[start + _lib.MAP_HEADER: start + _lib.MAP_HEADER + tab.size // 2] = torch.as_tensor(
-            tab.reshape(-1), device=dev).view(torch.float64)
+            tab, device=dev).view(torch.float64)
         out[start + rec_at: start + p8_at] = torch.cat(records).reshape(-1)
         torch.cuda.current_stream(dev).synchronize()
     return out, (_lib.MAP_TAG << 16) | (start // unit)

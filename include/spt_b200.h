@@ -220,15 +220,18 @@ typedef struct {
  * doubles: a header of SPT_MAP_HEADER (1 / side of the root square, its lowest
  * z, the offset of the cell records, the offset of the panels' Gauss-8 nodes --
  * rows rho, z, w of 8 n_seg, segment-major, w = area * density --; the root's
- * lowest rho is 0), int32 tables of 64
- * entries (three quadtree levels each, entry 8 * z index + rho index: a cell's
- * number, -1 for none, or -2 - the number of the next table), then one record
+ * lowest rho is 0), an int32 table of 4^SPT_MAP_ROOT_BITS entries (the first
+ * quadtree levels, z-index major: a cell's number, -1 for none, or -2 - the
+ * number of the next table), int32 tables of 4^SPT_MAP_BITS entries (the levels
+ * below, alike), then one record
  * of SPT_MAP_REC per cell: centre rho, centre z, 1 / half-width, 5 unused, and
  * coefficient (component c, rho power i, z power j) at 8 + (2 j + c) *
  * SPT_MAP_N + i. */
 #define SPT_MAP_TAG 0x4d50u
 #define SPT_MAP_UNIT 64
 #define SPT_MAP_HEADER 8
+#define SPT_MAP_ROOT_BITS 8
+#define SPT_MAP_BITS 5
 #define SPT_MAP_N 12
 #define SPT_MAP_REC (8 + 2 * SPT_MAP_N * SPT_MAP_N)
 /* a cell keeps this many panel lengths from each panel: the quadrature changes

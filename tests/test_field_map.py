@@ -9,16 +9,16 @@ from bem_b200 import field_map as fm
 
 
 def _find(tab, u, v):
-    iu, iv, node = int(u * 2**30), int(v * 2**30), 0
-    for sh in range(27, -1, -3):
-        e = tab[node, ((iv >> sh) & 7) * 8 + ((iu >> sh) & 7)]
-        if e >= -1:
-            return e
-        node = -2 - e
-    return -1
+    R, B = fm._lib.MAP_ROOT_BITS, fm._lib.MAP_BITS
+    iu, iv, sh, low = int(u * 2**30), int(v * 2**30), 30 - R, (1 << B) - 1
+    e = tab[((iv >> sh) << R) + (iu >> sh)]
+    while e < -1 and sh >= B:
+        sh -= B
+        e = tab[(1 << 2 * R) + ((-2 - e) << 2 * B) + (((iv >> sh) & low) << B) + ((iu >> sh) & low)]
+    return e if e >= -1 else -1
 
 
-@pytest.mark.parametrize("depth", [1, 2, 3, 4, 7, 12])
+@pytest.mark.parametrize("depth", [1, 2, 3, 7, 8, 9, 13, 14, 18])
 def test_link_tables_find_every_cell(depth):
     rng = np.random.default_rng(depth)
     i = j = np.zeros(1, dtype=np.int64)
