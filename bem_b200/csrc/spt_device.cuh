@@ -3357,6 +3357,23 @@ int accel_launch(const SptAccelArgs* a, const SptGeometry* g, const SptBem& bem,
     return (int)cudaGetLastError();
 }
 
+// Whether an output of spt_accel overlaps an input: then each group's CTA must
+// read its inputs before it writes anything, as the one-launch form does.
+inline bool accel_in_place(const SptAccelArgs* a) {
+    const uintptr_t n = 8 * (uintptr_t)(a->n_particles > 0 ? a->n_particles : (long long)a->n_groups * a->max_group_size);
+    const double* in[] = {a->x, a->y, a->z, a->charge, a->mass};
+    const double* out[] = {a->ax, a->ay, a->az};
+    for (const double* o : out) {
+        const uintptr_t p = reinterpret_cast<uintptr_t>(o), act = reinterpret_cast<uintptr_t>(a->active);
+        for (const double* i : in) {
+            const uintptr_t q = reinterpret_cast<uintptr_t>(i);
+            if (p < q + n && q < p + n) return true;
+        }
+        if (p < act + n / 8 && act < p + n) return true;
+    }
+    return false;
+}
+
 // The float64 form of a BEM geometry in two launches: the field of all
 // particles at once into ax, ay, az -- one point a warp or a point split over
 // several, whatever fills the SMs, where one CTA per group leaves them idle
@@ -3418,7 +3435,11 @@ int accel_dispatch(const SptAccelArgs* a, const SptGeometry* g, const SptBem& be
     constexpr bool kBem = KIND == SPT_GEOM_TIP_BEM || KIND == SPT_GEOM_WELL_BEM || KIND == SPT_GEOM_POST_BEM;
     const int far = kBem ? bem.far_rule : SPT_FAR_REFERENCE;
     if constexpr (kBem) {
-        if (a->form == SPT_FORM_FP64) return accel_launch_split<KIND>(a, g, bem, stream);
+        if (a->form == SPT_FORM_FP64 && !accel_in_place(a)) return accel_launch_split<KIND>(a, g, bem, stream);
+        if (a->form == SPT_FORM_FP64 && far == SPT_FAR_REFERENCE)
+            return accel_launch<KIND, SPT_FORM_FP64, SPT_FAR_REFERENCE>(a, g, bem, stream);
+        if (a->form == SPT_FORM_FP64 && far == SPT_FAR_ADAPTIVE)
+            return accel_launch<KIND, SPT_FORM_FP64, SPT_FAR_ADAPTIVE>(a, g, bem, stream);
         if (a->form == SPT_FORM_MIXED && far == SPT_FAR_REFERENCE)
             return accel_launch<KIND, SPT_FORM_MIXED, SPT_FAR_REFERENCE>(a, g, bem, stream);
         if (a->form == SPT_FORM_MIXED && far == SPT_FAR_ADAPTIVE)

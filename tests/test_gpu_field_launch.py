@@ -92,6 +92,13 @@ def test_stage_of_ragged_groups_is_its_groups_alone(kind, rule):
     got = out.T.cpu().numpy()
     np.testing.assert_array_equal(got[:1], 7.0)
     np.testing.assert_allclose(got[1:], whole[1:], rtol=0, atol=1e-12 * np.linalg.norm(whole, axis=-1).max())
+    # in place: the accelerations over the positions
+    a.n_groups, a.n_particles, a.group_offset = len(sizes), n, to.data_ptr()
+    a.ax, a.ay, a.az = a.x, a.y, a.z
+    _lib.check(_lib.lib().spt_accel(ctypes.byref(a), ctypes.byref(s), ctypes.byref(view),
+                                    ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "spt_accel")
+    got = torch.stack([x, y, z], -1).cpu().numpy()
+    np.testing.assert_allclose(got, whole, rtol=0, atol=1e-12 * np.linalg.norm(whole, axis=-1).max())
 
 
 def test_on_surface_offset_around_its_threshold():
