@@ -305,6 +305,7 @@ struct Ctx {
     uint64_t* bars;
     uint32_t phase[3];          // parity of the next phase to wait for on bars[0..2] (identical in every thread)
     unsigned long long* cnt;    // shared-memory counter partials of the CTA (flushed by flush_counters)
+    unsigned long long pairs = 0;  // this thread's pair interactions since the last group
     // learned form
     uint8_t *act, *wt;          // BF16 operand tiles (activations, weights), canonical K-major, 32 KiB each
     double *sout, *st, *sd;     // surrogate E (rho, z) per record; closest-point parameter and distance
@@ -2088,15 +2089,15 @@ __device__ void stage_accel(Ctx& c, double* out, int* status_flag) {
 
     // 3. per live particle: field + pair sums over the live sources.  Each
     // target's sources are split over T lanes of a warp (as many as the CTA has
-    // threads per live particle, a power of two, at most 32), whose partial sums
-    // are added with shuffles.  Mixed form: the sums run in float32 first; a
+    // threads per live particle and no more than their number asks for, a power
+    // of two, at most 32), whose partial sums are added with shuffles.  Mixed form: the sums run in float32 first; a
     // target whose sum of |float32 terms| / m exceeds kappa times its whole
     // acceleration is summed again in float64.
     const int nl = c.nl[0];
     for (int i = tid; i < E; i += c.nt)
         if (!c.live[i]) out[i] = out[E + i] = out[2 * E + i] = 0.0;
     int T = 1;
-    while (T < 32 && T * 2 * nl <= c.nt) T *= 2;
+    while (T < 32 && T < nl && T * 2 * nl <= c.nt) T *= 2;
     const int per_pass = c.nt / T;
     const int sub = tid & (T - 1);
     const int lead = (tid & 31) & ~(T - 1);  // lane of the target's first sub-lane
@@ -2243,8 +2244,8 @@ __device__ void stage_accel(Ctx& c, double* out, int* status_flag) {
             out[2 * E + i] = az;
         }
     }
-    count_add(c, SPT_CNT_FP64_TARGETS, redone);
-    count_add(c, SPT_CNT_PAIR_EVALS, pairs);
+    if constexpr (FORM != SPT_FORM_FP64) count_add(c, SPT_CNT_FP64_TARGETS, redone);
+    c.pairs += pairs;  // counted once a group: a warp sum here would be in every stage's chain
     __syncthreads();
 }
 
@@ -2676,6 +2677,8 @@ trace_kernel(const __grid_constant__ SptState st, const __grid_constant__ SptTra
             st.n_accepted[g] = gs.n_acc;
             st.n_rejected[g] = gs.n_rej;
         }
+        count_add(c, SPT_CNT_PAIR_EVALS, c.pairs);
+        c.pairs = 0;
         __syncthreads();
         flush_counters(c, prm.counters);
         __syncthreads();
