@@ -150,6 +150,7 @@ __global__ void __launch_bounds__(kThreads, MP <= 16 ? 2 : 1) image_force_kernel
     for (int g = blockIdx.x; g < a.n_groups; g += gridDim.x) {
         const long long off = a.group_offset[g];
         const int E = (int)(a.group_offset[g + 1] - off);
+        if (E <= 0) continue;  // an empty group: nothing to write (alike in every thread)
         auto load = [&](int i, double& x, double& y, double& z, double& q) {
             x = a.x[off + i];
             y = a.y[off + i];

@@ -445,7 +445,7 @@ __device__ void group_force(const SptImage& im, const ImgParams& a, int E, Load 
     // E
     int wpp = 1;  // warps a particle (FAST): then every warp passes the loop and its barrier once
     if constexpr (FAST)
-        while (2 * wpp * E <= nw) wpp *= 2;
+        while (wpp < nw && 2 * wpp * E <= nw) wpp *= 2;
     const int wsub = warp % wpp;
     __shared__ double s_split[3 * 8];
     for (int i0 = warp / wpp; wpp > 1 ? i0 < nw / wpp : i0 < E; i0 += nw / wpp) {

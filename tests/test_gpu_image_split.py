@@ -51,3 +51,29 @@ def _oracle(geo, sol, pos, act, level):
     if level == "solution":
         return ref.image_force(p, q, a, sol.d_lo, sol.d_hi)[0]
     return np.where(a[0][:, None], oic.geometry_image_force(ref, p, q, a, geo.z0, geo.R, z_handoff=geo.z_handoff)[0], 0.0)
+
+
+@pytest.mark.parametrize("level", ["solution", "geometry"])
+def test_empty_groups_leave_the_others_as_they_are(level):
+    """Empty groups first, last, between others and alone: the forces are, bit
+    for bit, those of the batch without them (a group's sums depend on its own
+    particles and the launch's largest size only), and nothing else is written."""
+    geo = bg.HemisphericalTipBEMGeometry(-1e7, 50e-9, z0=3e-9, image_n_max=16, sigma=np.zeros(40))
+    sol = geo.image_solution("cuda")
+    rng = np.random.default_rng(7)
+    sizes = [0, 0, 3, 0, 1, 0, 0, 9, 0]
+    n = sum(sizes)
+    th, ph = rng.uniform(0, 1.0, n), rng.uniform(0, 6.28, n)
+    r = 50e-9 + 10 ** rng.uniform(-9.5, -6.5, n)
+    t = lambda v, d=torch.float64: torch.as_tensor(np.ascontiguousarray(v), dtype=d, device="cuda")
+    pos = t(np.stack([r * np.sin(th) * np.cos(ph), r * np.sin(th) * np.sin(ph), r * np.cos(th)], -1))
+    q, act = t(np.full(n, -ELEMENTARY_CHARGE)), t(np.ones(n), torch.uint8)
+    g = geo.to_struct() if level == "geometry" else None
+    off = lambda s: t(np.concatenate([[0], np.cumsum(s)]), torch.int64)
+    full = sol.force(pos, q, act, off([s for s in sizes if s]), 9, geometry=g)
+    out = torch.full((3, n), 7.0, dtype=torch.float64, device="cuda")
+    assert torch.equal(sol.force(pos, q, act, off(sizes), 9, geometry=g, out=out), full)
+    assert torch.isfinite(full).all()
+    out.fill_(7.0)
+    sol.force(pos, q, act, off([0, 0]), 9, geometry=g, out=out)
+    assert (out == 7.0).all()
