@@ -3285,15 +3285,15 @@ struct TraceLaunch {
 
 // Which points a field launch (spt_field.cu) evaluates: points 0 .. n-1
 // (active NULL), or of the particles group_offset[0] .. group_offset[n_groups]
-// - 1, at most n, the active ones in the geometry's valid region below its
-// handoff.
+// - 1, at most `most`, the active ones in the geometry's valid region below its
+// handoff (the others' field is set to zero).
 struct FieldMask {
     const uint8_t* active;
     const int64_t* group_offset;
     int n_groups;
     SptGeometry g;
 };
-int launch_field(const double* x, const double* y, const double* z, long long n, const SptBem& b,
+int launch_field(const double* x, const double* y, const double* z, long long n, long long most, const SptBem& b,
                  const FieldMask& mask, double* ex, double* ey, double* ez, cudaStream_t st);
 
 // Shared memory and grid of a trace launch; returns 0 or a cudaError_t.
@@ -3381,13 +3381,14 @@ inline bool accel_in_place(const SptAccelArgs* a) {
 // particles at once into ax, ay, az -- one point a warp or a point split over
 // several, whatever fills the SMs, where one CTA per group leaves them idle
 // for few groups and waits for its slowest point for many -- then the groups'
-// pair sums.  Either far rule: only the first launch depends on it.
+// pair sums.  Either far rule: only the first launch depends on it.  Every
+// particle of the groups gets its field whatever a caller left in n_particles.
 template <int KIND>
 int accel_launch_split(const SptAccelArgs* a, const SptGeometry* g, const SptBem& bem, cudaStream_t stream) {
     const FieldMask mask{a->active, a->group_offset, a->n_groups, *g};
     const long long most = (long long)a->n_groups * a->max_group_size;
     const long long n = a->n_particles > 0 && a->n_particles < most ? a->n_particles : most;
-    const int e = launch_field(a->x, a->y, a->z, n, bem, mask, a->ax, a->ay, a->az, stream);
+    const int e = launch_field(a->x, a->y, a->z, n, most, bem, mask, a->ax, a->ay, a->az, stream);
     if (e == -1) return (int)cudaErrorInvalidValue;
     if (e) return e;
     return accel_launch<KIND, SPT_FORM_FP64, SPT_FAR_REFERENCE, true>(a, g, bem, stream);

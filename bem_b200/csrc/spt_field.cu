@@ -15,7 +15,10 @@ __device__ __forceinline__ long long field_range(const FieldMask& m, long long n
 }
 
 // Points the caller wants: all of them, or (spt_accel) the active particles in
-// the valid region with blend weight > 0.
+// the valid region with blend weight > 0.  The others get a zero field:
+// spt_accel's second launch makes this test again, compiled by itself, and a
+// point on the threshold to the last bit must not find there what the caller's
+// memory held.
 __device__ __forceinline__ bool field_wanted(const FieldMask& m, long long i, double x, double y, double z) {
     if (!m.active) return true;
     if (!m.active[i] || !(blend_weight(z, m.g.z_handoff) > 0.0)) return false;
@@ -62,6 +65,7 @@ field_points_kernel(const double* x, const double* y, const double* z, long long
         py = y[i];
         pz = z[i];
         in = field_wanted(mask, i, px, py, pz);
+        if (!in) ex[i] = ey[i] = ez[i] = 0.0;
     }
     if (map) {
         const double rho = hypot(px, py);
@@ -154,6 +158,7 @@ field_quad_kernel(const double* x, const double* y, const double* z, long long n
         py = y[i];
         pz = z[i];
         in = field_wanted(mask, i, px, py, pz);
+        if (!in && sub == 0 && rank == 0 && lane == 0) ex[i] = ey[i] = ez[i] = 0.0;
     }
     PointCounts cnt;
     if (in && sub == 0) {
@@ -247,8 +252,10 @@ field_quad_kernel(const double* x, const double* y, const double* z, long long n
     }
 }
 
-// Launches the field of n points; 0, a cudaError_t, or -1 for too many points.
-int launch_field(const double* x, const double* y, const double* z, long long n, const SptBem& b,
+// Launches the field of about n points (the work split is chosen for n, the
+// grid covers `most`; what lies past the masked range returns at once); 0, a
+// cudaError_t, or -1 for too many points.
+int launch_field(const double* x, const double* y, const double* z, long long n, long long most, const SptBem& b,
                  const FieldMask& mask, double* ex, double* ey, double* ez, cudaStream_t st) {
     constexpr long long kWarps = 148 * 2 * kMaxWarps;  // resident warps: two CTAs of 128 registers a thread on each SM
     if (b.far_rule == SPT_FAR_ADAPTIVE) {
@@ -257,7 +264,7 @@ int launch_field(const double* x, const double* y, const double* z, long long n,
         long long chunk = n <= kCtas ? 1 : (n <= 2 * kCtas ? 2 : (n <= 4 * kCtas ? 4 : 8 * ((n + kWarps - 1) / kWarps)));
         if (chunk > kMaxThreads) chunk = kMaxThreads;
         const size_t smem = kMaxWarps * (kWarpScratchInts * 4) + (chunk < kMaxWarps ? kSplitDoubles * 8 : 0);
-        const long long grid = (n + chunk - 1) / chunk;
+        const long long grid = (most + chunk - 1) / chunk;
         if (grid > 0x7fffffffLL) return -1;
         const cudaError_t e = cudaFuncSetAttribute(field_points_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    (int)smem);
@@ -272,7 +279,7 @@ int launch_field(const double* x, const double* y, const double* z, long long n,
     int shares = 1;
     while (shares < 64 && n * shares < 4 * kWarps && 2 * shares <= n_run) shares *= 2;
     const int in_cta = shares < kMaxWarps ? shares : kMaxWarps, ranks = shares / in_cta;
-    const long long grid = (n * in_cta + kMaxWarps - 1) / kMaxWarps * ranks;
+    const long long grid = (most * in_cta + kMaxWarps - 1) / kMaxWarps * ranks;
     if (grid > 0x7fffffffLL) return -1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)grid);

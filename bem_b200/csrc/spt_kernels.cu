@@ -628,7 +628,7 @@ int spt_bem_field(const double* x, const double* y, const double* z, int64_t n, 
         return cuda_check(cudaGetLastError(), "bem_field_kernel launch");                                         \
     }
     if (form == SPT_FORM_FP64) {
-        rc = spt::launch_field(x, y, z, n, *b, spt::FieldMask{}, ex, ey, ez, st);
+        rc = spt::launch_field(x, y, z, n, n, *b, spt::FieldMask{}, ex, ey, ez, st);
         if (rc == -1) return fail(SPT_ERR_CAPACITY, "too many points");
         return cuda_check((cudaError_t)rc, "field kernel launch");
     }

@@ -129,3 +129,47 @@ def test_on_surface_offset_around_its_threshold():
         out.append(torch.stack(e, -1).cpu().numpy())
     assert np.isfinite(out[0]).all()
     np.testing.assert_array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("rule", ["reference", "adaptive"])
+@pytest.mark.parametrize("kind", ["post", "well"])
+def test_stage_reads_no_field_that_was_not_written(kind, rule):
+    """Outputs full of NaN on entry, particles on the edge of the valid region
+    to the last bits, n_particles below the groups' total (it only sizes the
+    launch): every acceleration is finite, and that of the one-launch form to
+    1e-12 of the largest, edge points aside (there the two may differ in what
+    they take for vacuum)."""
+    geo = _geometry(kind)
+    rng = np.random.default_rng(5)
+    n, R = 512, geo.R
+    top = geo.L if kind == "post" else 0.0
+    ph = rng.uniform(0, 6.28, n)
+    edge = np.arange(n) < n // 2
+    rho = np.where(edge, R * (1 - 1e-6), R * rng.uniform(0.1, 0.9, n))
+    pos = np.stack([rho * np.cos(ph), rho * np.sin(ph), np.full(n, top)], -1)
+    pos[edge, 2] -= 0.5 * (geo.L if kind == "post" else geo.H)  # the post's and the well's wall
+    pos[~edge, 2] += R * 10 ** rng.uniform(0.1, 0.5, (~edge).sum())
+    pos[edge, 0] *= 1 + rng.integers(-3, 4, edge.sum()) * 2.0**-53
+    t = lambda v, d=torch.float64: torch.as_tensor(np.ascontiguousarray(v), dtype=d, device="cuda")
+    act, q, m, off = t(np.ones(n), torch.uint8), t(np.full(n, gu.Q_E)), t(np.full(n, gu.M_E)), t([0, 200, 300, n], torch.int64)
+    view, s = geo.bem_tables("cuda").view(rule), geo.to_struct()
+
+    def stage(n_particles, in_place=False):
+        x = t(pos.T.copy())
+        out = x if in_place else torch.full((3, n), float("nan"), dtype=torch.float64, device="cuda")
+        a = _lib.SptAccelArgs()
+        a.n_groups, a.max_group_size, a.n_particles, a.group_offset = 3, 256, n_particles, off.data_ptr()
+        a.x, a.y, a.z = (x[k].data_ptr() for k in range(3))
+        a.active, a.charge, a.mass = act.data_ptr(), q.data_ptr(), m.data_ptr()
+        a.charge_to_mass, a.coulomb_constant, a.plummer_radius = gu.CM, engine.COULOMB_CONSTANT, 1e-12
+        a.ax, a.ay, a.az = (out[k].data_ptr() for k in range(3))
+        _lib.check(_lib.lib().spt_accel(ctypes.byref(a), ctypes.byref(s), ctypes.byref(view),
+                                        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "spt_accel")
+        return out.T.cpu().numpy()
+
+    one = stage(n, in_place=True)
+    scale = np.linalg.norm(one[~edge], axis=-1).max()
+    for n_particles in (n, 0, 1, 100):
+        got = stage(n_particles)
+        assert np.isfinite(got).all()
+        np.testing.assert_allclose(got[~edge], one[~edge], rtol=0, atol=1e-12 * scale)
