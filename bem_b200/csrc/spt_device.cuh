@@ -3082,7 +3082,12 @@ trace_warp_kernel(const __grid_constant__ SptState st, const __grid_constant__ S
             break;
         }
         const bool run = have;
-        if (!__syncthreads_or(run)) break;
+        if (!__syncthreads_or(run)) {
+            // nobody runs: the queue is empty, unless the last running single
+            // ended above (no step left), when nobody else was taking groups
+            if (may_take) break;
+            continue;
+        }
         c.E = E;
         const bool live = run && in && (t >= tb) && (t < td);
         // seven stage evaluations (batched_rk45.py:326-370), in step across the CTA

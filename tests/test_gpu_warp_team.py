@@ -202,3 +202,22 @@ def test_tuned_warp_team_is_not_applied_to_other_forms():
     assert fp64.team == _lib.TEAM_AUTO  # the library then gives the warp team the launches it fills
     autotune.apply(dict(cfg, team=_lib.TEAM_CTA), fp64)
     assert fp64.team == _lib.TEAM_CTA
+
+
+def test_single_that_ends_between_attempts_leaves_the_queue_served():
+    """One warp, groups of one taken one after another: the first electron's
+    error overflows (a mass of 1e-185 kg, rtol 0), with min_factor 0 its step
+    shrinks to nothing, and it ends as non-finite before its second attempt.
+    The groups behind it are still traced, in the same launch."""
+    g, geo = _c1()
+    pos, vel, tb, sizes = _groups(g, [1] * 12, 3)
+    mass = np.full(12, gu.M_E)
+    mass[0] = 1e-185
+    tr = engine.Tracer(geo, form="fp64", far_rule="adaptive", z_max=1e-3)
+    b = engine.GroupBatch(pos, vel, tb, np.full(12, gu.Q_E), mass, sizes)
+    p = tr.params(1e-12, 0.0, 1e-12, 1e-12, gu.CM, 100_000, min_factor=0.0, cta_threads=32, team=_lib.TEAM_WARP)
+    p.max_ctas = 1
+    tr.launch(b, p)
+    status, att = b.status.cpu().numpy(), (b.n_accepted + b.n_rejected).cpu().numpy()
+    assert status[0] == _lib.GROUP_NONFINITE and att[0] == 1
+    assert np.all(status[1:] == _lib.GROUP_DONE) and np.all(b.t.cpu().numpy()[1:] == 1e-12)
