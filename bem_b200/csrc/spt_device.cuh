@@ -1877,9 +1877,12 @@ __device__ __forceinline__ void list_live(Ctx& c) {
 }
 
 // 1 / sqrt(x)^3 times q, for positive normal x: the hardware's 20-bit estimate
-// and one third-order Newton step (the next term is 5 e^3 / 16 < 1e-17).
+// and one third-order Newton step (the next term is 5 e^3 / 16 < 1e-17).  From
+// 1e300 on, infinity included (a softening that turns the pair force off, a
+// runaway particle's square), the result is 0, as the quotient's is.
 __device__ __forceinline__ double pair_coef(double x, double q) {
     double y;
+    x = x > 1e300 ? 1e300 : x;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     const double e = fma(-(x * y), y, 1.0);
     y = fma(y * e, fma(0.375, e, 0.5), y);

@@ -201,3 +201,33 @@ def test_bem_solve_matches_reference(fixture):
     Ez = float(g["E_gun"])
     sigma = solve_dirichlet(g["profile"], lambda rho, z: Ez * z)
     np.testing.assert_allclose(sigma, g["sigma"], rtol=1e-9, atol=1e-11 * np.abs(g["sigma"]).max())
+
+
+@pytest.mark.parametrize("kind", ["flat", "tip", "post_bem"])
+@pytest.mark.parametrize("size", [2, 33, 200])
+def test_pair_forces_vanish_at_infinite_softening_and_distance(kind, size):
+    """A softening of infinity, or whose square overflows, turns the pair and
+    image forces off: the accelerations are those without a Coulomb constant,
+    bit for bit.  A particle 1e160 m away (its square overflows too) leaves the
+    others' accelerations as they are without it (another order of the sums:
+    1e-13 of each)."""
+    if kind == "post_bem":
+        g = load_golden("trace_post")
+        spec = dict(kind=kind, E_gun=float(g["E_gun"]), R=float(g["R"]), L=float(g["L"]), z0=float(g["z0"]),
+                    profile=g["profile"], sigma=g["sigma"], n_subdiv=int(g["n_subdiv"]),
+                    z_handoff=float(g["z_handoff"]), kill_z_below=0.0)
+    else:
+        spec = dict(kind=kind, E_gun=-1e7, z0=3e-9, R=50e-9)
+    geo = gu.device_geometry(spec)
+    top, R = spec.get("L", 0.0) + spec["R"] * (kind != "flat"), spec["R"]
+    rng = np.random.default_rng(size)
+    pos = np.stack([rng.normal(0, 0.3 * R, size), rng.normal(0, 0.3 * R, size), top + R * rng.uniform(0.1, 3, size)], -1)
+    q, m, on = np.full(size, gu.Q_E), np.full(size, gu.M_E), np.ones(size, np.uint8)
+    run = lambda p, a, **kw: engine.accel(geo, p, a, q, m, [size], gu.CM, **{"plummer_radius": 1e-12, **kw}).cpu().numpy()
+    off = run(pos, on, coulomb_constant=0.0)
+    for plummer in (1e200, float("inf")):
+        np.testing.assert_array_equal(run(pos, on, plummer_radius=plummer), off)
+    away, rest = pos.copy(), on.copy()
+    away[-1], rest[-1] = (0.0, 0.0, 1e160), 0
+    got, want = run(away, on)[:-1], run(pos, rest)[:-1]
+    assert (np.linalg.norm(got - want, axis=-1) <= 1e-13 * np.linalg.norm(want, axis=-1)).all()
