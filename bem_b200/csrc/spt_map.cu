@@ -63,6 +63,7 @@ map_cells_kernel(const double* cells, const __grid_constant__ SptBem bem, const 
     constexpr int N = SPT_MAP_N;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const double rc = cells[3 * blockIdx.x], zc = cells[3 * blockIdx.x + 1], h = cells[3 * blockIdx.x + 2];
+    const bool axis = rc < 1.5 * h;  // nodes in rho^2 / (2 h^2) - 1, E_rho divided by rho / h
     if (tid < N) s_x[tid] = cheb[tid];
     for (int e = tid; e < kMapN2; e += blockDim.x) {
         s_d[e] = dct[e];
@@ -82,10 +83,11 @@ map_cells_kernel(const double* cells, const __grid_constant__ SptBem bem, const 
         // rho: row i, z: row j; no panel is near
         PointSums S(0, 1);
         double er, ez, mr, mz, mabs;
-        far_adaptive_warp<false>(c, rc + h * s_x[t / N], zc + h * s_x[t % N], S, cnt, mr, mz, mabs);
+        const double u = axis ? sqrt(2.0 * (1.0 + s_x[t / N])) : 1.0;  // rho / h on the axis
+        far_adaptive_warp<false>(c, axis ? h * u : rc + h * s_x[t / N], zc + h * s_x[t % N], S, cnt, mr, mz, mabs);
         S.total(er, ez);
         if (lane == 0) {
-            s_f[t] = er;
+            s_f[t] = er / u;
             s_f[kMapN2 + t] = ez;
         }
         __syncwarp();

@@ -226,7 +226,9 @@ typedef struct {
  * below, alike), then one record
  * of SPT_MAP_REC per cell: centre rho, centre z, 1 / half-width, 5 unused, and
  * coefficient (component c, rho power i, z power j) at 8 + (2 j + c) *
- * SPT_MAP_N + i. */
+ * SPT_MAP_N + i.  The powers are of (rho - centre) / half-width, and of
+ * rho^2 / (2 half-width^2) - 1 in a cell on the axis (centre rho =
+ * half-width), where component 0 is E_rho half-width / rho. */
 #define SPT_MAP_TAG 0x4d50u
 #define SPT_MAP_UNIT 64
 #define SPT_MAP_HEADER 8
@@ -413,7 +415,7 @@ int spt_map_classify(const double* cells, int32_t n, const SptBem* bem, double k
                      double* far_ratio, void* stream);
 
 /* Samples the field of each candidate cell at its SPT_MAP_N x SPT_MAP_N
- * Chebyshev points (adaptive far rule with bem's thresholds, which must be
+ * Chebyshev points, in rho^2 for a cell on the axis (adaptive far rule with bem's thresholds, which must be
  * without a map; no panel may be near) and writes the cell's record, and
  * tail[k] = its largest Chebyshev coefficient of the two highest orders over
  * its largest one.  cheb: the SPT_MAP_N nodes; dct [N, N]: values at the nodes

@@ -92,3 +92,25 @@ def test_points_without_a_cell():
     pts = np.array([[1.0, 0, 0], [0, 0, -5.0], [0, 0, 7.0], [nan, 0, 0], [0, nan, 1e-6], [0, 0, nan], [inf, 0, 0],
                     [0, 0, inf], [0, 0, -inf]])
     np.testing.assert_array_equal(engine.bem_field(tab, pts, far_rule="adaptive").cpu().numpy(), _direct(tab, pts))
+
+
+@pytest.mark.parametrize("fixture", ["bem_sphere", "bem_well", "bem_post", "sigma_c1", "sigma_c3"])
+def test_radial_field_near_the_axis_keeps_its_digits(fixture):
+    """E_rho from 1e-12 to 1e-6 of the surface's distance off the axis against
+    the reference quadrature (whose near-axis terms are exact there): it falls
+    with rho, and so does its error.  A cell's error is bounded by 2e-12 of
+    the field, as at its edges, times rho / half-width; cells are at least a
+    24th of their distance from the surface wide (one twice as wide that is 12
+    half-widths away is taken), so 24 x 2e-12 x rho / distance."""
+    g = load_golden(fixture)
+    prof = g["profile"]
+    tab = BemTables(prof, g["sigma"], int(g["n_subdiv"]) if "n_subdiv" in g else 8)
+    assert tab.field_map() is not None
+    scale = np.hypot(prof[:, 0], prof[:, 1] - prof[:, 1].mean()).max()
+    d = scale * 10 ** np.linspace(-2.6, 0.8, 35)
+    for f in (1e-12, 1e-9, 1e-7, 1e-6):
+        pts = np.stack([f * d, np.zeros_like(d), prof[0, 1] + d], -1)  # every profile starts on the axis
+        got, ref = engine.bem_field(tab, pts, far_rule="adaptive").cpu().numpy(), engine.bem_field(tab, pts).cpu().numpy()
+        uniform = np.abs(float(g["E_gun"])) if "E_gun" in g else np.linalg.norm(ref, axis=-1).max()
+        bound = 24 * 2e-12 * f * np.maximum(np.linalg.norm(ref, axis=-1), uniform)
+        assert (np.abs(got[:, 0] - ref[:, 0]) <= bound).all()
