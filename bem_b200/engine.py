@@ -502,9 +502,10 @@ class TraceRecords:
 
 
 def _columns(p):
-    """The three columns of p [N, 3], contiguous: one copy for all of them (a
-    call of few points is bound by the host's launches and allocations)."""
-    return p.t().contiguous().unbind(0)
+    """The first three columns of p [N, >= 3, ...], contiguous: one copy for all
+    of them (a call of few points is bound by the host's launches and
+    allocations)."""
+    return p.movedim(1, 0)[:3].contiguous().unbind(0)
 
 
 def accel(geometry, pos, active, charge, mass, group_sizes, charge_to_mass, plummer_radius, device="cuda",
@@ -521,7 +522,7 @@ def accel(geometry, pos, active, charge, mass, group_sizes, charge_to_mass, plum
     q = _as_dev(charge, torch.float64, d).reshape(-1)
     m = _as_dev(mass, torch.float64, d).reshape(-1)
     off_t = torch.as_tensor(offs, device=d)
-    out = torch.empty((3, len(x)), dtype=torch.float64, device=d)
+    out = torch.empty((3, *x.shape), dtype=torch.float64, device=d)
     a = _lib.SptAccelArgs()
     a.n_groups = len(sizes)
     a.max_group_size = int(sizes.max())
@@ -540,7 +541,7 @@ def accel(geometry, pos, active, charge, mass, group_sizes, charge_to_mass, plum
     _lib.check(_lib.lib().spt_accel(ctypes.byref(a), ctypes.byref(geom),
                                     ctypes.byref(tables.view(far_rule)) if tables is not None else None,
                                     ctypes.c_void_p(stream.cuda_stream)), "spt_accel")
-    return out.t().contiguous()
+    return out.movedim(0, -1).contiguous()
 
 
 def bem_field(tables, points, form="fp64", far_rule="reference", **rule_kw):

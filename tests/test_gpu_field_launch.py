@@ -173,3 +173,15 @@ def test_stage_reads_no_field_that_was_not_written(kind, rule):
         got = stage(n_particles)
         assert np.isfinite(got).all()
         np.testing.assert_allclose(got[~edge], one[~edge], rtol=0, atol=1e-12 * scale)
+
+
+def test_stage_takes_wider_and_deeper_rows():
+    """Positions as rows of six (positions and velocities) and as [N, 3, 1]:
+    the same accelerations, the latter in its shape."""
+    geo = _geometry("post")
+    rng = np.random.default_rng(6)
+    pos = np.stack([*rng.normal(0, geo.R, (2, 5)), geo.L + geo.R * rng.uniform(1.1, 2, 5)], -1)
+    run = lambda p: engine.accel(geo, p, np.ones(5, np.uint8), np.full(5, gu.Q_E), np.full(5, gu.M_E), [2, 3], gu.CM, 1e-12)
+    want = run(pos)
+    assert torch.equal(run(np.concatenate([pos, pos], 1)), want)
+    assert torch.equal(run(pos[:, :, None]), want[:, None, :])
