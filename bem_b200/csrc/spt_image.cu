@@ -274,7 +274,7 @@ int spt_image_force(const double* x, const double* y, const double* z, const dou
     a.img = im;
     a.prm = spt_img::image_params(im, geom, coulomb_constant, plummer_radius);
     a.fx = fx; a.fy = fy; a.fz = fz;
-    const size_t limit = 227 * 1024;
+    const size_t limit = 227 * 1024 - 8;  // the kernel's static shared int takes the rest
     int chunks = spt_img::kThreads / im.n_nodes;
     chunks = chunks < 1 ? 1 : (chunks > 8 ? 8 : chunks);
     size_t bytes = 0;

@@ -445,9 +445,9 @@ __device__ void group_force(const SptImage& im, const ImgParams& a, int E, Load 
     // E
     int wpp = 1;  // warps a particle (FAST): then every warp passes the loop and its barrier once
     if constexpr (FAST)
-        while (wpp < nw && 2 * wpp * E <= nw) wpp *= 2;
+        while (2 * MPN >= 3 * nw && wpp < nw && 2 * wpp * E <= nw) wpp *= 2;
     const int wsub = warp % wpp;
-    __shared__ double s_split[3 * 8];
+    double* const s_split = rhs_c;  // 3 a warp, where the right-hand sides were (read by D, before its barrier)
     for (int i0 = warp / wpp; wpp > 1 ? i0 < nw / wpp : i0 < E; i0 += nw / wpp) {
         const int i = i0 < E ? i0 : 0;
         const double qi = i0 < E ? sq[i] : 0.0;

@@ -14,6 +14,7 @@ if not torch.cuda.is_available():
 
 from bem_b200 import geometry as bg  # noqa: E402
 from bem_b200.constants import ELEMENTARY_CHARGE  # noqa: E402
+from bem_b200.image_charge import ImageChargeSolution  # noqa: E402
 from oracle import image_charge as oic  # noqa: E402
 
 SIZES = (1, 2, 3, 4, 5, 8, 9, 33)
@@ -77,3 +78,21 @@ def test_empty_groups_leave_the_others_as_they_are(level):
     out.fill_(7.0)
     sol.force(pos, q, act, off([0, 0]), 9, geometry=g, out=out)
     assert (out == 7.0).all()
+
+
+@pytest.mark.parametrize("n_max", [16, 20, 40])
+def test_scratch_to_the_last_byte_of_shared_memory(n_max):
+    """A profile and a max_group_size whose scratch leaves 8 to 200 bytes of a
+    CTA's 227 KiB: the launch takes it, and two electrons' forces are those of
+    a launch for groups of two (other partial sums of the right-hand sides:
+    1e-11 of the largest force)."""
+    P, E = next((P, E) for P in range(40, 65) for E in range(1, 513)
+                if 8 <= 227 * 1024 - 8 * (13 * E + 2 * (n_max + 1) * (E + P * (1 + 256 // P))) <= 200)
+    th = np.linspace(0, 0.5 * np.pi, P)
+    prof = np.stack([47e-9 * np.sin(th), 47e-9 * np.cos(th)], -1)
+    sol = ImageChargeSolution(prof, n_max, 0.5e-9, 5e-9)
+    t = lambda v, d=torch.float64: torch.as_tensor(np.ascontiguousarray(v), dtype=d, device="cuda")
+    pos = t([[10e-9, 5e-9, 60e-9], [-20e-9, 3e-9, 80e-9]])
+    args = (pos, t([-ELEMENTARY_CHARGE] * 2), t([1, 1], torch.uint8), t([0, 2], torch.int64))
+    want = sol.force(*args, 2)
+    assert (sol.force(*args, E) - want).abs().max() <= 1e-11 * want.abs().max()
