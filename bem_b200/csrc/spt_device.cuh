@@ -180,7 +180,7 @@ struct Layout {
     int red;                  // kMaxWarps * 3 * kRound (far-round reduction: E_rho, E_z, sum of |terms|)
     int ints;                 // int region start (in doubles)
     int total_doubles;
-    int live_off, list_off, lidx_off, flags_off;  // in ints from ints start
+    int list_off, lidx_off, live_off, flags_off;  // in ints from ints start
     size_t bytes;
     bool big;                 // slopes/y0/nw in global memory
 };
@@ -195,9 +195,9 @@ constexpr int kWarpChunk = 256;
 constexpr int kWarpRuns = 32;
 constexpr int kWarpScratchInts = 5 * kWarpChunk / 4 + 4 * kWarpRuns + SPT_MAX_CLUSTER_RUNS / 32;
 static_assert(kWarpScratchInts % 2 == 0, "per-warp scratch keeps 8-byte alignment");
-// Shared slots of the points that several warps share (bem_points_direct).
-constexpr int kSplitPoints = kMaxWarps / 2;
-constexpr int kSplitDoubles = kSplitPoints * 256;  // per point: 4 slots x 2 components x 32 lanes
+// Shared slots of the points that several warps share (split_shares: at most
+// half as many points as warps), per point 4 slots x 2 components x 32 lanes.
+__host__ __device__ constexpr int split_doubles(int warps) { return warps / 2 * 256; }
 
 // Shared-memory layout of one CTA for groups of up to E particles.  The far
 // rule decides the big region: node tiles for the reference rule (the TMA
@@ -240,23 +240,25 @@ __host__ __device__ inline Layout make_layout(int E, int far_rule, bool want_sur
     }
     o = (o + 1) & ~1;  // 16-byte alignment for the TMA tiles
     const int base = o;
-    const int n_ints = 3 * E + kRound * 256 / 4 + 4;  // live, list, live list, near flags (bytes), redo flag, live count
+    // list (ints), live list (16 bits each), live (bytes), near flags (bytes), redo flag, live count: no more
+    // than two ints a particle, as the group sizes that a CTA holds are part of the interface
+    L.list_off = 0;
+    L.lidx_off = E;
+    L.live_off = L.lidx_off + (E + 1) / 2;
+    L.flags_off = L.live_off + (E + 3) / 4;
+    const int n_ints = L.flags_off + kRound * 256 / 4 + 3;
     const bool tiles = want_tiles && far_rule == SPT_FAR_REFERENCE;
     const bool lists = want_tiles && far_rule != SPT_FAR_REFERENCE;
     for (int cap = kTileNodes; cap >= 256; cap >>= 1) {
         o = base;
         L.tile_cap = tiles ? cap : 0;
-        L.tiles = o; o += tiles ? 2 * 3 * cap : (lists ? warps * (kWarpScratchInts / 2) + kSplitDoubles : 0);
+        L.tiles = o; o += tiles ? 2 * 3 * cap : (lists ? warps * (kWarpScratchInts / 2) + split_doubles(warps) : 0);
         L.red = o; o += kMaxWarps * 3 * kRound;
         L.ints = o;
         L.total_doubles = o + (n_ints + 1) / 2;
         L.bytes = (size_t)L.total_doubles * 8 + 64;  // + mbarriers
         if (L.bytes <= kMaxSmem || !tiles) break;
     }
-    L.live_off = 0;
-    L.list_off = E;
-    L.lidx_off = 2 * E;
-    L.flags_off = 3 * E;
     return L;
 }
 
@@ -297,9 +299,9 @@ struct Ctx {
     double *y0, *nw_, *sp, *kp, *kv, *tb, *td, *q, *m, *cps, *fld, *img, *bpt, *tiles, *red, *imgs;
     double* ntmp;    // reference rule: near sums' E_z per record (stride 3)
     double* wrec;    // adaptive rule: this warp's record (8 doubles)
-    int* live;
+    unsigned char* live;
     int* list;
-    int* lidx;       // live particles in order
+    uint16_t* lidx;  // live particles in order
     int* nl;         // and their number
     unsigned char* nflag;
     uint64_t* bars;
@@ -364,9 +366,9 @@ __device__ inline void bind(Ctx& c, double* smem, int E, int far_rule, double* s
     c.red = smem + L.red;
     c.wrec = c.red + 8 * (threadIdx.x >> 5);  // (the adaptive rule has no block reduction)
     int* ib = reinterpret_cast<int*>(smem + L.ints);
-    c.live = ib + L.live_off;
     c.list = ib + L.list_off;
-    c.lidx = ib + L.lidx_off;
+    c.lidx = reinterpret_cast<uint16_t*>(ib + L.lidx_off);
+    c.live = reinterpret_cast<unsigned char*>(ib + L.live_off);
     c.nflag = reinterpret_cast<unsigned char*>(ib + L.flags_off);
     c.redo = ib + L.flags_off + kRound * 256 / 4;  // first spare int after the near-flag bytes
     c.nl = c.redo + 1;
@@ -1873,7 +1875,7 @@ __device__ __forceinline__ void list_live(Ctx& c) {
     for (int base = 0; base < c.E; base += 32) {
         const bool on = base + lane < c.E && c.live[base + lane];
         const unsigned m = __ballot_sync(0xffffffffu, on);
-        if (on) c.lidx[n + __popc(m & ((1u << lane) - 1u))] = base + lane;
+        if (on) c.lidx[n + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(base + lane);
         n += __popc(m);
     }
     if (lane == 0) {
@@ -2778,7 +2780,8 @@ constexpr int kWarpSlotDoubles = kWarpSlotComps * 32;
 constexpr int kWarpTeamDoubles = 8 + 4 * 32 + 4 * 32 + 3 * 32 + 16;
 
 __host__ __device__ inline size_t warp_team_smem(int warps) {
-    return (size_t)warps * ((size_t)kWarpScratchInts * 4 + (size_t)kWarpTeamDoubles * 8) + kSplitDoubles * 8;
+    return (size_t)warps * ((size_t)kWarpScratchInts * 4 + (size_t)kWarpTeamDoubles * 8) +
+           (size_t)split_doubles(warps) * 8;
 }
 
 __device__ __forceinline__ double warp_min_all(double v) {
@@ -2975,7 +2978,7 @@ trace_warp_kernel(const __grid_constant__ SptState st, const __grid_constant__ S
     c.tiles = smem;  // far-rule scratch of every warp (far_adaptive_warp takes its own by warp index)
     const WarpTeam w(smem, nw, warp);
     c.wrec = w.rec;
-    double* const part = smem + (warp_team_smem(nw) / 8 - kSplitDoubles);
+    double* const part = smem + (warp_team_smem(nw) / 8 - split_doubles(nw));
     const double* const map = field_map(bem);
     PointCounts pts;
     double* const slot = slots + ((size_t)blockIdx.x * nw + warp) * kWarpSlotDoubles + lane;

@@ -263,7 +263,7 @@ int launch_field(const double* x, const double* y, const double* z, long long n,
         constexpr long long kCtas = 148 * 2;
         long long chunk = n <= kCtas ? 1 : (n <= 2 * kCtas ? 2 : (n <= 4 * kCtas ? 4 : 8 * ((n + kWarps - 1) / kWarps)));
         if (chunk > kMaxThreads) chunk = kMaxThreads;
-        const size_t smem = kMaxWarps * (kWarpScratchInts * 4) + (chunk < kMaxWarps ? kSplitDoubles * 8 : 0);
+        const size_t smem = kMaxWarps * (kWarpScratchInts * 4) + (chunk < kMaxWarps ? split_doubles(kMaxWarps) * 8 : 0);
         const long long grid = (most + chunk - 1) / chunk;
         if (grid > 0x7fffffffLL) return -1;
         const cudaError_t e = cudaFuncSetAttribute(field_points_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

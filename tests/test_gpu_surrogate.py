@@ -249,3 +249,21 @@ def test_learned_form_measured_against_chosen_form():
     assert C["err"] <= 1e-6                         # the chosen form meets the bar
     assert L["per_stage"] < 0.5 * C["per_stage"]    # the network does replace most ring evaluations ...
     assert L["err"] > 1e-6 or L["t"] > C["t"]       # ... but does not beat the chosen form within 1e-6
+
+
+@pytest.mark.parametrize("size", [1, 5, 33, 227, 257, 651])
+def test_group_sizes_the_learned_form_holds(post, size):
+    """The learned form with the reference rule up to the largest group sizes
+    that its shared memory has always held, 227 with the slopes in shared
+    memory and 651 without: one attempt of one group, of which every particle
+    that is alive has moved (by its velocity at least)."""
+    g, geo, model = post
+    rho, z, pts = _points(geo, size, size)
+    vel = np.full((size, 3), 1e5)
+    tr = engine.Tracer(geo, form="surrogate", z_max=1e-3, surrogate=model)
+    b = engine.GroupBatch(pts, vel, np.zeros(size), np.full(size, gu.Q_E), np.full(size, gu.M_E), [size])
+    tr.launch(b, tr.params(1e-12, 1e-3, 1e-9, 1e-9, gu.CM, 1))
+    torch.cuda.synchronize()
+    assert int((b.n_accepted + b.n_rejected)[0]) == 1
+    moved = (b.positions().cpu().numpy() != pts).all(axis=-1)
+    assert np.isfinite(b.positions().cpu().numpy()).all() and (moved.all() or int(b.n_accepted[0]) == 0)
