@@ -408,6 +408,14 @@ __device__ __forceinline__ double seg_dist2(const SptBem& b, int s, double rq, d
     return __dadd_rn(__dmul_rn(dr, dr), __dmul_rn(dz, dz));
 }
 
+// Square root of a squared distance v >= 0 that may be 0: v held at 2^-996 by
+// its high word, as an unsigned number, so that a NaN of either sign stays one
+// (fmax gives the bound for a NaN, and a NaN point was near every panel).
+__device__ __forceinline__ double sqrt_dist2(double v) {
+    const unsigned hi = max((unsigned)__double2hiint(v), (unsigned)(1023 - 996) << 20);
+    return sqrt_pos(__hiloint2double((int)hi, __double2loint(v)));
+}
+
 // near test of bem/axisymmetric.py:566-570 -> (near, projection, distance)
 // FAST (the adaptive rule): a branch-free root, exact to the last bit or two.
 template <bool FAST = false>
@@ -417,7 +425,7 @@ __device__ __forceinline__ bool seg_near(const SptBem& b, int s, double re, doub
     const double along = dr * ur + dz * uz;
     proj = fmin(fmax(along, 0.0), L);
     const double ar = dr - proj * ur, az = dz - proj * uz;
-    if constexpr (FAST) dist = sqrt_pos(fmax(fma(ar, ar, az * az), 1e-300));
+    if constexpr (FAST) dist = sqrt_dist2(fma(ar, ar, az * az));
     else dist = sqrt(ar * ar + az * az);
     return dist < L;
 }
@@ -429,7 +437,7 @@ __device__ __forceinline__ bool seg_near(const SptBem& b, int s, double re, doub
 __device__ __forceinline__ double blk_lower(const SptBem& b, int q, double r, double z) {
     const double cr = __ldg(b.blk + q), cz = __ldg(b.blk + b.blk_stride + q), rad = __ldg(b.blk + 2 * b.blk_stride + q);
     const double dr = r - cr, dz = z - cz;
-    const double dc = sqrt_pos(fmax(fma(dr, dr, dz * dz), 1e-300));
+    const double dc = sqrt_dist2(fma(dr, dr, dz * dz));
     return dc - rad - 1e-9 * (dc + rad);
 }
 __device__ __forceinline__ double blk_lmax(const SptBem& b, int q) { return __ldg(b.blk + 3 * b.blk_stride + q); }

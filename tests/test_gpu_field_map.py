@@ -18,6 +18,8 @@ if not torch.cuda.is_available():
 from bem_b200 import _lib, engine  # noqa: E402
 from bem_b200.tables import BemTables  # noqa: E402
 
+import gpu_util as gu  # noqa: E402
+
 
 def _direct(tab, pts):
     v = tab.view("adaptive", field_map=False)
@@ -114,3 +116,33 @@ def test_radial_field_near_the_axis_keeps_its_digits(fixture):
         uniform = np.abs(float(g["E_gun"])) if "E_gun" in g else np.linalg.norm(ref, axis=-1).max()
         bound = 24 * 2e-12 * f * np.maximum(np.linalg.norm(ref, axis=-1), uniform)
         assert (np.abs(got[:, 0] - ref[:, 0]) <= bound).all()
+
+
+def test_nan_points_are_near_no_panel():
+    """A NaN coordinate is no panel's neighbour: one attempt of such a single
+    electron beside a healthy one counts that one's near panels only (the sinh
+    rule at 71 intervals a panel was what a NaN point cost), and a field call
+    gives the finite points beside NaN ones their own values."""
+    g = load_golden("trace_post")
+    spec = dict(kind="post_bem", E_gun=float(g["E_gun"]), R=float(g["R"]), L=float(g["L"]), z0=float(g["z0"]),
+                profile=g["profile"], sigma=g["sigma"], n_subdiv=int(g["n_subdiv"]), z_handoff=float(g["z_handoff"]),
+                kill_z_below=0.0)
+    geo = gu.device_geometry(spec)
+    near = []
+    for x in ([0.0, float("nan")], [0.0]):
+        pos = np.array([[v, 1e-9, geo.L + geo.R + 1e-11] for v in x])
+        n = len(pos)
+        tr = engine.Tracer(geo, far_rule="adaptive")
+        b = engine.GroupBatch(pos, np.zeros((n, 3)), np.zeros(n), np.full(n, gu.Q_E), np.full(n, gu.M_E), [1] * n)
+        tr.launch(b, tr.params(1e-12, 1e-8, 1e-12, 1e-12, gu.CM, 1))
+        near.append(tr.counter_dict()["near_pairs"])
+    assert near[0] == near[1] > 0
+    tab = geo.bem_tables("cuda")
+    pts = np.stack([np.zeros(64), np.full(64, 1e-9), geo.L + geo.R * (1 + 10.0 ** np.linspace(-6, 1, 64))], -1)
+    want = engine.bem_field(tab, pts, far_rule="adaptive").cpu().numpy()
+    mixed = pts.copy()
+    mixed[1::2, 0] = mixed[::4, 2] = np.nan
+    got = engine.bem_field(tab, mixed, far_rule="adaptive").cpu().numpy()
+    finite = np.isfinite(mixed).all(axis=-1)
+    np.testing.assert_array_equal(got[finite], want[finite])
+    assert np.isnan(got[~finite]).any(axis=-1).all()
