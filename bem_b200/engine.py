@@ -505,7 +505,8 @@ def _columns(p):
     """The first three columns of p [N, >= 3, ...], contiguous: one copy for all
     of them (a call of few points is bound by the host's launches and
     allocations)."""
-    return p.movedim(1, 0)[:3].contiguous().unbind(0)
+    cols = p.t() if p.dim() == 2 and p.shape[1] == 3 else p.movedim(1, 0)[:3]
+    return cols.contiguous().unbind(0)
 
 
 def accel(geometry, pos, active, charge, mass, group_sizes, charge_to_mass, plummer_radius, device="cuda",
@@ -541,7 +542,7 @@ def accel(geometry, pos, active, charge, mass, group_sizes, charge_to_mass, plum
     _lib.check(_lib.lib().spt_accel(ctypes.byref(a), ctypes.byref(geom),
                                     ctypes.byref(tables.view(far_rule)) if tables is not None else None,
                                     ctypes.c_void_p(stream.cuda_stream)), "spt_accel")
-    return out.movedim(0, -1).contiguous()
+    return (out.t() if out.dim() == 2 else out.movedim(0, -1)).contiguous()
 
 
 def bem_field(tables, points, form="fp64", far_rule="reference", **rule_kw):
