@@ -540,16 +540,17 @@ def accel(geometry, pos, active, charge, mass, group_sizes, charge_to_mass, plum
     tables = geometry.bem_tables(d) if geometry.is_bem else None
     stream = torch.cuda.current_stream(d)
     _lib.check(_lib.lib().spt_accel(ctypes.byref(a), ctypes.byref(geom),
-                                    ctypes.byref(tables.view(far_rule)) if tables is not None else None,
+                                    ctypes.byref(tables.view(far_rule, points=x.numel()))
+                                    if tables is not None else None,
                                     ctypes.c_void_p(stream.cuda_stream)), "spt_accel")
     return (out.t() if out.dim() == 2 else out.movedim(0, -1)).contiguous()
 
 
 def bem_field(tables, points, form="fp64", far_rule="reference", **rule_kw):
     """Perturbation field of a BEM solution at points [N, 3] (spt_bem_field)."""
-    view = tables.view(far_rule, **rule_kw)
     torch = _torch()
     x, y, z = _columns(_as_dev(points, torch.float64, tables.seg.device).reshape(-1, 3))
+    view = tables.view(far_rule, points=x.numel(), **rule_kw)
     out = torch.empty((3, x.numel()), dtype=torch.float64, device=tables.seg.device)
     stream = torch.cuda.current_stream(tables.seg.device)
     _lib.check(_lib.lib().spt_bem_field(x.data_ptr(), y.data_ptr(), z.data_ptr(), x.numel(),
@@ -622,8 +623,8 @@ def surrogate_field(tables, binding, points, far_rule="reference"):
     prm = binding.fill(_lib.SptTraceParams())
     stream = torch.cuda.current_stream(tables.seg.device)
     _lib.check(_lib.lib().spt_surrogate_field(x.data_ptr(), y.data_ptr(), z.data_ptr(), x.numel(),
-                                              ctypes.byref(tables.view(far_rule)), ctypes.byref(prm), out[0].data_ptr(),
-                                              out[1].data_ptr(), out[2].data_ptr(),
+                                              ctypes.byref(tables.view(far_rule, points=x.numel())), ctypes.byref(prm),
+                                              out[0].data_ptr(), out[1].data_ptr(), out[2].data_ptr(),
                                               ctypes.c_void_p(stream.cuda_stream)), "spt_surrogate_field")
     return torch.stack(out, dim=-1)
 

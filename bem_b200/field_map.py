@@ -10,6 +10,10 @@ own), and divided otherwise; near a panel (closer than two of its lengths)
 and behind the surface there are no cells, and points there take the direct
 sum, with the Gauss-8 panel nodes that are kept beside the map for it.  Not
 in the reference.
+
+Sampling the cells takes 10 to 250 ms, so it waits until a geometry has been
+asked for about as many points as its direct sums evaluate in that time
+(`worth`); until then its map has no cells, only the panel nodes.
 """
 
 import ctypes
@@ -25,6 +29,10 @@ KAPPA_SURE = 12.0    # ... and taken as it is: (2 KAPPA_SURE)^-N is far below ro
 REACH = 24.0         # half side of the root square, in radii of the profile's bounding sphere
 MAX_CELLS = 32768    # 76 MB; the levels nearest the surface are left out beyond it
 MAX_LEVEL = 28       # the tables' last level: MAP_ROOT_BITS + 4 MAP_BITS
+# points that the direct sums evaluate in the time the cells take: measured 0.9 M
+# (39 panels, 10 ms), 2.3 M (600, 56 ms), 13 M (2000, 180 ms), 7 M (3000, 250 ms)
+WORTH, WORTH_PER_PANEL = 1_000_000, 3000
+GAUSS = {8: np.polynomial.legendre.leggauss(8)}
 # thresholds of the samples' sums: Gauss-4 from 16 lengths, Gauss-2 from 1000,
 # the run rule from 8 arclengths, cluster expansions from 4 radii
 SAMPLE_RULE = dict(ratio4=16.0, ratio2=1000.0, ratio_run=8.0, cluster_kappa=4.0)
@@ -40,14 +48,18 @@ for _k in range(N):
 def panel_nodes(profile, sigma, n):
     """[3, n_seg * n]: the n-point Gauss rule over each whole segment, as
     (rho_q, z_q, area_q * sigma_q), segment-major."""
-    x, w = np.polynomial.legendre.leggauss(n)
+    x, w = GAUSS[n] if n in GAUSS else np.polynomial.legendre.leggauss(n)
     t = 0.5 * (x + 1.0)
     p0, tan = profile[:-1], profile[1:] - profile[:-1]
-    rho = p0[:, 0:1] + t * tan[:, 0:1]
-    z = p0[:, 1:2] + t * tan[:, 1:2]
-    area = 2.0 * np.pi * rho * (np.linalg.norm(tan, axis=-1)[:, None] * 0.5 * w)
-    dens = sigma[:-1, None] + t * (sigma[1:, None] - sigma[:-1, None])
-    return np.stack([rho.ravel(), z.ravel(), (area * dens).ravel()])
+    out = np.empty((3, len(p0), n))
+    rho, z, dens = out
+    np.add(np.multiply(tan[:, 0:1], t, out=rho), p0[:, 0:1], out=rho)
+    np.add(np.multiply(tan[:, 1:2], t, out=z), p0[:, 1:2], out=z)
+    np.add(np.multiply(sigma[1:, None] - sigma[:-1, None], t, out=dens), sigma[:-1, None], out=dens)
+    area = 2.0 * np.pi * rho
+    area *= np.sqrt((tan * tan).sum(axis=-1))[:, None] * 0.5 * w
+    dens *= area
+    return out.reshape(3, -1)
 
 
 def link_tables(leaves, divided):
@@ -98,10 +110,41 @@ def link_tables(leaves, divided):
     return np.concatenate([root.reshape(-1), tab.reshape(-1)])
 
 
+def worth(profile):
+    """The number of points from which the cells of a profile pay."""
+    return WORTH + WORTH_PER_PANEL * (len(profile) - 1)
+
+
+def _lay_out(tables, scale, z_lo, tab, records):
+    """(doubles tensor that starts with the cluster table, SptBem.reserved) of a
+    map on its device.  Synchronises: it may be read on any stream afterwards."""
+    import torch
+
+    dev = tables.seg.device
+    with torch.cuda.device(dev):
+        base, unit = tables.clusters.reshape(-1), _lib.MAP_UNIT
+        start = -(-base.numel() // unit) * unit
+        rec_at = -(-(_lib.MAP_HEADER + tab.size // 2) // 8) * 8
+        p8_at = rec_at + sum(r.numel() for r in records)
+        head = np.zeros(rec_at)
+        head[:4] = scale, z_lo, rec_at, p8_at
+        head[_lib.MAP_HEADER: _lib.MAP_HEADER + tab.size // 2] = tab.view(np.float64)
+        p8 = panel_nodes(tables.profile, tables.sigma, 8).ravel()
+        small = torch.as_tensor(np.concatenate([np.zeros(start - base.numel()), head, p8]), device=dev)
+        gap = start - base.numel() + rec_at
+        out = torch.cat([base, small[:gap], *(r.reshape(-1) for r in records), small[gap:]])
+        torch.cuda.current_stream(dev).synchronize()
+    return out, (_lib.MAP_TAG << 16) | (start // unit)
+
+
+def bare(tables):
+    """The map without cells: a root square of no extent, which holds no point,
+    and the panel nodes."""
+    return _lay_out(tables, np.inf, 0.0, np.zeros(0, dtype=np.int32), [])
+
+
 def build(tables):
-    """The map of a BemTables on its device, as (doubles tensor that starts
-    with the cluster table, SptBem.reserved), or None when there is nothing
-    to map.  Synchronises: the map may be read on any stream afterwards."""
+    """The map of a BemTables with its cells, or None when there is nothing to map."""
     import torch
 
     dev = tables.seg.device
@@ -151,18 +194,4 @@ def build(tables):
         if not kept or 0 not in divided:
             return None
         tab = link_tables(tuple(np.concatenate(c) for c in zip(*kept)), divided)
-        base = tables.clusters.reshape(-1)
-        unit = _lib.MAP_UNIT
-        start = -(-base.numel() // unit) * unit
-        rec_at = -(-(_lib.MAP_HEADER + tab.size // 2) // 8) * 8
-        p8_at = rec_at + n_kept * _lib.MAP_REC
-        p8 = panel_nodes(prof, tables.sigma, 8)
-        out = torch.zeros(start + p8_at + p8.size, dtype=torch.float64, device=dev)
-        out[: base.numel()] = base
-        out[start: start + 4] = t64([1.0 / side, z_lo, float(rec_at), float(p8_at)])
-        out[start + p8_at:] = t64(p8.reshape(-1))
-        out[start + _lib.MAP_HEADER: start + _lib.MAP_HEADER + tab.size // 2] = torch.as_tensor(
-            tab, device=dev).view(torch.float64)
-        out[start + rec_at: start + p8_at] = torch.cat(records).reshape(-1)
-        torch.cuda.current_stream(dev).synchronize()
-    return out, (_lib.MAP_TAG << 16) | (start // unit)
+    return _lay_out(tables, 1.0 / side, z_lo, tab, records)

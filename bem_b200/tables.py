@@ -38,6 +38,7 @@ import threading
 import numpy as np
 
 from . import _lib
+from . import field_map as _field_map
 
 GAUSS4_X, GAUSS4_W = np.polynomial.legendre.leggauss(4)
 GAUSS8_X, GAUSS8_W = np.polynomial.legendre.leggauss(8)
@@ -285,7 +286,10 @@ class BemTables:
             ct, levels = cluster_tables(self.profile, self.sigma, self.n_subdiv)
             self.clusters = torch.as_tensor(np.ascontiguousarray(ct), device=device)
             self.cluster_levels = levels
-        self._map = None          # (doubles, SptBem.reserved) of the field map, or False: none
+        self._map = None          # (doubles, SptBem.reserved) of the field map with its cells, or False: none
+        self._bare = None         # the same without cells, until those pay
+        self._map_points = 0      # points asked for so far
+        self._map_worth = _field_map.worth(self.profile)
         self._map_lock = threading.Lock()
         self.struct = _lib.SptBem()
         s = self.struct
@@ -322,27 +326,46 @@ class BemTables:
         self.image = solution
         self.struct.image = solution.struct
 
-    def field_map(self):
-        """(doubles, SptBem.reserved) of the field map, built on first use, or
-        None: no clusters or CUDA device, nothing to map, no memory for it,
-        or the current stream is being captured (the direct sums then serve;
-        a later view outside the capture builds it)."""
+    def field_map(self, points=None):
+        """(doubles, SptBem.reserved) of the field map, or None: no clusters or
+        CUDA device, or the current stream is being captured (the direct sums
+        then serve; a later view outside the capture builds it).  With `points`,
+        the number of points it is asked for, its cells are sampled once all
+        points asked for cost as much (field_map.worth), and before that the map
+        has none; without, at once.  Where memory for them lacks, the map
+        stays without, until as many points have been asked for again."""
         import torch
+        if self._map:
+            return self._map
         if self.clusters is None or self.seg.device.type != "cuda":
             return None
         with self._map_lock:
-            if self._map is None:
-                if torch.cuda.is_current_stream_capturing():
-                    return None
-                from . import field_map
-                try:
-                    self._map = field_map.build(self) or False
-                except torch.cuda.OutOfMemoryError:
-                    self._map = False
-            return self._map or None
+            if self._map:
+                return self._map
+            self._map_points += points or 0
+            sample = self._map is None and (points is None or self._map_points >= self._map_worth)
+            if self._bare and not sample:
+                return self._bare
+            if torch.cuda.is_current_stream_capturing():
+                self._map_points -= points or 0
+                return self._bare
+            try:
+                if sample:
+                    self._map_points = 0
+                    self._map = _field_map.build(self) or False
+                    if self._map:
+                        return self._map
+            except torch.cuda.OutOfMemoryError:
+                pass
+            try:
+                if self._bare is None:
+                    self._bare = _field_map.bare(self)
+            except torch.cuda.OutOfMemoryError:
+                pass
+            return self._bare
 
     def view(self, far_rule="reference", ratio4=RATIO4, ratio2=RATIO2, ratio_run=RATIO_RUN, bounds=True,
-             cluster_kappa=None, field_map=True):
+             cluster_kappa=None, field_map=True, points=None):
         """An SptBem over these tables with the given far rule (the tables
         must outlive it); ratio_run <= 0 turns the run rule off; bounds=False
         leaves out the run bounds, so every per-point scan visits every
@@ -350,7 +373,9 @@ class BemTables:
         cluster_kappa <= 0 turns the cluster expansions off.  The adaptive
         rule at its default thresholds takes the field map with it
         (field_map=False leaves it out): other thresholds ask for the sums
-        they describe."""
+        they describe.  points: how many points the caller will evaluate with
+        this view, which decides when the map's cells are sampled; None for a
+        view that is kept, as a trace's is: at once."""
         v = _lib.SptBem()
         ctypes.pointer(v)[0] = self.struct
         v.far_rule = _lib.FAR_RULES[far_rule] if isinstance(far_rule, str) else int(far_rule)
@@ -362,7 +387,7 @@ class BemTables:
             v.clusters, v.cluster_kappa = None, 0.0
         if (field_map and bounds and v.far_rule == _lib.FAR_ADAPTIVE
                 and (v.ratio4, v.ratio2, v.ratio_run, v.cluster_kappa) == (RATIO4, RATIO2, RATIO_RUN, CLUSTER_KAPPA)):
-            m = self.field_map()
+            m = self.field_map(points)
             if m is not None:
                 v.clusters, v.reserved = m[0].data_ptr(), m[1]
         return v

@@ -57,3 +57,64 @@ def test_power_coefficients_reproduce_the_samples():
     p = fm.MONO.T @ c @ fm.MONO
     V = x[:, None] ** np.arange(fm.N)
     assert np.abs(V @ p @ V.T - f).max() < 1e-13
+
+
+@pytest.fixture
+def tables(monkeypatch):
+    """The field map's bookkeeping of a 100-panel BemTables, sampling replaced
+    by a count of the calls."""
+    import types
+
+    import torch
+
+    from bem_b200.tables import BemTables
+
+    t = BemTables.__new__(BemTables)
+    t.clusters, t._map_worth = object(), fm.worth(np.zeros((101, 2)))
+    t.seg = types.SimpleNamespace(device=torch.device("cuda"))
+    t._map = t._bare = None
+    t._map_points, t._map_lock = 0, __import__("threading").Lock()
+    t.calls, t.capturing, t.memory = [], False, True
+
+    def build(tab):
+        t.calls.append("cells")
+        if not t.memory:
+            raise torch.cuda.OutOfMemoryError("no memory")
+        return ("cells", 1)
+
+    monkeypatch.setattr(fm, "build", build)
+    monkeypatch.setattr(fm, "bare", lambda tab: t.calls.append("bare") or ("bare", 2))
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: t.capturing)
+    return t
+
+
+def test_cells_are_sampled_when_the_points_asked_for_pay(tables):
+    n = tables._map_worth
+    assert n == fm.WORTH + 100 * fm.WORTH_PER_PANEL
+    for k in (1, 33, n // 2, n - n // 2 - 35):
+        assert tables.field_map(points=k)[0] == "bare"
+    assert tables.calls == ["bare"]
+    assert tables.field_map(points=1)[0] == "cells"
+    assert tables.field_map(points=1)[0] == "cells" and tables.calls == ["bare", "cells"]
+
+
+def test_a_kept_view_samples_the_cells_at_once(tables):
+    assert tables.field_map()[0] == "cells" and tables.calls == ["cells"]
+
+
+def test_nothing_is_built_under_capture(tables):
+    tables.capturing = True
+    assert tables.field_map() is None and tables.field_map(points=10**9) is None and tables.calls == []
+    tables.capturing = False
+    assert tables.field_map(points=1)[0] == "bare"
+    tables.capturing = True
+    assert tables.field_map(points=10**9)[0] == "bare" and tables.calls == ["bare"]
+
+
+def test_lack_of_memory_is_tried_again_after_as_many_points(tables):
+    n = tables._map_worth
+    tables.memory = False
+    assert tables.field_map(points=n)[0] == "bare" and tables.calls == ["cells", "bare"]
+    assert tables.field_map(points=n - 1)[0] == "bare" and tables.calls == ["cells", "bare"]
+    tables.memory = True
+    assert tables.field_map(points=1)[0] == "cells"

@@ -146,3 +146,38 @@ def test_nan_points_are_near_no_panel():
     finite = np.isfinite(mixed).all(axis=-1)
     np.testing.assert_array_equal(got[finite], want[finite])
     assert np.isnan(got[~finite]).any(axis=-1).all()
+
+
+def test_first_calls_do_without_cells_until_they_pay():
+    """A fresh geometry's first calls read a map without cells (every point its
+    own direct sum: the bits that a point near the surface has with cells too)
+    and keep the 2e-12 bound; the call that reaches field_map.worth points has
+    the cells, and then a point's value still does not depend on the points
+    beside it or on their number."""
+    from bem_b200 import field_map
+
+    g = load_golden("bem_sphere")
+    tab = BemTables(g["profile"], g["sigma"], int(g["n_subdiv"]))
+    R = g["profile"][0, 1]
+    rng = np.random.default_rng(3)
+    n = field_map.worth(g["profile"])
+    th, ph, d = rng.uniform(0, np.pi, n), rng.uniform(0, 2 * np.pi, n), 10 ** rng.uniform(-3, 1, n)
+    pts = R * (1 + d)[:, None] * np.stack([np.sin(th) * np.cos(ph), np.sin(th) * np.sin(ph), np.cos(th)], -1)
+    first = engine.bem_field(tab, pts[:2000], far_rule="adaptive")
+    assert tab.view("adaptive", points=0).reserved >> 16 == _lib.MAP_TAG and not tab._map
+    ref = engine.bem_field(tab, pts[:2000])
+    scale = ref.norm(dim=1).clamp(min=abs(float(g["E_gun"])))
+    assert ((first - ref).norm(dim=1) / scale).max() < 2e-12
+    whole = engine.bem_field(tab, pts, far_rule="adaptive")
+    rc, zc, h = _cells(tab)
+    assert tab._map and len(rc) > 0
+    # within two panel lengths of the surface no point has a cell
+    near = torch.as_tensor(d[:2000] * R < np.linalg.norm(np.diff(g["profile"], axis=0), axis=1).min(), device="cuda")
+    assert near.any() and torch.equal(whole[:2000][near], first[near])
+    assert ((whole[:2000] - ref).norm(dim=1) / scale).max() < 2e-12
+    for a, b in ((0, 1), (1, 8), (8, 17), (100, 357), (357, 357 + 2369), (3000, 40_003)):
+        assert torch.equal(engine.bem_field(tab, pts[a:b], far_rule="adaptive"), whole[a:b])
+    nan, inf = float("nan"), float("inf")
+    out = np.array([[1.0, 0, 0], [0, 0, -5.0], [0, 0, 7.0], [nan, 0, 0], [0, nan, 1e-6], [0, 0, nan], [inf, 0, 0]])
+    got = engine.bem_field(tab, out, far_rule="adaptive").cpu().numpy()
+    assert np.array_equal(np.isnan(got).any(axis=-1), ~np.isfinite(out).all(axis=-1))
