@@ -549,7 +549,7 @@ def accel(geometry, pos, active, charge, mass, group_sizes, charge_to_mass, plum
 def bem_field(tables, points, form="fp64", far_rule="reference", **rule_kw):
     """Perturbation field of a BEM solution at points [N, 3] (spt_bem_field)."""
     torch = _torch()
-    x, y, z = _columns(_as_dev(points, torch.float64, tables.seg.device).reshape(-1, 3))
+    x, y, z = _as_dev(points, torch.float64, tables.seg.device).reshape(-1, 3).t().contiguous().unbind(0)
     view = tables.view(far_rule, points=x.numel(), **rule_kw)
     out = torch.empty((3, x.numel()), dtype=torch.float64, device=tables.seg.device)
     stream = torch.cuda.current_stream(tables.seg.device)

@@ -334,11 +334,14 @@ class BemTables:
         points asked for cost as much (field_map.worth), and before that the map
         has none; without, at once.  Where memory for them lacks, the map
         stays without, until as many points have been asked for again."""
-        import torch
         if self._map:
             return self._map
+        if self._bare and points is not None and self._map_points + points < self._map_worth:
+            self._map_points += points  # (without the lock: a count that threads lose only comes later)
+            return self._bare
         if self.clusters is None or self.seg.device.type != "cuda":
             return None
+        import torch
         with self._map_lock:
             if self._map:
                 return self._map
