@@ -185,11 +185,9 @@ int launch_force(const spt_img::ForceArgs& a, size_t bytes, cudaStream_t st) {
     int rc = cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes),
                         "cudaFuncSetAttribute(image_force_kernel)");
     if (rc) return rc;
-    int per_sm = 1;
-    rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, spt_img::kThreads, bytes),
-                    "cudaOccupancyMaxActiveBlocksPerMultiprocessor(image_force_kernel)");
-    if (rc) return rc;
-    const int most = sm_count() * (per_sm < 1 ? 1 : per_sm);
+    // CTAs an SM holds: two by registers up to 16 modes, if their shared memory (1 KiB of the SM's 228 is the
+    // system's in each) fits too; asking the runtime cost the smallest calls 2 us of 36
+    const int most = sm_count() * (MP <= 16 && 2 * (bytes + 2048) <= 228 * 1024 ? 2 : 1);
     const int grid = a.n_groups < most ? a.n_groups : most;
     k<<<grid, spt_img::kThreads, bytes, st>>>(a);
     return cuda_check(cudaGetLastError(), "image_force_kernel launch");
