@@ -1451,7 +1451,7 @@ __device__ __forceinline__ void bem_sums(Ctx& c, int n, int* status_flag) {
 }
 
 // D: rotate E_rho of records [0, n) into (x, y) (record slots 5, 6, 7 = ex, ey, ez)
-static __device__ void bem_rotate(Ctx& c, int n, bool scatter) {
+static __device__ void bem_rotate(Ctx& c, int n) {
     const int tid = threadIdx.x;
     double* P = c.bpt;
     for (int k = tid; k < n; k += c.nt) {
@@ -1463,16 +1463,9 @@ static __device__ void bem_rotate(Ctx& c, int n, bool scatter) {
             ex = e_rho * (x / rho);
             ey = e_rho * (y / rho);
         }
-        if (scatter) {
-            const int i = c.list[k];
-            c.fld[3 * i + 0] = ex;
-            c.fld[3 * i + 1] = ey;
-            c.fld[3 * i + 2] = e_z;
-        } else {
-            P[8 * k + 5] = ex;
-            P[8 * k + 6] = ey;
-            P[8 * k + 7] = e_z;
-        }
+        P[8 * k + 5] = ex;
+        P[8 * k + 6] = ey;
+        P[8 * k + 7] = e_z;
     }
     __syncthreads();
 }
@@ -1705,7 +1698,7 @@ __device__ void surrogate_points(Ctx& c, int n, int* status_flag) {
         }
     }
     __syncthreads();
-    bem_rotate(c, n, false);
+    bem_rotate(c, n);
 }
 
 // Direct field of the point (x, y, z) by this warp, or its share of it: on-surface
@@ -1833,16 +1826,14 @@ __device__ void bem_points_fused(Ctx& c, int n) {
 // 8-double record): the reference's evaluation, phases A-D, or the adaptive
 // rule's one task per point.
 template <int FORM, int FAR>
-__device__ void bem_points(Ctx& c, int n, bool scatter, int* status_flag) {
+__device__ void bem_points(Ctx& c, int n, int* status_flag) {
     if constexpr (FAR == SPT_FAR_ADAPTIVE) {
-        if (!scatter) {
-            bem_points_fused<FORM>(c, n);
-            return;
-        }
+        bem_points_fused<FORM>(c, n);
+    } else {
+        bem_closest(c, n, false);
+        bem_sums<FORM, FAR>(c, n, status_flag);
+        bem_rotate(c, n);
     }
-    bem_closest(c, n, false);
-    bem_sums<FORM, FAR>(c, n, status_flag);
-    bem_rotate(c, n, scatter);
 }
 
 // Softened pair sum over the live sources of the group (forces.py:16-29), mixed
@@ -2068,7 +2059,7 @@ __device__ void stage_accel(Ctx& c, double* out, int* status_flag) {
             if constexpr (FORM == SPT_FORM_SURROGATE)
                 surrogate_points<FAR>(c, n_list, status_flag);
             else
-                bem_points<FORM, FAR>(c, n_list, false, status_flag);
+                bem_points<FORM, FAR>(c, n_list, status_flag);
             // scatter: fld[i] = blended field
             for (int k = tid; k < n_list; k += c.nt) {
                 const int i = c.list[k];

@@ -54,7 +54,7 @@ bem_field_kernel(const double* x, const double* y, const double* z, long long n,
     }
     if (threadIdx.x == 0) s_flag = 0;
     __syncthreads();
-    bem_points<FORM, FAR>(c, np_, false, &s_flag);
+    bem_points<FORM, FAR>(c, np_, &s_flag);
     for (int k = threadIdx.x; k < np_; k += c.nt) {
         ex[p0 + k] = c.bpt[8 * k + 5];
         ey[p0 + k] = c.bpt[8 * k + 6];

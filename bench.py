@@ -41,8 +41,9 @@ In the same run (rank 0):
               that subset (alive particles by position and velocity, killed
               ones by death time), and their attempt counts; beside it the
               plain form's own sensitivity (the same subset with vel0 x
-              (1 + 1e-15)), and the error over the particles that sensitivity
-              shows to be well conditioned (moved < 1e-7 by it).
+              (1 + 1e-15)) and the chosen form's (eight last-digit changes
+              of vel0), and the error over the particles that those show to
+              be well conditioned (moved < 1e-7 by each).
   e2e         the same whole traces through the public API with the state in
               pinned host memory: H2D of the initial state, the trace, D2H of
               the final state, every step.
@@ -76,6 +77,7 @@ UNIT = "particle-steps/s"
 FLOP_PER_RING = 64.0   # nominal FLOPs of one ring-kernel evaluation (26 algebra + 38 for K, E)
 FLOP_PER_PAIR = 20.0   # nominal FLOPs of one softened pair interaction
 FLOP_PER_CLUSTER = 12.0 * 32  # nominal FLOPs of one 32-term cluster expansion (12 per term)
+CHOSEN_STARTS = (-4, -3, -2, -1, 1, 2, 3, 4)  # starts of the chosen form's sensitivity, in 2^-52 of vel0
 WHOLE_TRACE = 1_000_000  # attempt budget of a whole-trace launch (every group reaches t_end far sooner)
 T_END = dict(c0=None, c1=20e-12, c2=20e-12, c3=30e-12, c4=20e-12)
 
@@ -591,6 +593,8 @@ def plain_and_accuracy(args, wl, pos, vel, tb, q, m, sizes, dev, t_max, budget):
         legs.append(("mixed", "mixed", "adaptive"))  # the float32 form, reported beside the chosen one
     if not args.no_sensitivity:
         legs.append(("plain_pert", "fp64", "reference"))  # the plain form's own sensitivity (vel0 x (1 + 1e-15))
+        # ... and the chosen form's, of which several starts cost less than one of the plain form's
+        legs += [(f"chosen_pert{j}", args.form, args.far_rule) for j in CHOSEN_STARTS]
     for name, form, rule in legs:
         tracer = make_tracer(args, wl, dev, form, rule)
         binned = False
@@ -601,7 +605,8 @@ def plain_and_accuracy(args, wl, pos, vel, tb, q, m, sizes, dev, t_max, budget):
                 autotune.apply(args.tuned_config, tracer)
             elif args.cta_threads:
                 tracer.cta_threads = args.cta_threads
-        leg = sub if name != "plain_pert" else (sub[0], sub[1] * (1.0 + 1e-15)) + sub[2:]
+        rel_vel = 1e-15 if name == "plain_pert" else (2.0**-52 * int(name[11:]) if name.startswith("chosen_pert") else 0.0)
+        leg = (sub[0], sub[1] * (1.0 + rel_vel)) + sub[2:]
         run = Runner(tracer, *leg, dev, binned=binned)
         prm = lambda a: tracer.params(t_max, wl["rtol"], wl["atol"], 1e-12, wl["cm"], a)
         # warm-up: a short slice, then the timed span from the initial state
@@ -645,20 +650,29 @@ def plain_and_accuracy(args, wl, pos, vel, tb, q, m, sizes, dev, t_max, budget):
                attempts_plain=int(P["c"]["attempts"]), attempts_chosen=int(C["c"]["attempts"]),
                accepted_steps_ratio=float(C["c"]["accepted"] / max(P["c"]["accepted"], 1)))
     if "plain_pert" in out:
-        # endpoints are only as well defined as the trajectory allows: a 1e-15 change of vel0 moves the
-        # plain form's own endpoints by `sens`; the chosen form is held to 1e-6 where sens < 1e-7
+        # endpoints are only as well defined as the trajectory allows: a last-digit change of vel0 moves a
+        # form's own endpoints by `sens`; the chosen form is held to 1e-6 where sens < 1e-7
         d0, d1, d2 = P["td"], C["td"], out["plain_pert"]["td"]
+        starts = [out[f"chosen_pert{j}"] for j in CHOSEN_STARTS]
         alive_all = ~np.isfinite(d0) & ~np.isfinite(d1) & ~np.isfinite(d2)
+        for X in starts:
+            alive_all &= ~np.isfinite(X["td"])
         rel = lambda X: np.linalg.norm(X["pos"] - P["pos"], axis=-1)[alive_all] / \
             np.linalg.norm(P["pos"], axis=-1)[alive_all]
         sens, err = rel(out["plain_pert"]), rel(C)
-        well = sens < 1e-7
+        spread = np.maximum.reduce([rel(dict(pos=X["pos"] - C["pos"] + P["pos"])) for X in starts])
+        from_plain = [float(rel(X).max()) for X in starts]
+        well = np.maximum(sens, spread) < 1e-7
         acc["plain_self_sensitivity"] = dict(
             what="plain form against itself with vel0 x (1 + 1e-15), alive particles", max_rel_pos=float(sens.max()),
             particles_above_1e6=int((sens > 1e-6).sum()), seconds=out["plain_pert"]["t"])
+        acc["chosen_self_sensitivity"] = dict(
+            what="chosen form against itself with vel0 x (1 + j 2^-52), alive particles", j=list(CHOSEN_STARTS),
+            max_rel_pos=float(spread.max()), particles_above_1e6=int((spread > 1e-6).sum()),
+            max_rel_pos_against_plain=from_plain)
         acc["max_rel_pos_well_conditioned"] = float(err[well].max()) if well.any() else None
         acc["well_conditioned_particles"] = int(well.sum())
-        acc["max_error_over_sensitivity"] = float((err / np.maximum(sens, 1e-7)).max())
+        acc["max_error_over_sensitivity"] = float((err / np.maximum(np.maximum(sens, spread), 1e-7)).max())
     if "mixed" in out:
         X = out["mixed"]
         e = errors(X)
