@@ -208,7 +208,8 @@ def apply(config, tracer, batch=None):
     tracer.round_points = int(config["round_points"])
     tracer.cta_threads = int(config.get("cta_threads", 0))
     # the warp team as the library's choice: it takes launches whose groups fill
-    # every resident warp (and only the forms it serves), the CTA team the rest
+    # three eighths of the resident warps (and only the forms it serves), the CTA
+    # team the rest
     team = int(config.get("team", _lib.TEAM_AUTO))
     tracer.team = _lib.TEAM_CTA if team == _lib.TEAM_CTA else _lib.TEAM_AUTO
     if tracer.tables is not None:

@@ -346,11 +346,13 @@ int far_rule_of(const SptGeometry* g, const SptBem* b) { return is_bem(g->kind) 
 // 128 or 256, else by group size (narrow CTAs for small groups: more groups
 // per SM, fewer warps behind each barrier).  The reference far rule streams
 // 96 KiB node tiles per CTA, so it keeps 256 threads; so does the float64
-// adaptive form for groups of 17 to 64 while four CTAs an SM hold them all, as
-// warps to spare share the direct points (512 groups of 1 to 32 on a micrometre
-// tip: 72 ms, 99 ms with 128 threads; 2000 of them 146 and 129 ms); the learned
-// form needs at least 4 warps (one per 32 TMEM lanes of its 128-row
-// accumulator).
+// adaptive form for up to 592 groups of 17 to 64, twice the CTAs that 148 SMs
+// hold at once, as warps to spare share the direct points.  With 256 / 128
+// threads, log-uniform sizes on a micrometre tip: 64 groups of up to 64 144 / 232
+// ms, 590 of them 155 / 267, 590 of up to 32 70 / 99, 590 of up to 20 46 / 58, 2000
+// of up to 32 146 / 129; on the post tip 590 groups of 64 92 / 106, of 32 47 / 49,
+// of 20 37 / 34.  The learned form needs at least 4 warps (one per 32 TMEM lanes
+// of its 128-row accumulator).
 int trace_threads(const SptState* s, const SptTraceParams* p, int far) {
     const int want = p->cta_threads;
     int t;

@@ -23,8 +23,8 @@ Built once per geometry, like the reference's per-device field cache
   at probe points RATIO_RUN arclengths away, its 8-point sum matches the
   segment-wise Gauss-4 sum to RUN_TOL;
 * field map (field_map.py): the field as polynomials over cells of a quadtree,
-  built on the GPU at the first adaptive view, for the adaptive rule's
-  float64 form.  Not in the reference;
+  sampled on the GPU for a view that is kept or when the points asked for pay,
+  for the adaptive rule's float64 form.  Not in the reference;
 * cluster table [n_cluster, CLUSTER_TERMS + 2]: a binary tree over the runs
   (level l: clusters of 2^l consecutive runs) with, per cluster, its centre
   on the axis, its radius and the axisymmetric multipole moments of its

@@ -220,11 +220,11 @@ typedef struct {
  * doubles: a header of SPT_MAP_HEADER (1 / side of the root square, its lowest
  * z, the offset of the cell records, the offset of the panels' Gauss-8 nodes --
  * rows rho, z, w of 8 n_seg, segment-major, w = area * density --; the root's
- * lowest rho is 0), an int32 table of 4^SPT_MAP_ROOT_BITS entries (the first
+ * lowest rho is 0; a map without cells, which has the panel nodes only, gives
+ * 1 / side as infinite and no tables), an int32 table of 4^SPT_MAP_ROOT_BITS entries (the first
  * quadtree levels, z-index major: a cell's number, -1 for none, or -2 - the
  * number of the next table), int32 tables of 4^SPT_MAP_BITS entries (the levels
- * below, alike), then one record
- * of SPT_MAP_REC per cell: centre rho, centre z, 1 / half-width, 5 unused, and
+ * below, alike), then one record of SPT_MAP_REC per cell: centre rho, centre z, 1 / half-width, 5 unused, and
  * coefficient (component c, rho power i, z power j) at 8 + (2 j + c) *
  * SPT_MAP_N + i.  The powers are of (rho - centre) / half-width, and of
  * rho^2 / (2 half-width^2) - 1 in a cell on the axis (centre rho =
@@ -415,8 +415,8 @@ int spt_map_classify(const double* cells, int32_t n, const SptBem* bem, double k
                      double* far_ratio, void* stream);
 
 /* Samples the field of each candidate cell at its SPT_MAP_N x SPT_MAP_N
- * Chebyshev points, in rho^2 for a cell on the axis (adaptive far rule with bem's thresholds, which must be
- * without a map; no panel may be near) and writes the cell's record, and
+ * Chebyshev points, in rho^2 for a cell on the axis (adaptive far rule with
+ * bem's thresholds, which must be without a map; no panel may be near) and writes the cell's record, and
  * tail[k] = its largest Chebyshev coefficient of the two highest orders over
  * its largest one.  cheb: the SPT_MAP_N nodes; dct [N, N]: values at the nodes
  * to Chebyshev coefficients; mono [N, N]: mono[k * N + i] = coefficient of
