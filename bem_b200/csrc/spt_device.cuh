@@ -408,13 +408,10 @@ __device__ __forceinline__ double seg_dist2(const SptBem& b, int s, double rq, d
     return __dadd_rn(__dmul_rn(dr, dr), __dmul_rn(dz, dz));
 }
 
-// Square root of a squared distance v >= 0 that may be 0: v held at 2^-996 by
-// its high word, as an unsigned number, so that a NaN of either sign stays one
-// (fmax gives the bound for a NaN, and a NaN point was near every panel).
-__device__ __forceinline__ double sqrt_dist2(double v) {
-    const unsigned hi = max((unsigned)__double2hiint(v), (unsigned)(1023 - 996) << 20);
-    return sqrt_pos(__hiloint2double((int)hi, __double2loint(v)));
-}
+// Distance from its components, branch-free: 1e-300 keeps the square off zero (it
+// rounds away beside any real one), and a NaN stays a NaN, which is near no
+// panel (fmax in its place gave the bound for a NaN).
+__device__ __forceinline__ double dist_pos(double x, double y) { return sqrt_pos(fma(x, x, fma(y, y, 1e-300))); }
 
 // near test of bem/axisymmetric.py:566-570 -> (near, projection, distance)
 // FAST (the adaptive rule): a branch-free root, exact to the last bit or two.
@@ -425,7 +422,7 @@ __device__ __forceinline__ bool seg_near(const SptBem& b, int s, double re, doub
     const double along = dr * ur + dz * uz;
     proj = fmin(fmax(along, 0.0), L);
     const double ar = dr - proj * ur, az = dz - proj * uz;
-    if constexpr (FAST) dist = sqrt_dist2(fma(ar, ar, az * az));
+    if constexpr (FAST) dist = dist_pos(ar, az);
     else dist = sqrt(ar * ar + az * az);
     return dist < L;
 }
@@ -437,7 +434,7 @@ __device__ __forceinline__ bool seg_near(const SptBem& b, int s, double re, doub
 __device__ __forceinline__ double blk_lower(const SptBem& b, int q, double r, double z) {
     const double cr = __ldg(b.blk + q), cz = __ldg(b.blk + b.blk_stride + q), rad = __ldg(b.blk + 2 * b.blk_stride + q);
     const double dr = r - cr, dz = z - cz;
-    const double dc = sqrt_dist2(fma(dr, dr, dz * dz));
+    const double dc = dist_pos(dr, dz);
     return dc - rad - 1e-9 * (dc + rad);
 }
 __device__ __forceinline__ double blk_lmax(const SptBem& b, int q) { return __ldg(b.blk + 3 * b.blk_stride + q); }
