@@ -248,12 +248,6 @@ int cuda_check(cudaError_t e, const char* what) {
     if (e != cudaSuccess) return fail(SPT_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
     return SPT_OK;
 }
-}  // namespace spt_abi
-
-namespace {
-using spt_abi::cuda_check;
-using spt_abi::fail;
-using spt_abi::g_err;
 
 int check_bem(const SptBem* b) {
     if (!b || !b->seg || !b->node) return fail(SPT_ERR_ARG, "BEM tables required for this geometry");
@@ -296,6 +290,13 @@ int check_bem(const SptBem* b) {
     }
     return SPT_OK;
 }
+}  // namespace spt_abi
+
+namespace {
+using spt_abi::check_bem;
+using spt_abi::cuda_check;
+using spt_abi::fail;
+using spt_abi::g_err;
 
 bool is_bem(int kind) { return kind == SPT_GEOM_TIP_BEM || kind == SPT_GEOM_WELL_BEM || kind == SPT_GEOM_POST_BEM; }
 

@@ -146,16 +146,11 @@ map_cells_kernel(const double* cells, const __grid_constant__ SptBem bem, const 
 using spt_abi::cuda_check;
 using spt_abi::fail;
 
-static int check_map_args(const SptBem* b) {
-    if (!b || !b->seg || b->n_seg < 1) return fail(SPT_ERR_ARG, "BEM tables required");
-    return SPT_OK;
-}
-
 extern "C" int spt_map_classify(const double* cells, int32_t n, const SptBem* b, double kappa, int32_t* flag,
                                 double* far_ratio, void* stream) {
     if (n <= 0) return SPT_OK;
     if (!cells || !flag || !far_ratio) return fail(SPT_ERR_ARG, "null argument");
-    const int rc = check_map_args(b);
+    const int rc = spt_abi::check_bem(b);
     if (rc) return rc;
     const long long blocks = (n + spt::kMaxWarps - 1LL) / spt::kMaxWarps;
     spt::map_classify_kernel<<<(unsigned)blocks, spt::kMaxThreads, 0, static_cast<cudaStream_t>(stream)>>>(
@@ -167,9 +162,9 @@ extern "C" int spt_map_cells(const double* cells, int32_t n, const SptBem* b, co
                              const double* mono, double* rec, double* tail, void* stream) {
     if (n <= 0) return SPT_OK;
     if (!cells || !cheb || !dct || !mono || !rec || !tail) return fail(SPT_ERR_ARG, "null argument");
-    int rc = check_map_args(b);
+    const int rc = spt_abi::check_bem(b);
     if (rc) return rc;
-    if (b->far_rule != SPT_FAR_ADAPTIVE || !b->node || !b->coarse || b->nodes_per_seg <= 0 || b->reserved)
+    if (b->far_rule != SPT_FAR_ADAPTIVE || b->reserved)
         return fail(SPT_ERR_ARG, "spt_map_cells: needs the adaptive far rule's tables, without a map");
     const size_t smem = spt::kMaxWarps * spt::kWarpScratchInts * 4;
     spt::map_cells_kernel<<<(unsigned)n, spt::kMaxThreads, smem, static_cast<cudaStream_t>(stream)>>>(

@@ -153,3 +153,26 @@ def test_workspace_holds_the_warp_teams_slots():
     p.team = _lib.TEAM_AUTO
     assert _workspace(_state(n_groups=4096, max_size=33), p, geom, bem) == 256
     assert _workspace(_state(n_groups=4096, max_size=32), _params(_lib.FORM_MIXED), geom, bem) == 256
+
+
+@pytest.mark.parametrize("kw,msg", [
+    (dict(), "adaptive far rule's tables"),                                         # the reference rule's
+    (dict(far_rule=_lib.FAR_ADAPTIVE), "coarse node table"),
+    (dict(far_rule=_lib.FAR_ADAPTIVE, coarse=FAKE, coarse_stride=60, ratio4=8.0, ratio2=300.0, blk=FAKE, blk_stride=1,
+          clusters=FAKE, cluster_kappa=3.0, cluster_levels=9, cluster_terms=32), "levels"),
+    (dict(far_rule=_lib.FAR_ADAPTIVE, coarse=FAKE, coarse_stride=60, ratio4=8.0, ratio2=300.0, clusters=FAKE,
+          reserved=_lib.MAP_TAG << 16 | 1), "without a map"),
+    (dict(nodes_per_seg=257), "multiple of 4"),
+    (dict(seg_stride=9), "strides too small"),
+])
+def test_map_cells_checks_its_tables(kw, msg):
+    """The sampling reads the tables that every sum reads, under the same checks."""
+    L, b = _lib.lib(), _bem(**kw)
+    F = ctypes.c_void_p(FAKE)
+    assert L.spt_map_cells(F, 1, ctypes.byref(b), F, F, F, F, F, None) == _lib.SPT_ERR_ARG
+    assert msg in _lib.last_error()
+    if "far" not in msg and "map" not in msg:
+        assert L.spt_map_classify(F, 1, ctypes.byref(b), 3.0, F, F, None) == _lib.SPT_ERR_ARG
+    assert L.spt_map_cells(F, 1, None, F, F, F, F, F, None) == _lib.SPT_ERR_ARG
+    assert L.spt_map_cells(None, 1, ctypes.byref(b), F, F, F, F, F, None) == _lib.SPT_ERR_ARG
+    assert L.spt_map_cells(F, 0, ctypes.byref(b), F, F, F, F, F, None) == _lib.SPT_OK
