@@ -266,9 +266,7 @@ int launch_field(const double* x, const double* y, const double* z, long long n,
         const size_t smem = kMaxWarps * (kWarpScratchInts * 4) + (chunk < kMaxWarps ? split_doubles(kMaxWarps) * 8 : 0);
         const long long grid = (most + chunk - 1) / chunk;
         if (grid > 0x7fffffffLL) return -1;
-        const cudaError_t e = cudaFuncSetAttribute(field_points_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)smem);
-        if (e != cudaSuccess) return (int)e;
+        // (under the 48 KiB that need no attribute: one set per call would be two threads' to race for)
         field_points_kernel<<<(unsigned)grid, kMaxThreads, smem, st>>>(x, y, z, n, (int)chunk, b, mask, ex, ey, ez);
         return (int)cudaGetLastError();
     }

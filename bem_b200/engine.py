@@ -511,7 +511,8 @@ def _columns(p):
 
 def accel(geometry, pos, active, charge, mass, group_sizes, charge_to_mass, plummer_radius, device="cuda",
           form="fp64", coulomb_constant=COULOMB_CONSTANT, far_rule="reference"):
-    """One stage evaluation through spt_accel; returns acc [N, 3] (torch)."""
+    """One stage evaluation through spt_accel; returns acc [N, 3] (torch).  The
+    adaptive rule's field map as in bem_field."""
     torch = _torch()
     sizes = np.asarray(group_sizes, dtype=np.int64)
     offs = np.zeros(len(sizes) + 1, dtype=np.int64)
@@ -547,7 +548,10 @@ def accel(geometry, pos, active, charge, mass, group_sizes, charge_to_mass, plum
 
 
 def bem_field(tables, points, form="fp64", far_rule="reference", **rule_kw):
-    """Perturbation field of a BEM solution at points [N, 3] (spt_bem_field)."""
+    """Perturbation field of a BEM solution at points [N, 3] (spt_bem_field).
+    The adaptive rule's values change once by some 1e-14 of the field, when
+    the geometry has been asked for enough points that its map's cells pay
+    (tables.field_map() samples them beforehand; field_map=False does without)."""
     torch = _torch()
     x, y, z = _as_dev(points, torch.float64, tables.seg.device).reshape(-1, 3).t().contiguous().unbind(0)
     view = tables.view(far_rule, points=x.numel(), **rule_kw)

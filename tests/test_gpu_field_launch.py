@@ -185,3 +185,40 @@ def test_stage_takes_wider_and_deeper_rows():
     want = run(pos)
     assert torch.equal(run(np.concatenate([pos, pos], 1)), want)
     assert torch.equal(run(pos[:, :, None]), want[:, None, :])
+
+
+def test_threads_with_calls_of_different_sizes():
+    """Two threads on their own streams, one asking for a few points at a time
+    and one for many (different shared memory, clusters and splits), by both
+    rules: every call succeeds with the values it has alone."""
+    import threading
+
+    geo = _geometry("post")
+    tab = geo.bem_tables("cuda")
+    assert tab.field_map() is not None  # with its cells from the start: their coming changes the last digits
+    rng = np.random.default_rng(8)
+    d, th = 10 ** rng.uniform(-3, 0.5, 6000), rng.uniform(0, 1.0, 6000)
+    r = geo.R * (1 + d)
+    pts = torch.as_tensor(np.stack([r * np.sin(th), np.zeros_like(r), geo.L + r * np.cos(th)], -1), device="cuda")
+    want = {(n, rule): engine.bem_field(tab, pts[:n], far_rule=rule) for n in (1, 5, 6000) for rule in ("reference", "adaptive")}
+    torch.cuda.synchronize()
+    failed = []
+
+    def work(sizes):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for k in range(600):
+                    n, rule = sizes[k % len(sizes)], ("adaptive", "adaptive", "reference")[k % 3]
+                    got = engine.bem_field(tab, pts[:n], far_rule=rule)
+                    if k % 50 == 0 and not torch.equal(got, want[n, rule]):
+                        failed.append((n, rule))
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:  # noqa: BLE001
+            failed.append(repr(e))
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in ((1, 5), (6000,), (5, 6000))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed[:3]
